@@ -145,7 +145,7 @@ void free_bins(gbr_renderer* r) {
     r->d_items = nullptr;
     r->items_cap = 0;
     r->list_cap = 0;
-    r->seen_pairs = r->seen_visible = 0;
+    r->seen_pairs = r->seen_visible = r->seen_items = 0;
     cudaFree(r->d_dirty);
     r->d_dirty = nullptr;
     r->dirty_valid = false;
@@ -267,10 +267,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.chunk = kMaxChunk;
     F.stage = r->chunk;   // queue_chunk: entries per raster pass
     F.phase = r->raster_phase;
+    F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, (uint32_t)r->num_sms);
     if (r->seen_pairs) {
-        const uint64_t grid = (uint64_t)r->num_sms * (uint64_t)std::max(r->raster_blocks_per_sm, 1);
-        const uint64_t share = r->seen_pairs / (2u * grid);
-        F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), kMinChunk);
         if (F.phase == 0u) F.phase = r->seen_pairs < 4u * r->seen_visible ? kSparsePhase : kPhase;
         // small triangles: about (pairs per visible triangle - 1) x the bin
         // side of width + height each; with the library's phase the
@@ -281,6 +279,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
             F.raster_lanes = extent < kLaneExtentPx ? 1u : 0u;
             if (F.raster_lanes && r->raster_phase == 0u) F.phase = kMaxPhase;
         }
+        const bool record = F.raster_lanes || r->rec_tma;
+        const uint64_t grid = (uint64_t)r->num_sms * (uint64_t)(record ? r->raster_grid.record : r->raster_grid.block128 / 2);
+        const uint64_t share = r->seen_pairs / (2u * grid);
+        F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), record ? kMinChunk : kMinBlockChunk);
     }
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;
@@ -380,7 +382,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     }
     r->last_predicted = predicted;
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[2], s));
-    GBR_CUDA(launch_raster(F, (uint32_t)(r->num_sms * r->raster_blocks_per_sm), s));
+    GBR_CUDA(launch_raster(F, r->raster_grid, s));
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[4], s));
     GBR_CUDA(launch_shade(F, s));
     if (r->timing) {
@@ -423,6 +425,7 @@ gbr_status finish_frame(gbr_renderer* r, cudaStream_t s) {
     if (r->h_ctl->overflow) return fail(GBR_ERR_OUT_OF_MEMORY, "bin storage overflow persists");
     r->seen_pairs = r->h_ctl->num_pairs;
     r->seen_visible = r->h_ctl->num_visible;
+    r->seen_items = r->h_ctl->num_items;
     // predicted capacities that did not fit the list: grow it for the next
     // frames, within reason (the frame itself was re-binned exactly)
     const uint64_t want = r->h_ctl->pred_capacity;
@@ -527,9 +530,7 @@ gbr_status gbr_setup_bins(gbr_renderer* r, uint32_t num_bins_x, uint32_t num_bin
     GBR_CUDA(cudaMemset(r->d_feat, 0, (size_t)kFeatSlots * nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMemset(r->d_feat + 4u * nb, 0xFF, nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMalloc(&r->d_features_out, (size_t)kFeatures * nb * sizeof(float)));
-    int bps = 0;
-    GBR_CUDA(raster_configure(bin_w, bin_h, r->raster_ctas, &bps));
-    r->raster_blocks_per_sm = std::max(bps, 1);
+    GBR_CUDA(raster_configure(bin_w, bin_h, r->raster_ctas, &r->raster_grid));
     r->bins_ready = true;
     r->have_frame = false;
     return GBR_OK;
@@ -689,11 +690,7 @@ gbr_status gbr_set_raster_params(gbr_renderer* r, uint32_t phase, uint32_t ctas_
         return fail(GBR_ERR_INVALID_ARG, "phase %u (0..%u) / ctas_per_sm %u (0, 2..6)", phase, kMaxPhase, ctas_per_sm);
     r->raster_phase = phase;
     r->raster_ctas = ctas_per_sm;
-    if (r->bins_ready) {
-        int bps = 0;
-        GBR_CUDA(raster_configure(r->bw, r->bh, ctas_per_sm, &bps));
-        r->raster_blocks_per_sm = std::max(bps, 1);
-    }
+    if (r->bins_ready) GBR_CUDA(raster_configure(r->bw, r->bh, ctas_per_sm, &r->raster_grid));
     return GBR_OK;
 }
 

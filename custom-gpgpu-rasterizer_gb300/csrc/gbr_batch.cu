@@ -251,7 +251,7 @@ gbr_status ensure_layout(gbr_batch* b) {
     b->last_table.clear();
 
     int bps = 0;
-    GBR_CUDA(raster_configure_batch(bs, bs, b->cfg.raster_ctas, raster_threads(b->cfg), &bps));
+    GBR_CUDA(block_raster_configure(bs, bs, true, raster_threads(b->cfg), b->cfg.raster_ctas, &bps));
     b->raster_bps = std::max(bps, 1);
     b->layout_valid = true;
     return GBR_OK;
@@ -312,7 +312,6 @@ BatchDev batch_dev(const gbr_batch* b) {
     B.list_cap = b->list_cap;
     B.items_cap = b->items_cap;
     B.num_scenes = n;
-    B.phase = b->cfg.raster_phase;
     B.all_flat = b->all_flat;
     B.stage = b->cfg.queue_chunk;
     return B;

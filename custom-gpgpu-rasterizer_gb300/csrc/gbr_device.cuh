@@ -22,12 +22,13 @@ constexpr uint32_t kFlagRaster = 1u;              // fixed path, covered winding
 constexpr uint32_t kFlagFloat = 2u;               // outside the guard band: float edge functions
 constexpr int kMaxBinDim = 64;
 constexpr int kRasterThreads = 256;
-constexpr int kBatch = 2048;                      // bin entries the raster depth-sorts at once
+constexpr int kBatch = 2048;                      // bin entries the record raster depth-sorts at once
 constexpr int kDepthBuckets = 256;                // front-to-back buckets: top 8 bits of the depth key
 constexpr uint32_t kPhase = 16;                   // triangles between hierarchical-z refreshes
 constexpr uint32_t kMaxPhase = 128;               // setup records staged per phase (the record ring)
 constexpr uint32_t kSparsePhase = 64;             // the library's phase for frames of small triangles
 constexpr uint32_t kMinChunk = 64;                // smallest raster work item the library picks
+constexpr uint32_t kMinBlockChunk = 512;          // the same for the block raster
 constexpr uint32_t kMaxChunk = 4096;              // largest raster work item the library picks
 constexpr uint32_t kBatchChunk = 2048;            // raster work items of a batch frame
 // Exact binning counts each bin in `count_split` sub-counters (at most
@@ -40,7 +41,17 @@ __host__ __device__ inline uint32_t count_split_for(unsigned long long pairs, ui
     const unsigned long long per_bin = pairs / (bins ? bins : 1u);
     return per_bin >= 256u ? 8u : per_bin >= 64u ? 4u : per_bin >= 16u ? 2u : 1u;
 }
-constexpr uint32_t kDefaultRasterCtas = 6;
+constexpr uint32_t kDefaultRasterCtas = 6;    // record raster variant (CTAs per SM) used by default
+constexpr uint32_t kDefaultBlockCtas = 5;     // the block raster's
+// The block raster's CTAs in a single frame: 128 threads where the items
+// outnumber the SMs several times (fewer warps wait at each of an item's
+// barriers than in CTAs of 256: 1M soup 78 us against 88, 2M soup at 4K 201
+// against 285; of 64: 94 and 195), 512 where they don't and the longest item
+// decides.
+constexpr uint32_t kWideItemsPerSm = 6;
+__host__ __device__ inline uint32_t block_threads_for(unsigned long long items, uint32_t sms) {
+    return items < (unsigned long long)kWideItemsPerSm * sms ? 512u : 128u;
+}
 // The raster's small-triangle variant: in phases of at least kLanePhase
 // triangles a warp takes kLaneGrab sorted triangles at once and each lane
 // rasterises its own when its pixel box holds at most kLanePixels pixels.
@@ -50,7 +61,7 @@ constexpr uint32_t kDefaultRasterCtas = 6;
 constexpr uint32_t kLanePhase = 32;
 constexpr uint32_t kLaneGrab = 16;
 constexpr int kLanePixels = 16;
-constexpr double kLaneExtentPx = 16.0;        // raster_kernel variant (CTAs per SM) used by default
+constexpr double kLaneExtentPx = 16.0;
 // Exact binning with block-private counter rows: one block of kRowThreads
 // per SM counts its pairs per bin in shared memory (num_bins <=
 // kMaxRowBins), then takes its run of every bin it touched with one global
@@ -199,7 +210,7 @@ struct FrameDev {
     uint32_t px_begin, px_end;
     uint32_t rec_tma;          // raster: setup records staged by bulk asynchronous copies (1) or loads (0)
     uint32_t raster_lanes;     // raster: the small-triangle variant (a lane per triangle; phases >= kLanePhase)
-    uint32_t rows_pad;
+    uint32_t block_threads;    // block raster: threads per CTA, 128 or 512
     // two-pass shading of a sparse frame: one byte per bin, "may hold drawn
     // pixels".  dirty_rd: after the last frame; dirty_wr: this frame's, zeroed
     // by its first scan and set by the raster for every bin it draws.  The
@@ -283,7 +294,6 @@ struct BatchDev {
     unsigned long long list_cap;
     uint32_t items_cap;
     uint32_t num_scenes;
-    uint32_t phase;               // raster: triangles between hierarchical-z refreshes (0: kPhase)
     uint32_t all_flat;            // every scene shades flat: the shade pass runs its flat variant
     uint32_t stage;               // raster pass size (FrameDev::stage)
 };

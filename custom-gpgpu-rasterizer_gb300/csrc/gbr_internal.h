@@ -10,6 +10,7 @@
 
 #include "../../include/gbr.h"
 #include "gbr_device.cuh"
+#include "gbr_kernels.h"
 
 namespace gbr {
 
@@ -58,7 +59,7 @@ struct gbr_renderer {
     bool bins_ready = false;
     uint32_t binning = GBR_BINNING_EXACT;
     int timing = 0;           // GBR_TIMING_*
-    int raster_blocks_per_sm = 1;
+    gbr::RasterGrid raster_grid;   // resident raster CTAs per SM
     uint32_t raster_phase = 0;   // 0: library default
     uint32_t raster_ctas = 0;    // 0: library default
     uint32_t row0 = 0, row1 = 0;      // gbr_set_bin_rows: this renderer's bin rows (row1 0: all)
@@ -67,7 +68,7 @@ struct gbr_renderer {
     uint32_t scan_silent_tile1 = 0;   // gbr_set_scan_wait: 1 + the silent tile (0: none)
     // the last finished frame's pair and visible-triangle counts: they size
     // the next frames' raster work items and phases (0: none seen yet)
-    uint64_t seen_pairs = 0, seen_visible = 0;
+    uint64_t seen_pairs = 0, seen_visible = 0, seen_items = 0;
 
     // predicted-capacity binning
     uint32_t* d_feat = nullptr;

@@ -16,11 +16,11 @@
 //   fill_kernel  : second pass: each pair's id goes to its bin's offset +
 //                  rank, no atomics (fill_rows_kernel: to the block's run,
 //                  slots from shared-memory cursors).
-//   raster_kernel: persistent CTAs pull work items; a CTA depth-sorts its
-//                  chunk by the key bounds, rasterises front to back into a
-//                  shared-memory tile of packed (depth key, prim id) with
-//                  64-bit atomicMin (hierarchical-z rejection between phases),
-//                  and publishes the tile to the merge buffer.
+//   block_raster_kernel (gbr_raster.cu): persistent CTAs pull work items,
+//                  depth-sort the chunk by the key bounds and rasterise it
+//                  front to back, a warp to 8x4 pixels; raster_kernel, here,
+//                  takes frames of small triangles (a lane per triangle) and
+//                  the bulk-copy staging on request.
 //   shade_kernel : each pixel's winner shaded once: colour, depth and id.
 //
 // Reference stages replaced: VS_Kernel, TA_Kernel, TB_Kernel,
@@ -31,6 +31,7 @@
 
 #include "gbr_device.cuh"
 #include "gbr_kernels.h"
+#include "gbr_raster.cuh"
 #include "gbr_shade.cuh"
 
 namespace gbr {
@@ -382,35 +383,21 @@ cudaError_t launch_list_touch(const FrameDev& F, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Raster + ROP + shade
 // ---------------------------------------------------------------------------
-// A raster CTA of THREADS threads stages 8 entries per thread at once and
-// sorts them into THREADS depth buckets (one per thread): the top
-// log2(THREADS) bits of the 31-bit depth key.
-template <int THREADS>
-struct RasterGeom {
-    static_assert(THREADS == 128 || THREADS == 256, "raster CTAs of 128 or 256 threads");
-    static constexpr uint32_t kEntries = 8u * THREADS;             // entries depth-sorted at once
-    static constexpr uint32_t kKeyShift = THREADS == 256 ? 23u : 24u;   // depth key -> bucket
-};
-static_assert(RasterGeom<kRasterThreads>::kEntries == (uint32_t)kBatch, "the 256-thread raster sorts kBatch entries");
-
-template <int THREADS>
-struct RasterSharedT {
+struct RasterShared {
     TriSetup rec[kMaxPhase];     // setup records of the running phase
-    uint32_t prim[RasterGeom<THREADS>::kEntries];   // staged bin entries (rasterisable triangles)
-    uint32_t key[RasterGeom<THREADS>::kEntries];    // their depth-key lower bounds
-    uint16_t order[RasterGeom<THREADS>::kEntries];  // staged triangles, front to back by depth bucket
-    uint32_t bucket[THREADS];    // counts -> starts -> (after the scatter) ends
-    uint32_t warp_count[THREADS / 32];
-    uint32_t warp_max[THREADS / 32];
+    uint32_t prim[kBatch];       // staged bin entries (rasterisable triangles)
+    uint32_t key[kBatch];        // their depth-key lower bounds
+    uint16_t order[kBatch];      // staged triangles, front to back by depth bucket
+    uint32_t bucket[kDepthBuckets];   // counts -> starts -> (after the scatter) ends
+    uint32_t warp_count[kRasterThreads / 32];
+    uint32_t warp_max[kRasterThreads / 32];
     uint32_t item[4];
     __align__(16) uint4 item_next;   // the next work item, copied ahead by thread 0
     int next;
-    uint32_t scene_next;         // batch: scene of the fetched work item
-    uint32_t scene_loaded;       // batch: scene whose descriptor `frame` holds
     __align__(8) unsigned long long rec_bar[2];   // mbarriers: a phase's setup records have landed (phases alternate)
-    __align__(16) FrameDev frame;
 };
-using RasterShared = RasterSharedT<kRasterThreads>;
+static_assert(kDepthBuckets == kRasterThreads, "one depth bucket per thread");
+constexpr uint32_t kKeyShift = 23u;   // depth key -> bucket: the top 8 bits of the 31-bit key
 
 // Setup records reach shared memory by bulk asynchronous copies (the TMA
 // engine's cp.async.bulk, one 48-byte copy per record), each completing
@@ -604,45 +591,24 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
     F.ids[gi] = prim;
 }
 
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Work item `idx` into shared memory by an asynchronous 16-byte copy (the
-// end marker when the queue is drained); cp_async_wait_all() completes it.
-__device__ __forceinline__ void fetch_item(uint4* dst, const uint4* items, uint32_t idx, uint32_t num_items) {
-    if (idx >= num_items) {
-        *dst = make_uint4(0xFFFFFFFFu, 0u, 0u, 0u);
-        return;
-    }
-    const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(items + idx) : "memory");
-}
-
-// Persistent raster.  Single frame (BATCH false): work items of F.  Batch
-// (BATCH true): work items of all scenes of B; the scene of an item is
-// found from its global bin, and its frame descriptor is copied to shared
-// memory when it differs from the previous item's.
-// MIN_CTAS counts CTAs of 256 threads: a 128-thread variant keeps twice as
-// many resident (the same registers per thread).
-// LANES: the small-triangle variant (kLanePhase), a kernel of its own so
-// that the one-triangle-per-warp path keeps its registers.
-template <int MIN_CTAS, bool BATCH, bool TMA = false, int THREADS = kRasterThreads, bool LANES = false>
-__global__ void __launch_bounds__(THREADS, MIN_CTAS * (kRasterThreads / THREADS)) raster_kernel(FrameDev F, BatchDev B) {
+// The record raster: persistent CTAs that stage a phase's setup records in
+// shared memory and merge fragments into a shared tile.  It runs the frames
+// of small triangles (TMA false: a lane per triangle, kLanePhase) and, on
+// request, the bulk-copy staging (TMA); the others take the block raster.
+template <int MIN_CTAS, bool TMA>
+__global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameDev F) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using Shared = RasterSharedT<THREADS>;
-    constexpr uint32_t kEntries = RasterGeom<THREADS>::kEntries, kKeyShift = RasterGeom<THREADS>::kKeyShift;
-    Shared& S = *reinterpret_cast<Shared*>(smem_raw);
-    unsigned long long* tile = reinterpret_cast<unsigned long long*>(smem_raw + sizeof(Shared));
+    constexpr uint32_t kEntries = kBatch, THREADS = kRasterThreads;
+    RasterShared& S = *reinterpret_cast<RasterShared*>(smem_raw);
+    unsigned long long* tile = reinterpret_cast<unsigned long long*>(smem_raw + sizeof(RasterShared));
     pdl_wait();
-    Ctl* const Q = BATCH ? B.ctl : F.ctl;
-    const uint4* const items = BATCH ? B.items : F.items;
+    Ctl* const Q = F.ctl;
+    const uint4* const items = F.items;
     if (Q->overflow) return;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t num_items = Q->num_items;
-    const uint32_t phase_req = BATCH ? B.phase : F.phase;
-    const uint32_t phase = phase_req == 0u ? kPhase : min(phase_req, kMaxPhase);
-    const uint32_t stage_req = BATCH ? B.stage : F.stage;
-    const uint32_t pass = stage_req == 0u ? kEntries : min(stage_req, kEntries);   // entries per raster pass
-    if (BATCH && tid == 0) S.scene_loaded = 0xFFFFFFFFu;
+    const uint32_t phase = F.phase == 0u ? kPhase : min(F.phase, kMaxPhase);
+    const uint32_t pass = F.stage == 0u ? kEntries : min(F.stage, kEntries);   // entries per raster pass
     // thread 0 runs one item ahead: the next item's queue slot is taken when
     // an item starts and its descriptor copied to shared memory
     // (asynchronously) while the item is staged
@@ -662,41 +628,25 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS * (kRasterThreads / THREADS)
     for (;;) {
         if (tid == 0) {
             cp_async_wait_all();
-            uint4 it = S.item_next;
-            if (BATCH && it.x != 0xFFFFFFFFu) {
-                const uint32_t sc = __ldg(B.bin_scene + it.x);
-                S.scene_next = sc;
-                it.x -= __ldg(B.bin_base + sc);
-            }
+            const uint4 it = S.item_next;
             S.item[0] = it.x; S.item[1] = it.y; S.item[2] = it.z; S.item[3] = it.w;
             if (it.x != 0xFFFFFFFFu) next_idx = atomicAdd(&Q->item_next, 1u);
         }
         __syncthreads();
         const uint32_t bin = S.item[0];
         if (bin == 0xFFFFFFFFu) break;
-        if (!BATCH && tid == 0 && F.dirty_wr) F.dirty_wr[bin] = 1u;   // the bin's pixels may now be drawn
-        if (BATCH) {
-            const uint32_t sc = S.scene_next;
-            if (sc != S.scene_loaded) {   // uniform across the CTA
-                const uint4* src = reinterpret_cast<const uint4*>(B.scenes + sc);
-                uint4* dst = reinterpret_cast<uint4*>(&S.frame);
-                for (uint32_t i = tid; i < sizeof(FrameDev) / 16u; i += THREADS) dst[i] = __ldg(src + i);
-                __syncthreads();
-                if (tid == 0) S.scene_loaded = sc;
-            }
-        }
-        const FrameDev& G = BATCH ? S.frame : F;
+        if (tid == 0 && F.dirty_wr) F.dirty_wr[bin] = 1u;   // the bin's pixels may now be drawn
         const uint32_t start = S.item[1], count = S.item[2], nchunks = S.item[3];
-        const int tx0 = (int)((bin % G.nbx) * G.bw), ty0 = (int)((bin / G.nbx) * G.bh);
-        const int tw = min((int)G.bw, (int)G.width - tx0), th = min((int)G.bh, (int)G.height - ty0);
+        const int tx0 = (int)((bin % F.nbx) * F.bw), ty0 = (int)((bin / F.nbx) * F.bh);
+        const int tw = min((int)F.bw, (int)F.width - tx0), th = min((int)F.bh, (int)F.height - ty0);
         const int npx = (tw > 0 && th > 0) ? tw * th : 0;
-        const uint32_t* const list = G.list;
-        const TriSetup* const setup = G.setup;
-        unsigned long long* const gvis = G.gvis;
-        const uint32_t width = G.width;
+        const uint32_t* const list = F.list;
+        const TriSetup* const setup = F.setup;
+        unsigned long long* const gvis = F.gvis;
+        const uint32_t width = F.width;
         for (int i = (int)tid; i < npx; i += THREADS) tile[i] = kEmptyVis;
         if (tid == 0) fetch_item(&S.item_next, items, next_idx, num_items);
-        const uint32_t* const keys = G.keys;
+        const uint32_t* const keys = F.keys;
         for (uint32_t b0 = 0; b0 < count && npx > 0; b0 += pass) {
             // stage the entries with their depth-key bounds (no setup record
             // is read before a triangle's phase comes) and count the
@@ -818,7 +768,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS * (kRasterThreads / THREADS)
                 // kLanePhase triangles, each lane rasterises its own when its
                 // pixel box holds at most kLanePixels pixels, and the warp the
                 // others
-                const bool lanes = LANES && phase >= kLanePhase;
+                const bool lanes = !TMA && phase >= kLanePhase;
                 for (;;) {
                     int kb = 0;
                     if (lane == 0) kb = atomicAdd(&S.next, lanes ? (int)kLaneGrab : 1);
@@ -1114,11 +1064,6 @@ __global__ void __launch_bounds__(256) batch_shade_kernel(BatchDev B, uint32_t c
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-size_t raster_smem_bytes(uint32_t bw, uint32_t bh, uint32_t threads) {
-    const size_t shared = threads == 128u ? sizeof(RasterSharedT<128>) : sizeof(RasterSharedT<256>);
-    return shared + (size_t)bw * bh * sizeof(unsigned long long);
-}
-
 // Blocks of 256 threads for a triangle pass: one per 256 triangles, at most
 // 8 per SM.  The blocks stride over the triangles, so a guarded launch that
 // does not run costs one grid of early exits; more blocks than are resident
@@ -1181,26 +1126,45 @@ cudaError_t launch_fill(const FrameDev& F, cudaStream_t s) {
     return launch_pdl(fill_kernel, dim3(blocks), dim3(256), 0, s, F);
 }
 
-template <bool BATCH, bool TMA = false, int THREADS = kRasterThreads, bool LANES = false>
-static cudaError_t launch_raster_variant(const FrameDev& F, const BatchDev& B, uint32_t ctas, uint32_t grid, size_t smem,
-                                         cudaStream_t s) {
-    const dim3 g(grid), b(THREADS);
+static size_t record_smem(uint32_t bw, uint32_t bh) {
+    return sizeof(RasterShared) + (size_t)bw * bh * sizeof(unsigned long long);
+}
+
+using RecordRaster = void (*)(FrameDev);
+
+template <bool TMA>
+static RecordRaster record_variant(uint32_t ctas) {
     switch (ctas ? ctas : kDefaultRasterCtas) {
-        case 2: return launch_pdl(raster_kernel<2, BATCH, TMA, THREADS, LANES>, g, b, smem, s, F, B);
-        case 3: return launch_pdl(raster_kernel<3, BATCH, TMA, THREADS, LANES>, g, b, smem, s, F, B);
-        case 5: return launch_pdl(raster_kernel<5, BATCH, TMA, THREADS, LANES>, g, b, smem, s, F, B);
-        case 6: return launch_pdl(raster_kernel<6, BATCH, TMA, THREADS, LANES>, g, b, smem, s, F, B);
-        default: return launch_pdl(raster_kernel<4, BATCH, TMA, THREADS, LANES>, g, b, smem, s, F, B);
+        case 2: return raster_kernel<2, TMA>;
+        case 3: return raster_kernel<3, TMA>;
+        case 5: return raster_kernel<5, TMA>;
+        case 6: return raster_kernel<6, TMA>;
+        default: return raster_kernel<4, TMA>;
     }
 }
 
-cudaError_t launch_raster(const FrameDev& F, uint32_t grid, cudaStream_t s) {
+cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid* per_sm) {
+    const size_t smem = record_smem(bw, bh);
+    for (const RecordRaster k : {record_variant<true>(ctas), record_variant<false>(ctas)}) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm->record, k, kRasterThreads, smem);
+        if (e != cudaSuccess) return e;
+    }
+    cudaError_t e = block_raster_configure(bw, bh, false, 128u, ctas, &per_sm->block128);
+    if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, 512u, ctas, &per_sm->block512);
+    for (int* n : {&per_sm->record, &per_sm->block128, &per_sm->block512}) *n = std::max(*n, 1);
+    return e;
+}
+
+cudaError_t launch_raster(const FrameDev& F, const RasterGrid& per_sm, cudaStream_t s) {
+    if (F.rec_tma || F.raster_lanes)
+        return launch_pdl(F.rec_tma ? record_variant<true>(F.raster_ctas) : record_variant<false>(F.raster_ctas),
+                          dim3((uint32_t)(sm_count() * per_sm.record)), dim3(kRasterThreads), record_smem(F.bw, F.bh), s,
+                          F);
     BatchDev none;
     memset(&none, 0, sizeof none);
-    const size_t smem = raster_smem_bytes(F.bw, F.bh);
-    if (F.rec_tma) return launch_raster_variant<false, true>(F, none, F.raster_ctas, grid, smem, s);
-    if (F.raster_lanes) return launch_raster_variant<false, false, kRasterThreads, true>(F, none, F.raster_ctas, grid, smem, s);
-    return launch_raster_variant<false>(F, none, F.raster_ctas, grid, smem, s);
+    return launch_block_raster(F, none, false, F.block_threads, F.raster_ctas, F.bw, F.bh,
+                               (uint32_t)(sm_count() * per_sm.block(F.block_threads)), s);
 }
 
 cudaError_t launch_shade(const FrameDev& F, cudaStream_t s) {
@@ -1236,9 +1200,7 @@ cudaError_t launch_batch(const BatchDev& B, const BatchLaunch& L, cudaStream_t s
     if (L.tri_blocks) batch_fill_kernel<<<L.tri_blocks, 256, 0, s>>>(B);
     FrameDev none;
     memset(&none, 0, sizeof none);
-    const size_t smem = raster_smem_bytes(L.bin_w, L.bin_h, L.raster_threads);
-    e = L.raster_threads == 128u ? launch_raster_variant<true, false, 128>(none, B, L.raster_ctas, L.raster_grid, smem, s)
-                                 : launch_raster_variant<true>(none, B, L.raster_ctas, L.raster_grid, smem, s);
+    e = launch_block_raster(none, B, true, L.raster_threads, L.raster_ctas, L.bin_w, L.bin_h, L.raster_grid, s);
     if (e != cudaSuccess) return e;
     if (L.px_blocks) {
         if (B.all_flat) batch_shade_kernel<true><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
@@ -1250,46 +1212,6 @@ cudaError_t launch_batch(const BatchDev& B, const BatchLaunch& L, cudaStream_t s
 cudaError_t launch_clear(const FrameDev& F, cudaStream_t s) {
     clear_kernel<<<1024, 256, 0, s>>>(F);
     return cudaGetLastError();
-}
-
-template <int MIN_CTAS, bool BATCH, int THREADS>
-static cudaError_t configure_variant(size_t smem, int* blocks_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(raster_kernel<MIN_CTAS, BATCH, false, THREADS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (!BATCH) {   // the bulk-copy staging and small-triangle variants of a single frame
-        e = cudaFuncSetAttribute(raster_kernel<MIN_CTAS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(raster_kernel<MIN_CTAS, false, false, kRasterThreads, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_kernel<MIN_CTAS, BATCH, false, THREADS>,
-                                                         THREADS, smem);
-}
-
-template <bool BATCH, int THREADS = kRasterThreads>
-static cudaError_t configure(uint32_t bw, uint32_t bh, uint32_t ctas, int* blocks_per_sm) {
-    const size_t smem = raster_smem_bytes(bw, bh, THREADS);
-    switch (ctas ? ctas : kDefaultRasterCtas) {
-        case 2: return configure_variant<2, BATCH, THREADS>(smem, blocks_per_sm);
-        case 3: return configure_variant<3, BATCH, THREADS>(smem, blocks_per_sm);
-        case 5: return configure_variant<5, BATCH, THREADS>(smem, blocks_per_sm);
-        case 6: return configure_variant<6, BATCH, THREADS>(smem, blocks_per_sm);
-        default: return configure_variant<4, BATCH, THREADS>(smem, blocks_per_sm);
-    }
-}
-
-cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, int* blocks_per_sm) {
-    return configure<false>(bw, bh, ctas, blocks_per_sm);
-}
-
-cudaError_t raster_configure_batch(uint32_t bw, uint32_t bh, uint32_t ctas, uint32_t threads, int* blocks_per_sm) {
-    return threads == 128u ? configure<true, 128>(bw, bh, ctas, blocks_per_sm) : configure<true>(bw, bh, ctas, blocks_per_sm);
-}
-
-cudaError_t raster_configure(uint32_t bw, uint32_t bh, int* blocks_per_sm) {
-    return raster_configure(bw, bh, 0u, blocks_per_sm);
 }
 
 }  // namespace gbr

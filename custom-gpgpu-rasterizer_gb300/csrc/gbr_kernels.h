@@ -30,11 +30,22 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// threads: raster CTA width (128 or 256)
-size_t raster_smem_bytes(uint32_t bw, uint32_t bh, uint32_t threads = 256);
-cudaError_t raster_configure(uint32_t bw, uint32_t bh, int* blocks_per_sm);
-// ctas: the raster_kernel variant compiled for 2..6 CTAs per SM (0: default)
-cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, int* blocks_per_sm);
+// Resident CTAs per SM of the raster kernels of a single frame with bins of
+// bw x bh pixels.  ctas: the variant compiled for 2..6 CTAs per SM (0:
+// default).
+struct RasterGrid {
+    int block128 = 1, block512 = 1;   // block raster, CTAs of 128 and of 512 threads
+    int record = 1;                   // record raster (small-triangle and bulk-copy variants)
+    int block(uint32_t threads) const { return threads == 128u ? block128 : block512; }
+};
+cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid* per_sm);
+// The block raster (gbr_raster.cu) for a batch frame (B's scenes) or a single
+// frame (F), in CTAs of 128 or 256 threads (a batch) or of
+// 128 or 512 (a frame).
+cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas,
+                                   int* blocks_per_sm);
+cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,
+                                uint32_t bw, uint32_t bh, uint32_t grid, cudaStream_t s);
 cudaError_t launch_setup(const FrameDev& F, bool predicted, cudaStream_t s);
 // The bin scan of a frame (mode: kScanExact, ...), one launch.
 ScanDev scan_of(const FrameDev& F, uint32_t mode);
@@ -45,7 +56,7 @@ cudaError_t launch_fill(const FrameDev& F, cudaStream_t s);
 // list_touch_kernel); worth its launch once a frame holds ~1M entries.
 constexpr unsigned long long kListTouchMinPairs = 1ull << 20;
 cudaError_t launch_list_touch(const FrameDev& F, cudaStream_t s);
-cudaError_t launch_raster(const FrameDev& F, uint32_t grid, cudaStream_t s);
+cudaError_t launch_raster(const FrameDev& F, const RasterGrid& per_sm, cudaStream_t s);
 cudaError_t launch_shade(const FrameDev& F, cudaStream_t s);
 cudaError_t launch_clear(const FrameDev& F, cudaStream_t s);
 
@@ -61,7 +72,6 @@ struct BatchLaunch {
 };
 // reset, setup + count, bin scan (three launches), fill, raster, shade
 cudaError_t launch_batch(const BatchDev& B, const BatchLaunch& L, cudaStream_t s);
-cudaError_t raster_configure_batch(uint32_t bw, uint32_t bh, uint32_t ctas, uint32_t threads, int* blocks_per_sm);
 
 // Message returned by gbr_last_error_string() on the calling thread.
 void set_last_error(const char* msg);

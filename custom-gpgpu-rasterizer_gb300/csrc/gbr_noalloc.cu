@@ -147,8 +147,8 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
         }
         slot = s;
     }
-    int blocks_per_sm = 0;
-    e = raster_configure(bin_w, bin_h, &blocks_per_sm);
+    RasterGrid per_sm;
+    e = raster_configure(bin_w, bin_h, 0u, &per_sm);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
 
     unsigned char* b = slot.base;
@@ -164,6 +164,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     F.num_tris = (uint32_t)tris;
     F.chunk = kMaxChunk;      // work items: the library's split
     F.stage = queue_chunk;    // entries per raster pass
+    F.block_threads = block_threads_for(nb, (uint32_t)slot.num_sms);
     for (int k = 0; k < 3; ++k) { F.cam_pos[k] = cam->pos[k]; F.cam_fwd[k] = cam->fwd[k]; }
     F.meshes = reinterpret_cast<const MeshDev*>(b + kOffMesh);
     F.setup = reinterpret_cast<TriSetup*>(b + kOffSetup);
@@ -215,7 +216,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     if (e == cudaSuccess) e = launch_setup(F, false, s);
     if (e == cudaSuccess) e = launch_scan(scan_of(F, kScanExact), s);
     if (e == cudaSuccess) e = launch_fill(F, s);
-    if (e == cudaSuccess) e = launch_raster(F, (uint32_t)(slot.num_sms * (blocks_per_sm > 0 ? blocks_per_sm : 1)), s);
+    if (e == cudaSuccess) e = launch_raster(F, per_sm, s);
     if (e == cudaSuccess) e = launch_shade(F, s);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
     // the frame is only valid if its bin entries fitted the static storage

@@ -1,0 +1,20 @@
+// gbr_raster.cuh -- the raster kernels' work queue.
+#pragma once
+#include "gbr_device.cuh"
+
+namespace gbr {
+
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Work item `idx` into shared memory by an asynchronous 16-byte copy (the
+// end marker when the queue is drained); cp_async_wait_all() completes it.
+__device__ __forceinline__ void fetch_item(uint4* dst, const uint4* items, uint32_t idx, uint32_t num_items) {
+    if (idx >= num_items) {
+        *dst = make_uint4(0xFFFFFFFFu, 0u, 0u, 0u);
+        return;
+    }
+    const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(items + idx) : "memory");
+}
+
+}  // namespace gbr

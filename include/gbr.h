@@ -95,7 +95,8 @@ gbr_status gbr_destroy(gbr_renderer *r);
  * keeps the queue size's role in the raster: a bin's triangles are
  * depth-sorted and rasterised into its tile queue_chunk at a time (at most
  * 2048; 0 = 4096, i.e. 2048).  Long bins are split across raster CTAs by the
- * library, in work items of 64..4096 entries sized from the last frame. */
+ * library, in work items of 64..4096 entries (512..4096 in the block raster)
+ * sized from the last frame. */
 gbr_status gbr_setup_bins(gbr_renderer *r, uint32_t num_bins_x, uint32_t num_bins_y,
                           uint32_t bin_w, uint32_t bin_h, uint32_t queue_chunk);
 
@@ -221,9 +222,11 @@ gbr_status gbr_set_lights(gbr_renderer *r, const gbr_light *lights, uint32_t n);
 /* Binning method for the following frames. */
 gbr_status gbr_set_binning(gbr_renderer *r, uint32_t method);
 /* Raster tuning (no counterpart in the reference; used by the autotuner):
- * phase = triangles rasterised between hierarchical-z refreshes, 0..128 (0: the library's choice: 16,
- * 64 for frames of small triangles, 128 with the raster's small-triangle variant),
- * ctas_per_sm = occupancy variant of the raster kernel, 2..6 (0: 6). */
+ * phase = triangles the small-triangle and bulk-copy raster variants rasterise between hierarchical-z
+ * refreshes, 0..128 (0: the library's choice: 16, 64 for frames of small triangles, 128 with the
+ * small-triangle variant; below 32 the small-triangle variant is not taken; the block raster refreshes after
+ * every triangle), ctas_per_sm = occupancy variant of the raster kernel in CTAs of 256 threads, 2..6 (0: the
+ * library's choice). */
 gbr_status gbr_set_raster_params(gbr_renderer *r, uint32_t phase, uint32_t ctas_per_sm);
 /* How the raster stages triangle-setup records into shared memory (no
  * counterpart in the reference, whose RA_PerTileKernel reads them from global
@@ -298,10 +301,11 @@ typedef struct {
     uint32_t bin_size;     /* bins of bin_size x bin_size pixels, 1..64 */
     uint32_t queue_chunk;  /* entries depth-sorted and rasterised per pass over a tile, >= 1 (at most 2048
                               used); work items hold 2048 entries */
-    uint32_t raster_ctas;  /* raster variant: CTAs per SM, 2..6 (0: 6), counted in CTAs of 256 threads */
-    uint32_t raster_phase; /* triangles between hierarchical-z refreshes, 0..128 (0: 16) */
+    uint32_t raster_ctas;  /* raster variant: CTAs per SM, 2..6 (0: 5), counted in CTAs of 256 threads */
+    uint32_t raster_phase; /* 0..128; kept, without effect: a batch's raster refreshes its depth bounds after
+                              every triangle */
     uint32_t raster_threads; /* threads per bin: raster CTAs of 128 or 256 threads (0: 256); a 128-thread CTA
-                                depth-sorts 1024 entries at a time into 128 buckets, and twice raster_ctas
+                                depth-sorts 1024 entries at a time (else 2048), and twice raster_ctas
                                 of them are resident per SM */
 } gbr_batch_config;
 typedef struct {

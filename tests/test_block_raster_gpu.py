@@ -1,0 +1,67 @@
+"""The block raster (gbr_raster.cu) where its split can go wrong, against the
+oracle's fixed-point mode: bins that are not whole 8x4 blocks, bins of fewer
+blocks than a CTA has warps and of many times more, items around one phase
+(32 triangles) and around one sorted pass (1024 and 2048 entries), triangles
+around and far above the extent that keeps 32-bit edge values, and triangles
+on the float path.  Winners and depth bit-exact, colour within 1 LSB."""
+import numpy as np
+import pytest
+
+import scenes
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def triangles(kind, n, width, height, seed):
+    v = scenes.soup_vertices(n, width, height, seed)
+    if kind == "small":
+        return v
+    if kind == "inside":   # every triangle meets the screen
+        v["p"][:, :2] = v["p"][:, :2].clip(-0.95, 0.95)
+        return v
+    rng = np.random.default_rng(seed)
+    p = v["p"].reshape(-1, 3, 3)
+    # every fourth triangle's first vertex thrown out to the given distance:
+    # extents around 128 to 1024 px (the 32-bit limit is 2^14 px over the
+    # bin's width + height), thousands of px, or beyond the guard band
+    far = {"wide": (100.0, 1100.0), "huge": (2000.0, 8000.0), "float": (8300.0, 50000.0)}[kind]
+    k = np.arange(0, len(p), 4)
+    angle, reach = rng.uniform(0, 2 * np.pi, len(k)), rng.uniform(*far, len(k))
+    p[k, 0, 0] += (2.0 * reach * np.cos(angle) / width).astype(np.float32)
+    p[k, 0, 1] += (2.0 * reach * np.sin(angle) / height).astype(np.float32)
+    v["p"] = p.reshape(-1, 3)
+    return v
+
+
+@pytest.mark.parametrize("bw,bh,w,h,n,kind", [
+    (1, 1, 40, 24, 60, "small"),           # one pixel a bin, eight warps on one block
+    (8, 4, 96, 60, 400, "small"),          # one block a bin
+    (7, 5, 100, 61, 600, "wide"),          # ragged blocks, ragged last bins
+    (8, 8, 128, 96, 33, "huge"),           # items of at most a phase
+    (24, 20, 333, 250, 3000, "wide"),
+    (16, 16, 640, 480, 4000, "huge"),
+    (16, 16, 320, 240, 500, "float"),
+    (64, 64, 300, 200, 9000, "wide"),      # 128 blocks a bin, several passes an item
+    (64, 64, 64, 64, 32, "inside"),        # one bin: a whole phase, then one more
+    (64, 64, 64, 64, 33, "inside"),
+    (64, 64, 64, 64, 1024, "inside"),      # a whole pass of a 128-thread CTA, then one more
+    (64, 64, 64, 64, 1025, "inside"),
+    (64, 64, 64, 64, 2049, "inside"),      # one entry past a 256-thread CTA's pass
+    (33, 17, 66, 34, 5000, "huge"),
+])
+def test_block_raster_against_the_oracle(gbr_lib, cuda_device, bw, bh, w, h, n, kind):
+    v = triangles(kind, n, w, h, seed=31)
+    s = scenes.Scene(kind, w, h, bw, bh, scenes.identity_camera(), [scenes.Mesh(vertices=v)], cull=scenes.CULL_NONE)
+    o = oracle.render(s, oracle.RASTER_FIXED)
+    with gbr_lib.Renderer(w, h) as r:
+        r.load_scene(s)
+        for frame in range(3):   # without history, then with the CTAs and items the last frame calls for
+            r.set_raster_params(16, (0, 4, 6)[frame])   # a phase below 32: never the small-triangle variant
+            r.render_scene(s)
+            colour, depth = r.readback()
+            assert np.array_equal(r.readback_ids(), o["ids"]), f"frame {frame}: winners differ"
+            assert np.array_equal(depth.view(np.uint32), o["depth"].view(np.uint32)), f"frame {frame}: depth differs"
+            c, oc = colour.astype(np.int64), o["colour"].astype(np.int64)
+            assert max(np.abs(((c >> k) & 255) - ((oc >> k) & 255)).max() for k in (0, 8, 16)) <= 1
+            assert r.stats()["raster_lanes"] == 0
