@@ -502,7 +502,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 }
 
 // Walks the bins of the warp's packed rectangles; called by whole warps of
-// 256-thread blocks (kRowThreads blocks in modes 4 and 5).  The warp's (triangle, bin) pairs are expanded
+// 256-thread blocks.  The warp's (triangle, bin) pairs are expanded
 // load-balanced, 32 consecutive pairs per round: the lane whose pair range
 // covers the round's first pair is found with a ballot, the starts of the
 // other ranges inside the round with one OR-reduction, and a lane's pair
@@ -514,9 +514,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 // Mode 0: count (atomicAdd on the walk's sub-counter of the bin; its return,
 // the pair's rank there, is kept in the walk's rank slots), 1: fill (entry
 // at the sub-counter's list start + rank: no atomics), 2: predicted fill (append within the bin's predicted
-// capacity), 3: pre-pass count (atomicAdd on the first feature slot),
-// 4: count into the block's shared-memory row `s_row` (no return), 5: fill
-// from the block's shared-memory cursors `s_row` (kRowThreads blocks).  A
+// capacity), 3: pre-pass count (atomicAdd on the first feature slot).  A
 // walk is identified by `walk` (its first triangle slot / 32), so the count
 // and fill passes of the same triangles meet the same slots.  One atomic per
 // pair: merging the atomics of same-bin lanes -- every such lane of the warp
@@ -528,10 +526,8 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 constexpr uint32_t kPairsPerLane = GBR_PAIRS_PER_LANE;
 
 template <int MODE>
-__device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t entry, bool valid, uint32_t walk,
-                                         uint32_t* s_row = nullptr) {
-    constexpr uint32_t kWarps = MODE >= 4 ? kRowThreads / 32u : 8u;
-    __shared__ uint4 s_tab[kWarps][32];   // per warp: (first pair, width, bx0 | by0 << 16, entry) of each lane
+__device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t entry, bool valid, uint32_t walk) {
+    __shared__ uint4 s_tab[8][32];   // per warp: (first pair, width, bx0 | by0 << 16, entry) of each lane
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t bx0 = rect.x & 0xFFFFu, bx1 = rect.x >> 16;
     const uint32_t by0 = rect.y & 0xFFFFu, by1 = (rect.y >> 16) & 0x7FFFu;
@@ -594,17 +590,6 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
 #pragma unroll
             for (uint32_t u = 0; u < kPairsPerLane; ++u)
                 if (act[u]) atomicAdd(&F.feat[bin[u]], 1u);
-        } else if (MODE == 4) {
-#pragma unroll
-            for (uint32_t u = 0; u < kPairsPerLane; ++u)
-                if (act[u]) atomicAdd(&s_row[bin[u]], 1u);
-        } else if (MODE == 5) {
-            uint32_t pos[kPairsPerLane];
-#pragma unroll
-            for (uint32_t u = 0; u < kPairsPerLane; ++u) pos[u] = act[u] ? atomicAdd(&s_row[bin[u]], 1u) : 0u;
-#pragma unroll
-            for (uint32_t u = 0; u < kPairsPerLane; ++u)
-                if (act[u]) F.list[pos[u]] = ent[u];
         } else if (MODE == 0) {
             // count, keeping the pair's rank within its bin (slots past the
             // storage are dropped: that frame overflows and is not filled)
@@ -638,6 +623,144 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
         }
     }
     __syncwarp();   // the warp's table row is rewritten by its next walk
+}
+
+// Counts a rectangle of bins in the block's shared-memory row (nbx x nby
+// words) as a difference: one at its first bin, less one past its last
+// column and row, one past both.  prefix_2d() of the finished row gives
+// every bin's count.  Four shared-memory adds a triangle, whatever its
+// bins: enumerating the (triangle, bin) pairs for this took most of the
+// count pass (1M soup, 8 pairs a triangle: setup 65.6 -> 37.6 us).
+__device__ __forceinline__ void count_rect(uint32_t* row, uint2 rect, uint32_t nbx, uint32_t nby) {
+    const uint32_t bx0 = rect.x & 0xFFFFu, bx1 = rect.x >> 16;
+    const uint32_t by0 = rect.y & 0xFFFFu, by1 = (rect.y >> 16) & 0x7FFFu;
+    if (bx0 > bx1 || by0 > by1) return;
+    uint32_t* const top = row + by0 * nbx;
+    atomicAdd(&top[bx0], 1u);
+    if (bx1 + 1u < nbx) atomicSub(&top[bx1 + 1u], 1u);
+    if (by1 + 1u < nby) {
+        uint32_t* const below = row + (by1 + 1u) * nbx;
+        atomicSub(&below[bx0], 1u);
+        if (bx1 + 1u < nbx) atomicAdd(&below[bx1 + 1u], 1u);
+    }
+}
+
+// Inclusive prefix sums of the row's nbx x nby words over x, then over y, by
+// the whole block (kRowThreads): a warp per grid row, then a thread per
+// column and segment of grid rows.
+__device__ __forceinline__ void prefix_2d(uint32_t* row, uint32_t nbx, uint32_t nby) {
+    __shared__ uint32_t s_seg[kRowThreads];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    for (uint32_t y = warp; y < nby; y += kRowThreads / 32u) {
+        uint32_t carry = 0;
+        for (uint32_t x0 = 0; x0 < nbx; x0 += 32u) {
+            const uint32_t x = x0 + lane;
+            uint32_t v = x < nbx ? row[y * nbx + x] : 0u;
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, v, d);
+                if (lane >= d) v += t;
+            }
+            v += carry;
+            if (x < nbx) row[y * nbx + x] = v;
+            carry = __shfl_sync(0xFFFFFFFFu, v, 31);
+        }
+    }
+    __syncthreads();
+    if (nbx >= kRowThreads) {   // a thread per column
+        for (uint32_t x = tid; x < nbx; x += kRowThreads) {
+            uint32_t sum = 0;
+            for (uint32_t y = 0; y < nby; ++y) row[y * nbx + x] = sum += row[y * nbx + x];
+        }
+        __syncthreads();
+        return;
+    }
+    const uint32_t segs = kRowThreads / nbx, rows = (nby + segs - 1u) / segs;
+    const uint32_t seg = tid / nbx, x = tid - seg * nbx;
+    const uint32_t y0 = min(seg * rows, nby), y1 = seg < segs ? min(y0 + rows, nby) : y0;
+    uint32_t sum = 0;
+#pragma unroll 4
+    for (uint32_t y = y0; y < y1; ++y) row[y * nbx + x] = sum += row[y * nbx + x];
+    s_seg[tid] = sum;
+    __syncthreads();
+    sum = 0;
+    for (uint32_t s = 0; s < seg && seg < segs; ++s) sum += s_seg[s * nbx + x];
+    if (sum)
+#pragma unroll 4
+        for (uint32_t y = y0; y < y1; ++y) row[y * nbx + x] += sum;
+    __syncthreads();
+}
+
+// Fill from the block's shared-memory cursors (kRowThreads blocks): the
+// entry of each of the warp's rectangles goes to the next slot of every bin
+// it covers.  The warp's pairs are cut into 32 runs of consecutive pairs, a
+// lane each: a lane finds its first pair's rectangle once and then steps
+// from bin to bin (finding every pair's rectangle anew, 32 consecutive pairs
+// a round, cost about four times the instructions: 1M soup fill 49 -> 30
+// us).  Lanes sit in different rectangles, so their shared-memory cursors
+// rarely meet, and a store goes to a sector of its own either way.
+__device__ __forceinline__ void fill_walk(const FrameDev& F, uint2 rect, uint32_t entry, uint32_t* cursor) {
+    __shared__ uint4 s_tab[kRowThreads / 32u][32];   // the warp's non-empty rectangles: first pair, first bin, w | h << 16, entry
+    const uint32_t lane = threadIdx.x & 31u;
+    uint4* const tab = s_tab[threadIdx.x >> 5];
+    const uint32_t bx0 = rect.x & 0xFFFFu, bx1 = rect.x >> 16;
+    const uint32_t by0 = rect.y & 0xFFFFu, by1 = (rect.y >> 16) & 0x7FFFu;
+    uint32_t w = 0, h = 0;
+    if (bx0 <= bx1 && by0 <= by1) {
+        w = bx1 - bx0 + 1u;
+        h = by1 - by0 + 1u;
+    }
+    const uint32_t n = w * h;
+    uint32_t incl = n;   // inclusive prefix of pair counts over the warp
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += t;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    if (total == 0u) return;   // warp-uniform
+    const uint32_t some = __ballot_sync(0xFFFFFFFFu, n != 0u), rects = (uint32_t)__popc(some);
+    if (n) tab[__popc(some & ((1u << lane) - 1u))] = make_uint4(incl - n, by0 * F.nbx + bx0, w | (h << 16), entry);
+    __syncwarp();
+    // the lane's run: total / 32 pairs, one more in the first total % 32 lanes
+    const uint32_t each = total >> 5, rest = total & 31u;
+    const uint32_t first = lane * each + min(lane, rest), count = each + (lane < rest ? 1u : 0u);
+    uint32_t o = 0;   // the last rectangle that starts at or before the run
+#pragma unroll
+    for (uint32_t s = 16; s > 0; s >>= 1)
+        if (o + s < rects && tab[o + s].x <= first) o += s;
+    uint4 d = tab[o];
+    uint32_t wide = d.z & 0xFFFFu, x = first - d.x;
+    uint32_t left = wide * (d.z >> 16) - x;   // the rectangle's pairs from here on
+    const uint32_t y = x / wide;
+    x -= y * wide;
+    uint32_t bin = d.y + y * F.nbx + x;
+    for (uint32_t k = 0; k < count; k += kPairsPerLane) {
+        uint32_t pos[kPairsPerLane], ent[kPairsPerLane];
+#pragma unroll
+        for (uint32_t u = 0; u < kPairsPerLane; ++u) {
+            if (k + u >= count) break;
+            pos[u] = atomicAdd(&cursor[bin], 1u);
+            ent[u] = d.w;
+            ++x;
+            ++bin;
+            if (--left == 0u) {
+                o = min(o + 1u, rects - 1u);
+                d = tab[o];
+                wide = d.z & 0xFFFFu;
+                left = wide * (d.z >> 16);
+                bin = d.y;
+                x = 0;
+            } else if (x == wide) {
+                x = 0;
+                bin += F.nbx - wide;
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kPairsPerLane; ++u)
+            if (k + u < count) F.list[pos[u]] = ent[u];
+    }
+    __syncwarp();   // the warp's table is rewritten by its next walk
 }
 
 }  // namespace gbr

@@ -169,7 +169,7 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
     const uint32_t counts = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, visible)) |
                             ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, fpath)) << 16);
     if (MODE == 0) bin_walk<0>(F, rect, 0u, visible, walk);
-    else if (MODE == 2) bin_walk<4>(F, rect, 0u, visible, walk, s_row);
+    else if (MODE == 2) count_rect(s_row, visible ? rect : empty_rect(), F.nbx, F.nby);
     else bin_walk<2>(F, rect, prim | (no_raster ? kNoRasterBit : 0u), visible, walk);
     return counts;
 }
@@ -235,6 +235,32 @@ __global__ void __launch_bounds__(256) fill_kernel(FrameDev F) {
 // sweep at different bins, so the blocks' atomics on one bin do not arrive
 // together); the run's start, relative to the bin, goes to the block's row
 // of F.row_base.
+
+// One run per bin the block touched: an atomic on the bin's counter each,
+// `done(bin, count, start)` with its return.  Blocks start their sweep at
+// different bins, and a thread's atomics are issued back to back.
+template <typename Done>
+__device__ __forceinline__ void reserve_runs(const uint32_t* counts, uint32_t nb, uint32_t* to, Done done) {
+    const uint32_t shift = (uint32_t)(((unsigned long long)blockIdx.x * nb) / gridDim.x);
+    for (uint32_t i0 = 0; i0 < nb; i0 += 8u * kRowThreads) {
+        uint32_t bb[8], cc[8], rr[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; ++u) {
+            const uint32_t i = i0 + u * kRowThreads + threadIdx.x;
+            uint32_t b = i + shift;
+            if (b >= nb) b -= nb;
+            bb[u] = b;
+            cc[u] = i < nb ? counts[b] : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; ++u)
+            if (cc[u]) rr[u] = atomicAdd(&to[bb[u]], cc[u]);
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; ++u)
+            if (cc[u]) done(bb[u], cc[u], rr[u]);
+    }
+}
+
 __global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F) {
     extern __shared__ uint32_t s_row[];
     pdl_wait();
@@ -255,14 +281,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F) 
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < F.touch_words; w += gridDim.x * blockDim.x)
         zero_to[w] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
+    prefix_2d(s_row, F.nbx, F.nby);
     uint32_t* const row = F.row_base + (size_t)blockIdx.x * nb;
-    const uint32_t shift = (uint32_t)(((unsigned long long)blockIdx.x * nb) / gridDim.x);
-    for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) {
-        uint32_t b = i + shift;
-        if (b >= nb) b -= nb;
-        const uint32_t c = s_row[b];
-        if (c) row[b] = atomicAdd(&F.counts[b], c);
-    }
+    reserve_runs(s_row, nb, F.counts, [&](uint32_t b, uint32_t, uint32_t at) { row[b] = at; });
     add_block_stats(F.ctl, vis, fp);
     pdl_release();
 }
@@ -284,7 +305,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
         const bool in_range = prim < F.num_tris;
         const uint2 rect = in_range ? F.rects[prim] : empty_rect();
         const uint32_t entry = prim | ((rect.y & 0x80000000u) ? kNoRasterBit : 0u);
-        bin_walk<5>(F, rect, entry, in_range, prim >> 5, s_row);
+        fill_walk(F, rect, entry, s_row);
     }
     pdl_release();
 }
@@ -317,32 +338,14 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
         fp += c >> 16;
     }
     __syncthreads();
-    // one run per bin the block touched (blocks start their sweep at
-    // different bins); a thread's atomics are issued back to back
-    const uint32_t shift = (uint32_t)(((unsigned long long)blockIdx.x * nb) / gridDim.x);
-    for (uint32_t i0 = 0; i0 < nb; i0 += 8u * kRowThreads) {
-        uint32_t bb[8], cc[8], rr[8];
-#pragma unroll
-        for (uint32_t u = 0; u < 8u; ++u) {
-            const uint32_t i = i0 + u * kRowThreads + tid;
-            uint32_t b = i + shift;
-            if (b >= nb) b -= nb;
-            bb[u] = b;
-            cc[u] = i < nb ? s_row[b] : 0u;
+    prefix_2d(s_row, F.nbx, F.nby);
+    reserve_runs(s_row, nb, F.cursors, [&](uint32_t b, uint32_t c, uint32_t at) {
+        if ((unsigned long long)at + c > __ldg(&F.bin_end[b])) {
+            s_ovf = 1u;
+            atomicOr(&F.ctl->pred_overflow, 1u);
         }
-#pragma unroll
-        for (uint32_t u = 0; u < 8u; ++u)
-            if (cc[u]) rr[u] = atomicAdd(&F.cursors[bb[u]], cc[u]);
-#pragma unroll
-        for (uint32_t u = 0; u < 8u; ++u) {
-            if (!cc[u]) continue;
-            if ((unsigned long long)rr[u] + cc[u] > __ldg(&F.bin_end[bb[u]])) {
-                s_ovf = 1u;
-                atomicOr(&F.ctl->pred_overflow, 1u);
-            }
-            s_row[bb[u]] = rr[u];
-        }
-    }
+        s_row[b] = at;
+    });
     __syncthreads();
     if (!s_ovf) {
         for (uint32_t base = blockIdx.x * kRowThreads; base < F.num_tris; base += gridDim.x * kRowThreads) {
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
             const bool in_range = prim < F.num_tris;
             const uint2 rect = in_range ? F.rects[prim] : empty_rect();
             const uint32_t entry = prim | ((rect.y & 0x80000000u) ? kNoRasterBit : 0u);
-            bin_walk<5>(F, rect, entry, in_range, prim >> 5, s_row);
+            fill_walk(F, rect, entry, s_row);
         }
     }
     add_block_stats(F.ctl, vis, fp);
