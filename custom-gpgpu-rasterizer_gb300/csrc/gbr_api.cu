@@ -286,6 +286,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     }
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;
+    if (md.size() == 1u) F.one = flat_mesh(md[0]);
     F.setup = r->d_setup; F.rects = r->d_rects; F.keys = r->d_keys;
     F.counts = r->d_counts; F.sub_base = r->d_sub_base; F.count_stride = nb; F.offsets = r->d_offsets;
     F.cursors = r->d_cursors; F.capacity = r->d_capacity;

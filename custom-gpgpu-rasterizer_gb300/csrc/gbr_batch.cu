@@ -68,7 +68,7 @@ struct gbr_batch {
     uint32_t* d_counts = nullptr;     // kCountSplit x bins
     uint32_t* d_sub_base = nullptr;   // kCountSplit x bins
     uint32_t count_split = 1;         // sub-counters per bin in use
-    uint32_t all_flat = 0;            // every scene shades flat (the captured shade variant)
+    uint32_t all_flat = 0;            // BatchDev::all_flat (the captured shade variant)
     uint32_t* d_offsets = nullptr;
     uint32_t* d_cursors = nullptr;
     ScanState* d_scan = nullptr;   // bin scan state (zeroed once)
@@ -192,7 +192,7 @@ gbr_status ensure_layout(gbr_batch* b) {
         tris += L.tris;
         meshes += L.num_meshes;
         tri_blocks += ceil_div(L.tris, 256u);
-        px_blocks += ceil_div((uint64_t)L.W * L.H, 256u);
+        px_blocks += (uint64_t)ceil_div(L.W, kTileW) * ceil_div(L.H, kTileH);
     }
     tables[n] = (uint32_t)tri_blocks;
     tables[(n + 1u) + n] = (uint32_t)px_blocks;
@@ -276,6 +276,7 @@ void build_table(gbr_batch* b, std::vector<unsigned char>& out) {
         F.phase = b->cfg.raster_phase;
         F.raster_ctas = b->cfg.raster_ctas;
         F.meshes = d_meshes + L.mesh_base;
+        if (L.num_meshes == 1u) F.one = flat_mesh(meshes[L.mesh_base]);
         F.setup = b->d_setup + L.tri_base;
         F.rects = b->d_rects + L.tri_base;
         F.keys = b->d_keys + L.tri_base;
@@ -366,9 +367,11 @@ gbr_status render_batch(gbr_batch* b, cudaStream_t s) {
     std::vector<unsigned char> table;
     build_table(b, table);
     // the shade pass's variant lives in the graph: a change is captured anew
-    uint32_t all_flat = 1u;
-    for (size_t i = 0; i < b->members.size(); ++i)
-        all_flat &= reinterpret_cast<const FrameDev*>(table.data())[i].flat_shade;
+    uint32_t all_flat = 2u;
+    for (size_t i = 0; i < b->members.size(); ++i) {
+        const FrameDev& F = reinterpret_cast<const FrameDev*>(table.data())[i];
+        all_flat = std::min(all_flat, !F.flat_shade ? 0u : F.one.vertices ? 2u : 1u);
+    }
     if (all_flat != b->all_flat) {
         b->all_flat = all_flat;
         drop_graph(b);

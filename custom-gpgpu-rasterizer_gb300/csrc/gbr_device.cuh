@@ -75,6 +75,12 @@ __host__ __device__ inline bool use_count_rows(unsigned long long pairs, uint32_
     return bins > 0u && bins <= kMaxRowBins && blocks > 0u && pairs >= (unsigned long long)bins * blocks;
 }
 
+// The shade passes' blocks of 256 threads cover tiles of kTileW x kTileH
+// pixels, each warp 8x4 of the upper half and 8x4 of the lower: fewer
+// triangles to a warp than in 32 pixels of a row, and every 32-byte sector of
+// the outputs still written whole.
+constexpr uint32_t kTileW = 32, kTileH = 16;
+
 enum : uint32_t { kVertexIVertex56 = 0, kVertexPos3Rgba8 = 1 };
 
 struct TexDev {
@@ -98,6 +104,19 @@ struct MeshDev {
     float world[16];
     TexDev tex[4];
 };
+
+// What flat shading needs of a mesh: its vertices and the row of its matrix
+// that gives the clip w.  A frame of one mesh carries it in its descriptor.
+struct FlatMesh {
+    const void* vertices;
+    const uint32_t* indices;   // null: non-indexed list
+    uint32_t vertex_format;
+    uint32_t topology;
+    float w[4];
+};
+__host__ __device__ inline FlatMesh flat_mesh(const MeshDev& m) {
+    return FlatMesh{m.vertices, m.indices, m.vertex_format, m.topology, {m.wvp[3], m.wvp[7], m.wvp[11], m.wvp[15]}};
+}
 
 // A scene light (the build's shading extension; gbr_light in gbr.h).
 constexpr uint32_t kMaxLights = 8;
@@ -141,7 +160,7 @@ struct Ctl {
 static_assert(sizeof(Ctl) == 64, "control block is 64 bytes");
 
 // Everything a kernel of the frame needs, passed by value.
-struct FrameDev {
+struct __align__(16) FrameDev {
     uint32_t width, height;
     uint32_t nbx, nby, bw, bh, num_bins;
     uint32_t cull, sample, vis, clear_colour32;
@@ -218,6 +237,7 @@ struct FrameDev {
     // pixels already hold the clear values.  (null: every pixel is written)
     uint8_t* dirty_rd;
     uint8_t* dirty_wr;
+    FlatMesh one;              // flat-shaded frames of one mesh: that mesh
 };
 static_assert(sizeof(FrameDev) % 16 == 0, "frame descriptors are copied as 16-byte words");
 
@@ -287,14 +307,14 @@ struct BatchDev {
     const uint32_t* px_blocks;    // num_scenes + 1
     const uint32_t* bin_base;     // num_scenes + 1
     const uint32_t* tri_scene;    // per triangle-pass block: its scene
-    const uint32_t* px_scene;     // per pixel-pass block: its scene
+    const uint32_t* px_scene;     // per pixel-pass block (a tile of kTileW x kTileH pixels): its scene
     const uint32_t* bin_scene;    // per global bin: its scene
     uint4* items;                 // (global bin, list start, count, chunks of the bin)
     Ctl* ctl;                     // the batch's list/item allocation, work queue and overflow flag
     unsigned long long list_cap;
     uint32_t items_cap;
     uint32_t num_scenes;
-    uint32_t all_flat;            // every scene shades flat: the shade pass runs its flat variant
+    uint32_t all_flat;            // every scene shades flat (1), from one mesh (2): the shade pass runs that variant
     uint32_t stage;               // raster pass size (FrameDev::stage)
 };
 
@@ -316,11 +336,8 @@ __device__ __forceinline__ int cvt_s16(float x) {
     return __float2int_rz(x);
 }
 
-__device__ __forceinline__ uint32_t cvt_u8(float x) {
-    if (!(x > 0.0f)) return 0u;
-    if (x >= 255.0f) return 255u;
-    return (uint32_t)__float2int_rz(x);
-}
+// (cvt.rzi.u32 clamps negative values and NaN to 0)
+__device__ __forceinline__ uint32_t cvt_u8(float x) { return min(__float2uint_rz(x), 255u); }
 
 __device__ __forceinline__ float M4(const float* m, int r, int c) { return m[c * 4 + r]; }
 
@@ -373,7 +390,8 @@ __device__ __forceinline__ F3 fetch_position(const MeshDev& m, uint32_t vi) {
 // Triangle assembly (TA_Kernel, CUDARenderer.cu:716-753); strips use the
 // intended order (the reference's strip branch reads an uninitialised
 // triangle).
-__device__ __forceinline__ void tri_vertex_ids(const MeshDev& m, uint32_t local, uint32_t v[3]) {
+template <typename Mesh>   // MeshDev or FlatMesh
+__device__ __forceinline__ void tri_vertex_ids(const Mesh& m, uint32_t local, uint32_t v[3]) {
     if (!m.indices) {
         v[0] = 3u * local; v[1] = 3u * local + 1u; v[2] = 3u * local + 2u;
     } else if (m.topology == 0u) {
@@ -630,7 +648,7 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
 // column and row, one past both.  prefix_2d() of the finished row gives
 // every bin's count.  Four shared-memory adds a triangle, whatever its
 // bins: enumerating the (triangle, bin) pairs for this took most of the
-// count pass (1M soup, 8 pairs a triangle: setup 65.6 -> 37.6 us).
+// count pass (1M soup, 8 pairs a triangle: setup 65.6 -> 41.5 us).
 __device__ __forceinline__ void count_rect(uint32_t* row, uint2 rect, uint32_t nbx, uint32_t nby) {
     const uint32_t bx0 = rect.x & 0xFFFFu, bx1 = rect.x >> 16;
     const uint32_t by0 = rect.y & 0xFFFFu, by1 = (rect.y >> 16) & 0x7FFFu;
@@ -696,9 +714,10 @@ __device__ __forceinline__ void prefix_2d(uint32_t* row, uint32_t nbx, uint32_t 
 // it covers.  The warp's pairs are cut into 32 runs of consecutive pairs, a
 // lane each: a lane finds its first pair's rectangle once and then steps
 // from bin to bin (finding every pair's rectangle anew, 32 consecutive pairs
-// a round, cost about four times the instructions: 1M soup fill 49 -> 30
-// us).  Lanes sit in different rectangles, so their shared-memory cursors
-// rarely meet, and a store goes to a sector of its own either way.
+// a round, cost about three times the instructions).  Lanes sit in different
+// rectangles, so their shared-memory cursors rarely meet, and a store goes
+// to a sector of its own either way: 8M of them bound the pass, whose time
+// stayed (50 us).
 __device__ __forceinline__ void fill_walk(const FrameDev& F, uint2 rect, uint32_t entry, uint32_t* cursor) {
     __shared__ uint4 s_tab[kRowThreads / 32u][32];   // the warp's non-empty rectangles: first pair, first bin, w | h << 16, entry
     const uint32_t lane = threadIdx.x & 31u;

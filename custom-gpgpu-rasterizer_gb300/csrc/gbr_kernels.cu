@@ -570,7 +570,14 @@ __device__ __forceinline__ void clear_pixel(const FrameDev& F, size_t gi) {
     F.ids[gi] = kInvalidPrim;
 }
 
-template <bool FLAT>
+// How a pass shades its winners: through the whole vertex stage and shader,
+// from vertex colours (the winner's mesh looked up, or the frame's only one),
+// or by depth.
+enum ShadeKind { kShadeFull, kShadeFlat, kShadeFlatOne, kShadeDepth };
+
+// Pixel (x, y) with raster result v: the winner's weights and depth as the
+// raster computed them, its colour, and the three outputs.
+template <ShadeKind KIND>
 __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, unsigned long long v) {
     const size_t gi = (size_t)y * F.width + (size_t)x;
     if (v == kEmptyVis) {
@@ -578,7 +585,7 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
         return;
     }
     const uint32_t prim = (uint32_t)(v & 0xFFFFFFFFull);
-    const uint4* rp = reinterpret_cast<const uint4*>(F.setup) + 3u * prim;
+    const uint4* rp = reinterpret_cast<const uint4*>(F.setup) + 3u * (size_t)prim;
     const uint4 a = __ldg(rp), b = __ldg(rp + 1), c = __ldg(rp + 2);
     TriSetup t;
     t.x0 = __uint_as_float(a.x); t.y0 = __uint_as_float(a.y); t.x1 = __uint_as_float(a.z); t.y1 = __uint_as_float(a.w);
@@ -588,8 +595,14 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
     if (t.flags & kFlagFloat) weights_float(t, (float)x, (float)y, w);
     else weights_fixed(t, x, y, w);
     const float z = interp_z(w[0], w[1], w[2], t.z0, t.z1, t.z2);
-    const MeshDev& m = F.meshes[t.mesh];
-    F.colour[gi] = shade_fragment<FLAT>(F, m, prim, w, z);
+    if (KIND == kShadeFlatOne) {   // needs no mesh lookup: the vertices load beside the record
+        F.colour[gi] = shade_flat(F.one, prim, w);
+    } else if (KIND == kShadeDepth) {
+        F.colour[gi] = shade_depth(z);
+    } else {
+        const MeshDev& m = F.meshes[t.mesh];
+        F.colour[gi] = KIND == kShadeFlat ? shade_flat(flat_mesh(m), prim - m.prim_base, w) : shade_fragment(F, m, prim, w, z);
+    }
     F.depth[gi] = z;
     F.ids[gi] = prim;
 }
@@ -816,23 +829,42 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
     }
 }
 
-// Shades pixel i of the frame: the winner the raster left in the merge
-// buffer (or the clear colour), and leaves the buffer empty for the next
-// frame.
-template <bool FLAT>
-__device__ __forceinline__ void shade_px(const FrameDev& F, uint32_t i) {
-    const unsigned long long v = F.gvis[i];
-    if (v != kEmptyVis) F.gvis[i] = kEmptyVis;
-    resolve_pixel<FLAT>(F, (int)(i % F.width), (int)(i / F.width), v);
+// Shades the thread's two pixels of tile (tx, ty), above row y1: the winners
+// the raster left in the merge buffer (or the clear colour), and leaves the
+// buffer empty for the next frame.  Both merge words are loaded before
+// either pixel is shaded: the pass waits on the chain merge word -> record
+// and vertices (2M soup at 4K: one pixel a thread 96 us, two 92, two with
+// eight blocks an SM 82).
+template <ShadeKind KIND>
+__device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint32_t ty, uint32_t y1) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint32_t x = tx * kTileW + (warp & 3u) * 8u + (lane & 7u);
+    const uint32_t y = ty + (warp >> 2) * 4u + (lane >> 3);
+    if (x >= F.width) return;
+    unsigned long long v[2];
+#pragma unroll
+    for (uint32_t k = 0; k < 2u; ++k) {
+        const uint32_t yk = y + k * (kTileH / 2u);
+        v[k] = yk < y1 ? F.gvis[(size_t)yk * F.width + x] : kEmptyVis;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 2u; ++k) {
+        const uint32_t yk = y + k * (kTileH / 2u);
+        if (yk >= y1) break;
+        if (v[k] != kEmptyVis) F.gvis[(size_t)yk * F.width + x] = kEmptyVis;
+        resolve_pixel<KIND>(F, (int)x, (int)yk, v[k]);
+    }
 }
 
-// One thread per pixel.
-template <bool FLAT>
-__global__ void __launch_bounds__(256) shade_kernel(FrameDev F) {
+// One-pass shading: a block per tile, pixel rows [y0, y1).  With the mesh in
+// the descriptor, colours converted without a table, reciprocals for
+// divisions and 8x4 pixels to a warp, 2M soup at 4K 108 -> 82 us.
+template <ShadeKind KIND>
+__global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : KIND == kShadeFlat ? 6 : 8) shade_kernel(FrameDev F, uint32_t y0,
+                                                                                                      uint32_t y1) {
     pdl_wait();
-    const uint32_t i = F.px_begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (F.px_end ? F.px_end : F.width * F.height) || F.ctl->overflow) return;
-    shade_px<FLAT>(F, i);
+    if (F.ctl->overflow) return;
+    shade_tile<KIND>(F, blockIdx.x, y0 + blockIdx.y * kTileH, y1);
 }
 
 // Two-pass shading, for frames that shade through the full vertex stage
@@ -958,7 +990,7 @@ __global__ void __launch_bounds__(256, 4) shade_list_kernel(FrameDev F) {
         const uint32_t i = __ldg(F.shade_list + j);
         const unsigned long long v = F.gvis[i];
         F.gvis[i] = kEmptyVis;
-        resolve_pixel<false>(F, (int)(i % F.width), (int)(i / F.width), v);
+        resolve_pixel<kShadeFull>(F, (int)(i % F.width), (int)(i / F.width), v);
     }
 }
 
@@ -1044,23 +1076,28 @@ __global__ void __launch_bounds__(256) batch_fill_kernel(BatchDev B) {
     fill_tri(sF, (blockIdx.x - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x, (blockIdx.x * 256u + threadIdx.x) >> 5);
 }
 
-// ALL_FLAT: every scene of the batch shades flat (B.all_flat), and the
-// kernel holds only the flat path's registers (40 against 80: twice the
-// resident warps for a batch of vertex-coloured soups).
-template <bool ALL_FLAT>
-__global__ void __launch_bounds__(256) batch_shade_kernel(BatchDev B, uint32_t chunks, uint32_t per) {
+// KIND: every scene of the batch shades flat (B.all_flat), from one mesh, and
+// the kernel holds only that path's registers; kShadeFull: each scene its own
+// way.
+template <ShadeKind KIND>
+__global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : 6) batch_shade_kernel(BatchDev B, uint32_t chunks, uint32_t per) {
     if (B.ctl->overflow) return;
     __shared__ __align__(16) FrameDev sF;
     const uint32_t c0 = blockIdx.x * per, c1 = min(c0 + per, chunks);
-    uint32_t loaded = 0xFFFFFFFFu;
+    uint32_t loaded = 0xFFFFFFFFu, tx = 0, ty = 0;
     for (uint32_t v = c0; v < c1; ++v) {
         const uint32_t sc = __ldg(B.px_scene + v);
-        enter_scene(B, sc, loaded, sF);
-        const uint32_t i = (v - __ldg(B.px_blocks + sc)) * 256u + threadIdx.x;
-        if (i >= sF.width * sF.height) continue;
-        if (ALL_FLAT) shade_px<true>(sF, i);
-        else if (sF.flat_shade) shade_px<true>(sF, i);
-        else shade_px<false>(sF, i);
+        if (enter_scene(B, sc, loaded, sF)) {
+            const uint32_t tile = v - __ldg(B.px_blocks + sc), across = (sF.width + kTileW - 1u) / kTileW;
+            ty = tile / across;
+            tx = tile - ty * across;
+        } else if (++tx * kTileW >= sF.width) {   // a range's tiles follow one another
+            tx = 0;
+            ++ty;
+        }
+        if (KIND != kShadeFull) shade_tile<KIND>(sF, tx, ty * kTileH, sF.height);
+        else if (sF.flat_shade) shade_tile<kShadeFlat>(sF, tx, ty * kTileH, sF.height);
+        else shade_tile<kShadeFull>(sF, tx, ty * kTileH, sF.height);
     }
 }
 
@@ -1171,9 +1208,9 @@ cudaError_t launch_raster(const FrameDev& F, const RasterGrid& per_sm, cudaStrea
 }
 
 cudaError_t launch_shade(const FrameDev& F, cudaStream_t s) {
-    const uint32_t npx = (F.px_end ? F.px_end : F.width * F.height) - F.px_begin;
-    const dim3 g((npx + 255u) / 256u), b(256);
+    const dim3 b(256);
     if (!F.flat_shade && F.shade_list) {
+        const uint32_t npx = (F.px_end ? F.px_end : F.width * F.height) - F.px_begin;
         const cudaError_t e = launch_pdl(shade_queue_kernel, dim3((npx + 1023u) / 1024u), b, 0, s, F);
         if (e != cudaSuccess) return e;
         // one resident wave: the queue is a few pixels per thread at most
@@ -1185,7 +1222,13 @@ cudaError_t launch_shade(const FrameDev& F, cudaStream_t s) {
         }
         return launch_pdl(shade_list_kernel, dim3((uint32_t)std::max(per_sm, 1) * (uint32_t)sm_count()), b, 0, s, F);
     }
-    return F.flat_shade ? launch_pdl(shade_kernel<true>, g, b, 0, s, F) : launch_pdl(shade_kernel<false>, g, b, 0, s, F);
+    const uint32_t y0 = F.row1 ? F.row0 * F.bh : 0u, y1 = F.row1 ? std::min(F.row1 * F.bh, F.height) : F.height;
+    if (y0 >= y1) return cudaSuccess;   // a band below the screen
+    const dim3 g((F.width + kTileW - 1u) / kTileW, (y1 - y0 + kTileH - 1u) / kTileH);
+    if (F.flat_shade && F.one.vertices) return launch_pdl(shade_kernel<kShadeFlatOne>, g, b, 0, s, F, y0, y1);
+    if (F.flat_shade) return launch_pdl(shade_kernel<kShadeFlat>, g, b, 0, s, F, y0, y1);
+    if (F.vis == 1u) return launch_pdl(shade_kernel<kShadeDepth>, g, b, 0, s, F, y0, y1);
+    return launch_pdl(shade_kernel<kShadeFull>, g, b, 0, s, F, y0, y1);
 }
 
 cudaError_t launch_batch(const BatchDev& B, const BatchLaunch& L, cudaStream_t s) {
@@ -1206,8 +1249,9 @@ cudaError_t launch_batch(const BatchDev& B, const BatchLaunch& L, cudaStream_t s
     e = launch_block_raster(none, B, true, L.raster_threads, L.raster_ctas, L.bin_w, L.bin_h, L.raster_grid, s);
     if (e != cudaSuccess) return e;
     if (L.px_blocks) {
-        if (B.all_flat) batch_shade_kernel<true><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
-        else batch_shade_kernel<false><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
+        if (B.all_flat == 2u) batch_shade_kernel<kShadeFlatOne><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
+        else if (B.all_flat) batch_shade_kernel<kShadeFlat><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
+        else batch_shade_kernel<kShadeFull><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
     }
     return cudaGetLastError();
 }

@@ -207,6 +207,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     mat4_mul(cam->proj, cam->view, vp);
     mat4_mul(vp, world, desc.wvp);
     memcpy(desc.world, world, sizeof desc.world);
+    F.one = flat_mesh(desc);
 
     cudaStream_t s = (cudaStream_t)stream;
     noalloc_prepare_kernel<<<256, 256, 0, s>>>(F, desc, (uint32_t)npx);

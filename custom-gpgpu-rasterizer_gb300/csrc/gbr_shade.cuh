@@ -13,17 +13,16 @@
 
 namespace gbr {
 
-// b / 255 for every byte value b, each the correctly rounded quotient
-// (evaluated at compile time in single precision): the RGBA8 vertex colours
-// read as GetRGBColor (RGBRaw.h:34-38) divides, without a division per use
-// (a product with 1/255 differs in 126 of the 256 values).
-struct ByteOver255 {
-    float v[256];
-    constexpr ByteOver255() : v() {
-        for (int b = 0; b < 256; ++b) v[b] = (float)b / 255.0f;
-    }
-};
-__device__ constexpr ByteOver255 kByteOver255{};
+// b / 255 for a byte value b, correctly rounded: the RGBA8 vertex colours and
+// texels read as GetRGBColor (RGBRaw.h:34-38) divides.  The quotient estimate
+// is corrected by its exact residual (Markstein); a product with 1/255 alone
+// differs in 126 of the 256 values, this in none.  Four operations and no
+// load: a table of the quotients cost a pixel nine scattered loads.
+__device__ __forceinline__ float over255(uint32_t b) {
+    const float x = (float)b, inv = 1.0f / 255.0f;
+    const float q = __fmul_rn(x, inv);
+    return __fmaf_rn(__fmaf_rn(-255.0f, q, x), inv, q);
+}
 
 struct OVtx {
     float px, py, pz, pw;  // NDC xyz, clip w
@@ -40,9 +39,9 @@ __device__ __forceinline__ void fetch_full(const MeshDev& m, uint32_t vi, float 
 #pragma unroll
         for (int k = 3; k < 11; ++k) iv[k] = 0.f;
         // GetRGBColor (RGBRaw.h:34-38): r = byte0 / 255
-        iv[11] = kByteOver255.v[rgba & 0xFFu];
-        iv[12] = kByteOver255.v[(rgba >> 8) & 0xFFu];
-        iv[13] = kByteOver255.v[(rgba >> 16) & 0xFFu];
+        iv[11] = over255(rgba & 0xFFu);
+        iv[12] = over255((rgba >> 8) & 0xFFu);
+        iv[13] = over255((rgba >> 16) & 0xFFu);
     } else {
         const float2* b = reinterpret_cast<const float2*>(reinterpret_cast<const float*>(m.vertices) + 14u * (size_t)vi);
 #pragma unroll
@@ -75,7 +74,7 @@ __device__ __forceinline__ OVtx vertex_stage(const MeshDev& m, const FrameDev& F
 }
 
 __device__ __forceinline__ F3 rgb_of(uint32_t c) {   // byte / 255 per channel
-    return f3(kByteOver255.v[c & 0xFFu], kByteOver255.v[(c >> 8) & 0xFFu], kByteOver255.v[(c >> 16) & 0xFFu]);
+    return f3(over255(c & 0xFFu), over255((c >> 8) & 0xFFu), over255((c >> 16) & 0xFFu));
 }
 
 // SamplePoint (CUDATextureSampler.cuh:87-104): u = int(uv.x*w + 0.5);
@@ -258,43 +257,55 @@ __device__ __forceinline__ F3 shade_pixel_safe(const FrameDev& F, const MeshDev&
     return fc;
 }
 
-// Colour of the fragment of primitive `prim` at pixel (x, y) with weights w.
-// FLAT: the frame is known to shade every pixel from vertex colours (PBR
-// view, no mesh with a diffuse map), which keeps the kernel's registers to
-// what that path needs.
-template <bool FLAT>
-__device__ __forceinline__ uint32_t shade_fragment(const FrameDev& F, const MeshDev& m, uint32_t prim,
-                                                   const float w[3], float z) {
-    if (!FLAT && F.vis == 1u) {  // Remap(z, 0.985, 1) * 255 into the blue byte
-        const float rz = __fdiv_rn(__fsub_rn(z, 0.985f), __fsub_rn(1.f, 0.985f));
-        return cvt_u8(__fmul_rn(rz, 255.f)) << 16;
-    }
+// Colour of a fragment shaded from vertex colours (PBR view, no diffuse map):
+// triangle `local` of mesh m, weights w.  The vertex colours are weighted by
+// w / w_clip, not multiplied by the interpolated w (CUDAROPs.cu:379-380); of
+// the vertex stage only each vertex's clip w and colour are needed, the same
+// operations as in vertex_stage.
+__device__ __forceinline__ uint32_t shade_flat(const FlatMesh& m, uint32_t local, const float w[3]) {
     uint32_t vid[3];
-    tri_vertex_ids(m, prim - m.prim_base, vid);
-    if (FLAT || (F.vis == 0u && !m.tex[0].px)) {
-        // untextured: the vertex colours weighted by w / w_clip, not
-        // multiplied by the interpolated w (CUDAROPs.cu:379-380); of the
-        // vertex stage only each vertex's clip w and colour are needed, the
-        // same operations as in vertex_stage
-        float ic[3];
-        F3 col[3];
+    tri_vertex_ids(m, local, vid);
+    float ic[3];
+    F3 col[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            float iv[14];
-            fetch_full(m, vid[k], iv);
-            const float* M = m.wvp;
-            const float cw = __fadd_rn(__fmaf_rn(M4(M, 3, 2), iv[2], __fmaf_rn(M4(M, 3, 0), iv[0], __fmul_rn(M4(M, 3, 1), iv[1]))),
-                                       M4(M, 3, 3));
-            ic[k] = __fdiv_rn(1.f, cw);
-            col[k] = f3(iv[11], iv[12], iv[13]);
+    for (int k = 0; k < 3; ++k) {
+        F3 p;
+        if (m.vertex_format == kVertexPos3Rgba8) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(m.vertices) + vid[k]);
+            const uint32_t rgba = __float_as_uint(v.w);
+            p = f3(v.x, v.y, v.z);
+            col[k] = f3(over255(rgba & 0xFFu), over255((rgba >> 8) & 0xFFu), over255((rgba >> 16) & 0xFFu));
+        } else {
+            const float* b = reinterpret_cast<const float*>(m.vertices) + 14u * (size_t)vid[k];
+            const float2 xy = __ldg(reinterpret_cast<const float2*>(b));
+            const float2 gb = __ldg(reinterpret_cast<const float2*>(b + 12));
+            p = f3(xy.x, xy.y, __ldg(b + 2));
+            col[k] = f3(__ldg(b + 11), gb.x, gb.y);
         }
+        const float cw = __fadd_rn(__fmaf_rn(m.w[2], p.z, __fmaf_rn(m.w[0], p.x, __fmul_rn(m.w[1], p.y))), m.w[3]);
+        ic[k] = __frcp_rn(cw);   // 1 / cw, rounded as the division is
+    }
 #define GBR_CINTERP(a0, a1, a2) \
     __fmaf_rn(w[2], __fmul_rn((a2), ic[2]), __fmaf_rn(w[0], __fmul_rn((a0), ic[0]), __fmul_rn(w[1], __fmul_rn((a1), ic[1]))))
-        const F3 c = f3(GBR_CINTERP(col[0].x, col[1].x, col[2].x), GBR_CINTERP(col[0].y, col[1].y, col[2].y),
-                        GBR_CINTERP(col[0].z, col[1].z, col[2].z));
+    const F3 c = f3(GBR_CINTERP(col[0].x, col[1].x, col[2].x), GBR_CINTERP(col[0].y, col[1].y, col[2].y),
+                    GBR_CINTERP(col[0].z, col[1].z, col[2].z));
 #undef GBR_CINTERP
-        return rgba_from_colour(c);
-    }
+    return rgba_from_colour(c);
+}
+
+// Remap(z, 0.985, 1) * 255 into the blue byte: the depth view.
+__device__ __forceinline__ uint32_t shade_depth(float z) {
+    const float rz = __fdiv_rn(__fsub_rn(z, 0.985f), __fsub_rn(1.f, 0.985f));
+    return cvt_u8(__fmul_rn(rz, 255.f)) << 16;
+}
+
+// Colour of the fragment of primitive `prim` with weights w and depth z.
+__device__ __forceinline__ uint32_t shade_fragment(const FrameDev& F, const MeshDev& m, uint32_t prim,
+                                                   const float w[3], float z) {
+    if (F.vis == 1u) return shade_depth(z);
+    if (F.vis == 0u && !m.tex[0].px) return shade_flat(flat_mesh(m), prim - m.prim_base, w);
+    uint32_t vid[3];
+    tri_vertex_ids(m, prim - m.prim_base, vid);
     const OVtx v0 = vertex_stage(m, F, vid[0]);
     const OVtx v1 = vertex_stage(m, F, vid[1]);
     const OVtx v2 = vertex_stage(m, F, vid[2]);
@@ -305,12 +316,6 @@ __device__ __forceinline__ uint32_t shade_fragment(const FrameDev& F, const Mesh
     F3 n = f3(GBR_INTERP(v0.n.x, v1.n.x, v2.n.x), GBR_INTERP(v0.n.y, v1.n.y, v2.n.y), GBR_INTERP(v0.n.z, v1.n.z, v2.n.z));
     n = f3(__fmul_rn(n.x, winterp), __fmul_rn(n.y, winterp), __fmul_rn(n.z, winterp));
     if (F.vis == 2u) return rgba_from_colour(n);
-    if (!m.tex[0].px) {
-        // colour is not multiplied by the interpolated w (CUDAROPs.cu:379-380)
-        const F3 c = f3(GBR_INTERP(v0.c.x, v1.c.x, v2.c.x), GBR_INTERP(v0.c.y, v1.c.y, v2.c.y),
-                        GBR_INTERP(v0.c.z, v1.c.z, v2.c.z));
-        return rgba_from_colour(c);
-    }
     const float u = __fmul_rn(GBR_INTERP(v0.u, v1.u, v2.u), winterp);
     const float vv = __fmul_rn(GBR_INTERP(v0.v, v1.v, v2.v), winterp);
     // tangent is not multiplied by the interpolated w (CUDAROPs.cu:371-372)
