@@ -113,6 +113,7 @@ void gbr::frame_basics(const gbr_renderer* r, const gbr_camera* cam, uint32_t cu
     F.cull = cull; F.sample = sample; F.vis = vis; F.clear_colour32 = 0x003F3F3Fu;
     F.num_meshes = (uint32_t)r->meshes.size();
     F.num_tris = (uint32_t)scene_triangles(r);
+    F.key_mask = key_mask_for(F.num_tris);
     for (int k = 0; k < 3; ++k) { F.cam_pos[k] = cam->pos[k]; F.cam_fwd[k] = cam->fwd[k]; }
     F.colour = r->d_colour; F.depth = r->d_depth; F.ids = r->d_ids; F.gvis = r->d_gvis;
     F.lights = r->d_lights;
@@ -322,6 +323,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         F.count_split = 1u;
     }
     r->last_row_blocks = F.row_blocks;
+    r->last_key_mask = F.key_mask;
     r->last_raster_lanes = F.raster_lanes;
     // frames shaded through the full vertex stage shade their covered
     // pixels in a second, densely packed pass
@@ -806,7 +808,7 @@ gbr_status gbr_get_bins(gbr_renderer* r, uint32_t* offsets, uint32_t* ids, uint6
             if (!all.empty())
                 GBR_CUDA(cudaMemcpy(all.data(), r->d_list, all.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
             for (uint32_t b = 0; b < nb; ++b)
-                for (uint32_t k = 0; k < out_off[b + 1] - out_off[b]; ++k) ids[out_off[b] + k] = all[off[b] + k] & ~kNoRasterBit;
+                for (uint32_t k = 0; k < out_off[b + 1] - out_off[b]; ++k) ids[out_off[b] + k] = list_id(all[off[b] + k], r->last_key_mask);
         }
         return GBR_OK;
     }
@@ -817,7 +819,7 @@ gbr_status gbr_get_bins(gbr_renderer* r, uint32_t* offsets, uint32_t* ids, uint6
         if (capacity < total) return fail(GBR_ERR_INVALID_ARG, "ids capacity %llu < %llu pairs",
                                           (unsigned long long)capacity, (unsigned long long)total);
         if (total) GBR_CUDA(cudaMemcpy(ids, r->d_list, total * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-        for (uint64_t i = 0; i < total; ++i) ids[i] &= ~kNoRasterBit;
+        for (uint64_t i = 0; i < total; ++i) ids[i] = list_id(ids[i], r->last_key_mask);
     }
     return GBR_OK;
 }

@@ -698,7 +698,7 @@ gbr_status gbr_batch_get_bins(gbr_batch* b, uint32_t index, uint32_t* offsets, u
         if (capacity < total) return fail(GBR_ERR_INVALID_ARG, "ids capacity %llu < %llu pairs",
                                           (unsigned long long)capacity, (unsigned long long)total);
         if (total) GBR_CUDA(cudaMemcpy(ids, b->d_list + off[0], total * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-        for (uint64_t i = 0; i < total; ++i) ids[i] &= ~kNoRasterBit;
+        for (uint64_t i = 0; i < total; ++i) ids[i] = list_id(ids[i], key_mask_for(L.tris));
     }
     return GBR_OK;
 }

@@ -14,12 +14,35 @@
 namespace gbr {
 
 constexpr uint32_t kInvalidPrim = 0xFFFFFFFFu;
-constexpr uint32_t kNoRasterBit = 0x80000000u;   // bin-list entry that cannot cover a pixel
+// A bin-list entry: the primitive, kNoRasterBit if it cannot cover a pixel,
+// and in frames of at most 2^kKeyedIdBits triangles the top 8 bits of its
+// depth-key bound (bits 23-30, where they sit in the key), by which the
+// raster sorts.  Sorting a bin then reads nothing but its list: gathering
+// the bounds of 980 entries a bin took 16 L1 wavefronts a load.  Larger
+// frames keep their bounds in FrameDev::keys alone.
+constexpr uint32_t kNoRasterBit = 0x80000000u;
+constexpr uint32_t kKeyedIdBits = 23;
+constexpr uint32_t kSortShift = 23;               // depth key -> depth bucket (256 buckets of the 31-bit key)
+__host__ __device__ constexpr uint32_t key_mask_for(unsigned long long tris) {
+    return tris <= (1ull << kKeyedIdBits) ? 0x7F800000u : 0u;
+}
+__host__ __device__ constexpr uint32_t list_id(uint32_t entry, uint32_t key_mask) {
+    return entry & ~(kNoRasterBit | key_mask);
+}
+__device__ __forceinline__ uint32_t list_entry(uint32_t prim, uint32_t key, bool no_raster, uint32_t key_mask) {
+    return prim | (no_raster ? kNoRasterBit : key & key_mask);
+}
+// The depth bucket of an entry that can cover a pixel.
+__device__ __forceinline__ uint32_t entry_bucket(uint32_t entry, uint32_t key_mask, const uint32_t* keys) {
+    return (key_mask ? entry : __ldg(keys + entry)) >> kSortShift;
+}
 constexpr unsigned long long kEmptyVis = 0xFFFFFFFFFFFFFFFFull;
 constexpr int kFxBits = 16;                       // 16.16 fixed-point screen coordinates
 constexpr float kGuardPx = 8192.0f;               // |coord| below this: exact int64 edge functions
-constexpr uint32_t kFlagRaster = 1u;              // fixed path, covered winding, area > 0
-constexpr uint32_t kFlagFloat = 2u;               // outside the guard band: float edge functions
+// Flags of a setup record, above its mesh index.
+constexpr uint32_t kFlagRaster = 0x40000000u;     // fixed path, covered winding, area > 0
+constexpr uint32_t kFlagFloat = 0x80000000u;      // outside the guard band: float edge functions
+constexpr uint32_t kMeshMask = 0x3FFFFFFFu;
 constexpr int kMaxBinDim = 64;
 constexpr int kRasterThreads = 256;
 constexpr int kBatch = 2048;                      // bin entries the record raster depth-sorts at once
@@ -42,7 +65,7 @@ __host__ __device__ inline uint32_t count_split_for(unsigned long long pairs, ui
     return per_bin >= 256u ? 8u : per_bin >= 64u ? 4u : per_bin >= 16u ? 2u : 1u;
 }
 constexpr uint32_t kDefaultRasterCtas = 6;    // record raster variant (CTAs per SM) used by default
-constexpr uint32_t kDefaultBlockCtas = 5;     // the block raster's
+constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
 // The block raster's CTAs in a single frame: 128 threads where the items
 // outnumber the SMs several times (fewer warps wait at each of an item's
 // barriers than in CTAs of 256: 1M soup 78 us against 88, 2M soup at 4K 201
@@ -130,13 +153,14 @@ static_assert(sizeof(LightDev) == 32, "light record is 32 bytes");
 
 // Raster setup record, 48 B: the triangle's float screen vertices (the
 // raster snaps them to 16.16 for coverage), NDC z per vertex, 1 / the float
-// area the reference divides its weights by, flags, mesh index.
+// area the reference divides its weights by, the depth-key bound (hiz_key),
+// mesh index and flags.
 struct __align__(16) TriSetup {
     float x0, y0, x1, y1;
     float x2, y2;
     float z0, z1;
     float z2, inv_area;
-    uint32_t flags;
+    uint32_t key;
     uint32_t mesh;
 };
 static_assert(sizeof(TriSetup) == 48, "setup record is 48 bytes");
@@ -173,7 +197,8 @@ struct __align__(16) FrameDev {
     const MeshDev* meshes;
     TriSetup* setup;
     uint2* rects;
-    uint32_t* keys;            // per triangle: lower bound of its fragments' depth keys (hiz_key)
+    uint32_t* keys;            // per triangle: lower bound of its fragments' depth keys (hiz_key), for the fill pass
+    uint32_t key_mask;         // bits of the lists' entries that hold the bound's top 8 bits (0: none)
     uint32_t* counts;          // kCountSplit sub-counters per bin: counts[k * count_stride + bin]
     uint32_t* sub_base;        // first list entry of each sub-counter's pairs (same layout)
     uint32_t* offsets;        // num_bins + 1

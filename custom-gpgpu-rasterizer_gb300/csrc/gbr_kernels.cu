@@ -73,7 +73,7 @@ __device__ __forceinline__ uint32_t find_mesh(const FrameDev& F, uint32_t prim) 
 // stored key is below it.  0: no bound (float path, vertices behind z = 0);
 // 0x7FFFFFFF: every fragment has z >= 1 and loses everywhere.
 __device__ __forceinline__ uint32_t hiz_key(const TriSetup& t) {
-    if (t.flags & kFlagFloat) return 0u;
+    if (t.mesh & kFlagFloat) return 0u;
     const float zmin = fminf(t.z0, fminf(t.z1, t.z2));
     if (!(zmin >= 0.f)) return 0u;
     const float zabs = fmaxf(fabsf(t.z0), fmaxf(fabsf(t.z1), fabsf(t.z2)));
@@ -97,6 +97,7 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
     const bool in_range = prim < F.num_tris;
     uint2 rect = empty_rect();
     bool visible = false, fpath = false, no_raster = true;
+    uint32_t key = 0u;
     if (in_range) {
         const uint32_t mi = find_mesh(F, prim);
         const MeshDev& m = F.meshes[mi];
@@ -152,17 +153,18 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
                 no_raster = false;
                 flags = kFlagFloat;
             }
-            uint4* rec = reinterpret_cast<uint4*>(F.setup) + 3u * prim;
-            rec[0] = make_uint4(__float_as_uint(s0.x), __float_as_uint(s0.y), __float_as_uint(s1.x), __float_as_uint(s1.y));
-            rec[1] = make_uint4(__float_as_uint(s2.x), __float_as_uint(s2.y), __float_as_uint(nz[0]), __float_as_uint(nz[1]));
-            rec[2] = make_uint4(__float_as_uint(nz[2]), __float_as_uint(inv_area), flags, mi);
-            rect = pack_rect(r, no_raster);
             // the raster depth-sorts a bin's triangles by this bound before it
             // reads their records
             TriSetup t;
             t.x0 = s0.x; t.y0 = s0.y; t.x1 = s1.x; t.y1 = s1.y; t.x2 = s2.x; t.y2 = s2.y;
-            t.z0 = nz[0]; t.z1 = nz[1]; t.z2 = nz[2]; t.inv_area = inv_area; t.flags = flags; t.mesh = mi;
-            F.keys[prim] = hiz_key(t);
+            t.z0 = nz[0]; t.z1 = nz[1]; t.z2 = nz[2]; t.inv_area = inv_area; t.mesh = mi | flags;
+            key = hiz_key(t);
+            uint4* rec = reinterpret_cast<uint4*>(F.setup) + 3u * (size_t)prim;
+            rec[0] = make_uint4(__float_as_uint(s0.x), __float_as_uint(s0.y), __float_as_uint(s1.x), __float_as_uint(s1.y));
+            rec[1] = make_uint4(__float_as_uint(s2.x), __float_as_uint(s2.y), __float_as_uint(nz[0]), __float_as_uint(nz[1]));
+            rec[2] = make_uint4(__float_as_uint(nz[2]), __float_as_uint(inv_area), key, mi | flags);
+            rect = pack_rect(r, no_raster);
+            F.keys[prim] = key;
         }
         F.rects[prim] = rect;
     }
@@ -170,7 +172,7 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
                             ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, fpath)) << 16);
     if (MODE == 0) bin_walk<0>(F, rect, 0u, visible, walk);
     else if (MODE == 2) count_rect(s_row, visible ? rect : empty_rect(), F.nbx, F.nby);
-    else bin_walk<2>(F, rect, prim | (no_raster ? kNoRasterBit : 0u), visible, walk);
+    else bin_walk<2>(F, rect, list_entry(prim, key, no_raster, F.key_mask), visible, walk);
     return counts;
 }
 
@@ -212,12 +214,16 @@ __global__ void __launch_bounds__(256) setup_kernel(FrameDev F) {
     pdl_release();
 }
 
+// The list entry of triangle `prim` with rectangle `rect`, in a fill pass.
+__device__ __forceinline__ uint32_t rect_entry(const FrameDev& F, uint32_t prim, uint2 rect, bool in_range) {
+    return list_entry(prim, in_range && F.key_mask ? F.keys[prim] : 0u, (rect.y & 0x80000000u) != 0u, F.key_mask);
+}
+
 // Second pass of exact binning for triangle `prim`.  Called by whole warps.
 __device__ __forceinline__ void fill_tri(const FrameDev& F, uint32_t prim, uint32_t walk) {
     const bool in_range = prim < F.num_tris;
     const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-    const uint32_t entry = prim | ((rect.y & 0x80000000u) ? kNoRasterBit : 0u);
-    bin_walk<1>(F, rect, entry, in_range, walk);
+    bin_walk<1>(F, rect, rect_entry(F, prim, rect, in_range), in_range, walk);
 }
 
 __global__ void __launch_bounds__(256) fill_kernel(FrameDev F) {
@@ -304,8 +310,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
         const uint32_t prim = base + threadIdx.x;
         const bool in_range = prim < F.num_tris;
         const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-        const uint32_t entry = prim | ((rect.y & 0x80000000u) ? kNoRasterBit : 0u);
-        fill_walk(F, rect, entry, s_row);
+        fill_walk(F, rect, rect_entry(F, prim, rect, in_range), s_row);
     }
     pdl_release();
 }
@@ -352,8 +357,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
             const uint32_t prim = base + tid;
             const bool in_range = prim < F.num_tris;
             const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-            const uint32_t entry = prim | ((rect.y & 0x80000000u) ? kNoRasterBit : 0u);
-            fill_walk(F, rect, entry, s_row);
+            fill_walk(F, rect, rect_entry(F, prim, rect, in_range), s_row);
         }
     }
     add_block_stats(F.ctl, vis, fp);
@@ -389,7 +393,6 @@ cudaError_t launch_list_touch(const FrameDev& F, cudaStream_t s) {
 struct RasterShared {
     TriSetup rec[kMaxPhase];     // setup records of the running phase
     uint32_t prim[kBatch];       // staged bin entries (rasterisable triangles)
-    uint32_t key[kBatch];        // their depth-key lower bounds
     uint16_t order[kBatch];      // staged triangles, front to back by depth bucket
     uint32_t bucket[kDepthBuckets];   // counts -> starts -> (after the scatter) ends
     uint32_t warp_count[kRasterThreads / 32];
@@ -400,7 +403,6 @@ struct RasterShared {
     __align__(8) unsigned long long rec_bar[2];   // mbarriers: a phase's setup records have landed (phases alternate)
 };
 static_assert(kDepthBuckets == kRasterThreads, "one depth bucket per thread");
-constexpr uint32_t kKeyShift = 23u;   // depth key -> bucket: the top 8 bits of the 31-bit key
 
 // Setup records reach shared memory by bulk asynchronous copies (the TMA
 // engine's cp.async.bulk, one 48-byte copy per record), each completing
@@ -416,7 +418,7 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)
 // kMaxPhase).
 __device__ __forceinline__ void issue_records(TriSetup* rec, const TriSetup* setup, const uint32_t* prim,
                                               const uint16_t* order, uint32_t p0, uint32_t pn, uint32_t bar,
-                                              uint32_t lane);
+                                              uint32_t lane, uint32_t key_mask);
 
 __device__ __forceinline__ void rec_copy(TriSetup* dst, const TriSetup* src, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 48, [%2];"
@@ -425,13 +427,13 @@ __device__ __forceinline__ void rec_copy(TriSetup* dst, const TriSetup* src, uin
 
 __device__ __forceinline__ void issue_records(TriSetup* rec, const TriSetup* setup, const uint32_t* prim,
                                               const uint16_t* order, uint32_t p0, uint32_t pn, uint32_t bar,
-                                              uint32_t lane) {
+                                              uint32_t lane, uint32_t key_mask) {
     if (lane == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(pn * 48u) : "memory");
     __syncwarp();
     for (uint32_t q = lane; q < pn; q += 32u) {
         const uint32_t k = p0 + q;
-        rec_copy(&rec[k & (kMaxPhase - 1u)], setup + prim[order[k]], bar);
+        rec_copy(&rec[k & (kMaxPhase - 1u)], setup + list_id(prim[order[k]], key_mask), bar);
     }
 }
 
@@ -506,7 +508,7 @@ __device__ __forceinline__ void raster_fixed(const TriSetup& t, uint32_t prim, u
 // float path or with a box of more than kLanePixels pixels.
 __device__ __forceinline__ bool raster_fixed_lane(const TriSetup& t, uint32_t prim, unsigned long long* tile, int tx0,
                                                   int ty0, int tw, int th, uint32_t key_bound) {
-    if (t.flags & kFlagFloat) return false;
+    if (t.mesh & kFlagFloat) return false;
     const int X0 = snap_fx(t.x0), Y0 = snap_fx(t.y0), X1 = snap_fx(t.x1);
     const int Y1 = snap_fx(t.y1), X2 = snap_fx(t.x2), Y2 = snap_fx(t.y2);
     const int minx = min(X0, min(X1, X2)), maxx = max(X0, max(X1, X2));
@@ -590,9 +592,9 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
     TriSetup t;
     t.x0 = __uint_as_float(a.x); t.y0 = __uint_as_float(a.y); t.x1 = __uint_as_float(a.z); t.y1 = __uint_as_float(a.w);
     t.x2 = __uint_as_float(b.x); t.y2 = __uint_as_float(b.y); t.z0 = __uint_as_float(b.z); t.z1 = __uint_as_float(b.w);
-    t.z2 = __uint_as_float(c.x); t.inv_area = __uint_as_float(c.y); t.flags = c.z; t.mesh = c.w;
+    t.z2 = __uint_as_float(c.x); t.inv_area = __uint_as_float(c.y); t.key = c.z; t.mesh = c.w;
     float w[3] = {0.f, 0.f, 0.f};
-    if (t.flags & kFlagFloat) weights_float(t, (float)x, (float)y, w);
+    if (t.mesh & kFlagFloat) weights_float(t, (float)x, (float)y, w);
     else weights_fixed(t, x, y, w);
     const float z = interp_z(w[0], w[1], w[2], t.z0, t.z1, t.z2);
     if (KIND == kShadeFlatOne) {   // needs no mesh lookup: the vertices load beside the record
@@ -600,7 +602,7 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
     } else if (KIND == kShadeDepth) {
         F.colour[gi] = shade_depth(z);
     } else {
-        const MeshDev& m = F.meshes[t.mesh];
+        const MeshDev& m = F.meshes[t.mesh & kMeshMask];
         F.colour[gi] = KIND == kShadeFlat ? shade_flat(flat_mesh(m), prim - m.prim_base, w) : shade_fragment(F, m, prim, w, z);
     }
     F.depth[gi] = z;
@@ -663,6 +665,7 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
         for (int i = (int)tid; i < npx; i += THREADS) tile[i] = kEmptyVis;
         if (tid == 0) fetch_item(&S.item_next, items, next_idx, num_items);
         const uint32_t* const keys = F.keys;
+        const uint32_t key_mask = F.key_mask;
         for (uint32_t b0 = 0; b0 < count && npx > 0; b0 += pass) {
             // stage the entries with their depth-key bounds (no setup record
             // is read before a triangle's phase comes) and count the
@@ -680,11 +683,8 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
                 if (j >= rows) break;
                 const uint32_t idx = j * THREADS + tid;
                 const uint32_t e = idx < n ? __ldg(list + start + b0 + idx) : kNoRasterBit;
-                const bool keep = !(e & kNoRasterBit);
-                const uint32_t k = keep ? __ldg(keys + e) : 0u;
                 S.prim[idx] = e;
-                S.key[idx] = k;
-                if (keep) atomicAdd(&S.bucket[k >> kKeyShift], 1u);
+                if (!(e & kNoRasterBit)) atomicAdd(&S.bucket[entry_bucket(e, key_mask, keys)], 1u);
             }
             __syncthreads();
             // bucket starts: exclusive scan of the 256 counts; their sum is the
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
                 if (j >= rows) break;
                 const uint32_t idx = j * THREADS + tid;
                 if (idx < n && !(S.prim[idx] & kNoRasterBit))
-                    S.order[atomicAdd(&S.bucket[S.key[idx] >> kKeyShift], 1u)] = (uint16_t)idx;
+                    S.order[atomicAdd(&S.bucket[entry_bucket(S.prim[idx], key_mask, keys)], 1u)] = (uint16_t)idx;
             }
             // now S.bucket[b] = end of bucket b
             // phases of `phase` triangles; the tile's max depth key is refreshed
@@ -733,17 +733,17 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
                 if (tma) {
                     if (warp == 0) {
                         if (p0 == 0u || !ahead)   // this phase's records were not prefetched
-                            issue_records(S.rec, setup, S.prim, S.order, p0, pn, bar, lane);
+                            issue_records(S.rec, setup, S.prim, S.order, p0, pn, bar, lane, key_mask);
                         if (next)
                             issue_records(S.rec, setup, S.prim, S.order, p0 + phase, min(phase, total - p0 - phase),
-                                          bar_next, lane);
+                                          bar_next, lane, key_mask);
                     }
                 } else {
                     // 16 bytes per thread (triangle k's record goes to slot k
                     // mod kMaxPhase: phase <= kMaxPhase)
                     for (uint32_t r = tid; r < 3u * pn; r += THREADS) {
                         const uint32_t q = r / 3u, k = p0 + q;
-                        const uint4* rp = reinterpret_cast<const uint4*>(setup) + 3u * S.prim[S.order[k]];
+                        const uint4* rp = reinterpret_cast<const uint4*>(setup) + 3u * (size_t)list_id(S.prim[S.order[k]], key_mask);
                         reinterpret_cast<uint4*>(&S.rec[k & (kMaxPhase - 1u)])[r - 3u * q] = __ldg(rp + (r - 3u * q));
                     }
                 }
@@ -769,8 +769,8 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
 #pragma unroll
                     for (uint32_t w = 0; w < THREADS / 32; ++w) tile_max = max(tile_max, S.warp_max[w]);
                 }
-                // buckets [0, tile_max >> kKeyShift] can still hold a winner
-                const uint32_t limit = tile_max >= 0x80000000u ? total : S.bucket[tile_max >> kKeyShift];
+                // buckets [0, tile_max >> kSortShift] can still hold a winner
+                const uint32_t limit = tile_max >= 0x80000000u ? total : S.bucket[tile_max >> kSortShift];
                 if (p0 >= limit) {   // uniform: every thread sees the same tile_max
                     if (next) {
                         if (!rec_wait(bar_next, (rec_parity >> (ph ^ 1u)) & 1u) && tid == 0) atomicOr(&Q->error, 8u);
@@ -796,20 +796,20 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
                         bool big = false;
                         if (lane < kLaneGrab && k < p1) {
                             const uint32_t i = S.order[k];
-                            const uint32_t key = S.key[i];
-                            if (key <= tile_max)
-                                big = !raster_fixed_lane(S.rec[k & (kMaxPhase - 1u)], S.prim[i], tile, tx0, ty0, tw, th,
-                                                         key);
+                            const TriSetup& t = S.rec[k & (kMaxPhase - 1u)];
+                            if (t.key <= tile_max)
+                                big = !raster_fixed_lane(t, list_id(S.prim[i], key_mask), tile, tx0, ty0, tw, th, t.key);
                         }
                         m = __ballot_sync(0xFFFFFFFFu, big);
                     } else {
-                        m = S.key[S.order[kb]] <= tile_max ? 1u : 0u;
+                        m = S.rec[(uint32_t)kb & (kMaxPhase - 1u)].key <= tile_max ? 1u : 0u;
                     }
                     for (; m; m &= m - 1u) {
                         const uint32_t k = (uint32_t)kb + (uint32_t)(__ffs(m) - 1), i = S.order[k];
                         const TriSetup& t = S.rec[k & (kMaxPhase - 1u)];
-                        if (t.flags & kFlagFloat) raster_float(t, S.prim[i], tile, tx0, ty0, tw, th, lane);
-                        else raster_fixed(t, S.prim[i], tile, tx0, ty0, tw, th, lane, S.key[i]);
+                        const uint32_t prim = list_id(S.prim[i], key_mask);
+                        if (t.mesh & kFlagFloat) raster_float(t, prim, tile, tx0, ty0, tw, th, lane);
+                        else raster_fixed(t, prim, tile, tx0, ty0, tw, th, lane, t.key);
                     }
                 }
             }

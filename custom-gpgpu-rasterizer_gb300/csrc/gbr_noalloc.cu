@@ -162,6 +162,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     F.flat_shade = vis == GBR_VIS_PBR ? 1u : 0u;
     F.num_meshes = 1u;
     F.num_tris = (uint32_t)tris;
+    F.key_mask = key_mask_for(tris);
     F.chunk = kMaxChunk;      // work items: the library's split
     F.stage = queue_chunk;    // entries per raster pass
     F.block_threads = block_threads_for(nb, (uint32_t)slot.num_sms);

@@ -32,7 +32,6 @@ namespace {
 
 constexpr int kBlockW = 8, kBlockH = 4;          // a warp's pixels
 constexpr uint32_t kSortBuckets = 256u;          // depth buckets: the top 8 bits of the 31-bit key
-constexpr uint32_t kSortShift = 23u;
 constexpr int kEdgeClamp = 1 << 30;
 // blk / nbw = blk * kInvBlocks[nbw] >> 10 for blk < 128, nbw <= 8 (a bin holds at most 8 x 16 blocks)
 __device__ constexpr uint16_t kInvBlocks[9] = {0, 1025, 513, 342, 257, 205, 171, 147, 129};
@@ -63,7 +62,7 @@ struct BlockShared {
     static constexpr uint32_t kEntries = THREADS == 128 ? 1024u : 2048u;   // entries depth-sorted at once
     static constexpr uint32_t kPhase = THREADS == 512 ? 128u : 32u;        // triangles reduced at once
     PhaseTris<kPhase> tri;
-    uint32_t sorted[kEntries];              // staged primitives, front to back by bucket
+    uint32_t sorted[kEntries];              // staged entries, front to back by bucket
     uint32_t hist[2][kSortBuckets];         // entries per bucket; passes alternate, each zeroed after its scan
     uint32_t start[kSortBuckets + 4u];      // first sorted entry of each bucket, then the total
     uint32_t item[2][6];                    // the running item (items alternate): bin, list start, count, chunks; x, y
@@ -91,7 +90,7 @@ __device__ __forceinline__ int narrow_edge(long long e) {
 // slot `k` of the phase.  One that covers none of the bin's pixels gets an
 // empty box.
 template <uint32_t P>
-__device__ __forceinline__ void reduce_triangle(const TriSetup* setup, uint32_t prim, uint32_t key, int tx0, int ty0,
+__device__ __forceinline__ void reduce_triangle(const TriSetup* setup, uint32_t prim, int tx0, int ty0,
                                                 int tw, int th, PhaseTris<P>& out, uint32_t k) {
     const uint4* rp = reinterpret_cast<const uint4*>(setup) + 3u * (size_t)prim;
     const uint4 r0 = __ldg(rp), r1 = __ldg(rp + 1), r2 = __ldg(rp + 2);
@@ -101,7 +100,7 @@ __device__ __forceinline__ void reduce_triangle(const TriSetup* setup, uint32_t 
     int dxa = 0, dya = 0, dxb = 0, dyb = 0, dxc = 0, dyc = 0;
     int px0 = 0, px1 = tw - 1, py0 = 0, py1 = th - 1;
     uint32_t kind = kTriFloat;
-    if (r2.z & kFlagFloat) {
+    if (r2.w & kFlagFloat) {
         if (x0 != x0 || y0 != y0 || x1 != x1 || y1 != y1 || x2 != x2 || y2 != y2) px1 = -1;
     } else {
         const int X0 = snap_fx(x0), Y0 = snap_fx(y0), X1 = snap_fx(x1);
@@ -134,7 +133,7 @@ __device__ __forceinline__ void reduce_triangle(const TriSetup* setup, uint32_t 
         box = (uint32_t)px0 | ((uint32_t)px1 << 8) | ((uint32_t)py0 << 16) | ((uint32_t)py1 << 24);
     out.a[k] = make_uint4((uint32_t)qa, (uint32_t)qb, (uint32_t)qc, prim);
     out.b[k] = make_uint4((uint32_t)dya, (uint32_t)-dxa, (uint32_t)dyb, (uint32_t)-dxb);
-    out.c[k] = make_uint4((uint32_t)dyc, (uint32_t)-dxc, key, box | (kind << 6));
+    out.c[k] = make_uint4((uint32_t)dyc, (uint32_t)-dxc, r2.z, box | (kind << 6));
     out.r0[k] = r0;
     out.r1[k] = r1;
     out.r2[k] = make_uint2(r2.x, r2.y);
@@ -187,7 +186,7 @@ __device__ __forceinline__ TriSetup load_record(const PhaseTris<P>& tri, uint32_
     TriSetup t;
     t.x0 = __uint_as_float(a.x); t.y0 = __uint_as_float(a.y); t.x1 = __uint_as_float(a.z); t.y1 = __uint_as_float(a.w);
     t.x2 = __uint_as_float(b.x); t.y2 = __uint_as_float(b.y); t.z0 = __uint_as_float(b.z); t.z1 = __uint_as_float(b.w);
-    t.z2 = __uint_as_float(c.x); t.inv_area = __uint_as_float(c.y); t.flags = 0u; t.mesh = 0u;
+    t.z2 = __uint_as_float(c.x); t.inv_area = __uint_as_float(c.y); t.key = 0u; t.mesh = 0u;
     return t;
 }
 
@@ -341,6 +340,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
         const uint32_t* const list = G.list;
         const TriSetup* const setup = G.setup;
         const uint32_t* const keys = G.keys;
+        const uint32_t key_mask = G.key_mask;
         const uint32_t nbw = (uint32_t)(tw + kBlockW - 1) / kBlockW;
         const uint32_t nblk = nbw * ((uint32_t)(th + kBlockH - 1) / kBlockH);
         const uint32_t inv = kInvBlocks[nbw];
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
 #pragma unroll
                 for (uint32_t j = 0; j < kPer; ++j) {
                     if (e[j] & kNoRasterBit) continue;
-                    const uint32_t bucket = __ldg(keys + e[j]) >> kSortShift;
+                    const uint32_t bucket = entry_bucket(e[j], key_mask, keys);
                     place[j] = (bucket << 16) | atomicAdd(&hist[bucket], 1u);
                 }
                 __syncthreads();   // also: every warp is done with the previous pass's order
@@ -409,9 +409,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
             for (uint32_t p0 = 0; p0 < total; p0 += kPhase) {
                 const uint32_t pn = min(kPhase, total - p0);
                 if (tid < pn) {
-                    const uint32_t prim = direct ? __ldg(list + first + tid) : S.sorted[p0 + tid];
-                    if (prim & kNoRasterBit) S.tri.c[tid].w = 63u | (63u << 16);   // an empty box
-                    else reduce_triangle(setup, prim, __ldg(keys + prim), tx0, ty0, tw, th, S.tri, tid);
+                    const uint32_t entry = direct ? __ldg(list + first + b0 + tid) : S.sorted[p0 + tid];
+                    if (entry & kNoRasterBit) S.tri.c[tid].w = 63u | (63u << 16);   // an empty box
+                    else reduce_triangle(setup, list_id(entry, key_mask), tx0, ty0, tw, th, S.tri, tid);
                 }
                 __syncthreads();
                 bool more = false;

@@ -301,7 +301,7 @@ typedef struct {
     uint32_t bin_size;     /* bins of bin_size x bin_size pixels, 1..64 */
     uint32_t queue_chunk;  /* entries depth-sorted and rasterised per pass over a tile, >= 1 (at most 2048
                               used); work items hold 2048 entries */
-    uint32_t raster_ctas;  /* raster variant: CTAs per SM, 2..6 (0: 5), counted in CTAs of 256 threads */
+    uint32_t raster_ctas;  /* raster variant: CTAs per SM, 2..6 (0: 4), counted in CTAs of 256 threads */
     uint32_t raster_phase; /* 0..128; kept, without effect: a batch's raster refreshes its depth bounds after
                               every triangle */
     uint32_t raster_threads; /* threads per bin: raster CTAs of 128 or 256 threads (0: 256); a 128-thread CTA

@@ -65,3 +65,29 @@ def test_block_raster_against_the_oracle(gbr_lib, cuda_device, bw, bh, w, h, n, 
             c, oc = colour.astype(np.int64), o["colour"].astype(np.int64)
             assert max(np.abs(((c >> k) & 255) - ((oc >> k) & 255)).max() for k in (0, 8, 16)) <= 1
             assert r.stats()["raster_lanes"] == 0
+
+
+@pytest.mark.parametrize("n", [1 << 23, (1 << 23) + 1])
+def test_list_entries_with_and_without_depth(gbr_lib, cuda_device, n):
+    """Up to 2^23 triangles a list entry carries its depth bucket beside the
+    primitive; one more and it does not.  Most of the frame's triangles lie
+    off the screen, the drawn ones are the first and the last, so ids use
+    every bit: bin lists and winners are the oracle's either way."""
+    drawn = scenes.soup_vertices(1500, 320, 240, seed=9)
+    off = np.zeros(3, scenes.POS3_RGBA8)
+    off["p"] = [(5.0, 5.0, 0.5), (6.0, 5.0, 0.5), (5.0, 6.0, 0.5)]
+    v = np.concatenate([drawn, off])
+    ix = np.tile(np.arange(len(drawn), len(v), dtype=np.uint32), n).reshape(n, 3)
+    d = np.arange(len(drawn), dtype=np.uint32).reshape(-1, 3)
+    ix[:700], ix[-800:] = d[:700], d[700:]
+    s = scenes.Scene("many", 320, 240, 16, 16, scenes.identity_camera(),
+                     [scenes.Mesh(vertices=v, indices=ix.reshape(-1))], cull=scenes.CULL_NONE)
+    o = oracle.render(s, oracle.RASTER_FIXED)
+    assert o["ids"][o["ids"] != 0xFFFFFFFF].max() >= n - 800
+    with gbr_lib.Renderer(320, 240) as r:
+        r.load_scene(s)
+        for _ in range(2):
+            r.render_scene(s)
+            offsets, bins = r.get_bins()
+            assert np.array_equal(offsets, o["offsets"]) and np.array_equal(bins, o["bins"])
+            assert np.array_equal(r.readback_ids(), o["ids"])
