@@ -328,7 +328,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     // frames shaded through the full vertex stage shade their covered
     // pixels in a second, densely packed pass
     if (!F.flat_shade && vis != GBR_VIS_DEPTH) {
-        if (!r->d_shade_list) GBR_CUDA(cudaMalloc(&r->d_shade_list, (size_t)r->W * r->H * sizeof(uint32_t)));
+        if (!r->d_shade_list) GBR_CUDA(cudaMalloc(&r->d_shade_list, (size_t)r->W * r->H * sizeof(uint2)));
         F.shade_list = r->d_shade_list;
         // the light pass leaves bins that stay clean untouched
         if (r->d_dirty) {
@@ -349,6 +349,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     const bool touch = r->seen_pairs >= kListTouchMinPairs;
     if (touch && F.row_blocks)   // the block-row count pass zeroes the last frame's entries (and 1/16 more)
         F.touch_words = (uint32_t)((std::min<uint64_t>(r->list_cap, r->seen_pairs + r->seen_pairs / 16u) + 3u) / 4u);
+    // the fill pass scans the bins itself (not where a test hook silences a
+    // tile of the scan kernel)
+    F.fused_scan = !predicted && nb <= kFusedBins && F.count_split == 1u && !F.scan_silent_tile1 && !F.scan_spin_limit &&
+                   (F.row_blocks || (F.num_tris > 0u && F.num_tris <= kFusedTris && !touch));
     if (r->timing) GBR_CUDA(cudaEventRecord(r->ev[0], s));
     GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
     if (predicted) {
@@ -379,7 +383,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         }
         GBR_CUDA(launch_setup(F, false, s));
         if (stages) GBR_CUDA(cudaEventRecord(r->ev[1], s));
-        GBR_CUDA(launch_scan(scan_of(F, kScanExact), s));
+        if (!F.fused_scan) GBR_CUDA(launch_scan(scan_of(F, kScanExact), s));
         if (touch && !F.row_blocks) GBR_CUDA(launch_list_touch(F, s));
         GBR_CUDA(launch_fill(F, s));
     }
@@ -387,7 +391,12 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[2], s));
     GBR_CUDA(launch_raster(F, r->raster_grid, s));
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[4], s));
-    GBR_CUDA(launch_shade(F, s));
+    ShadeOne one;
+    if (md.size() == 1u) {
+        one.mesh = md[0];
+        memcpy(one.lights, r->lights, sizeof one.lights);
+    }
+    GBR_CUDA(launch_shade(F, md.size() == 1u ? &one : nullptr, s));
     if (r->timing) {
         GBR_CUDA(cudaEventRecord(r->ev[3], s));
         r->ev_recorded = true;
@@ -677,6 +686,7 @@ gbr_status gbr_set_lights(gbr_renderer* r, const gbr_light* lights, uint32_t n) 
     if (n) {
         cudaDeviceSynchronize();   // frames in flight read the previous lights
         GBR_CUDA(cudaMemcpy(r->d_lights, lights, n * sizeof(LightDev), cudaMemcpyHostToDevice));
+        memcpy(r->lights, lights, n * sizeof(LightDev));
     }
     r->num_lights = n;
     return GBR_OK;

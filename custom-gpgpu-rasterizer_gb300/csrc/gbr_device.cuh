@@ -104,6 +104,13 @@ __host__ __device__ inline bool use_count_rows(unsigned long long pairs, uint32_
 // the outputs still written whole.
 constexpr uint32_t kTileW = 32, kTileH = 16;
 
+// The fill pass holds the bin scan (FrameDev::fused_scan) of frames of one
+// counter a bin and up to kFusedBins bins, in the block-row path or with up
+// to kFusedTris triangles: every block scans all the bins, which pays while
+// both are few (640x480 sphere, 1200 bins: 35.0 -> 30.2 us a frame; 1M soup,
+// 8160 bins: scan + fill 55.8 -> 57.1; 2M at 4K, 32,400 bins: 113 -> 129).
+constexpr uint32_t kFusedBins = 4096, kFusedTris = 1u << 16;
+
 enum : uint32_t { kVertexIVertex56 = 0, kVertexPos3Rgba8 = 1 };
 
 struct TexDev {
@@ -150,6 +157,13 @@ struct LightDev {
     float vec[3];
 };
 static_assert(sizeof(LightDev) == 32, "light record is 32 bytes");
+
+// What the heavy shade pass of a frame of one mesh reads besides the frame:
+// passed by value, so none of it is loaded on the way to a pixel's texels.
+struct ShadeOne {
+    MeshDev mesh;
+    LightDev lights[kMaxLights];
+};
 
 // Raster setup record, 48 B: the triangle's float screen vertices (the
 // raster snaps them to 16.16 for coverage), NDC z per vertex, 1 / the float
@@ -237,7 +251,7 @@ struct __align__(16) FrameDev {
     uint32_t* row_base;        // row_blocks x num_bins: a block's first entry in each bin it touched, bin-relative
     uint32_t row_blocks;       // blocks of the count and fill passes (0: sub-counters)
     uint32_t touch_words;      // block rows: 16-byte words of the list the count pass zeroes (list_touch_kernel)
-    uint32_t* shade_list;      // two-pass shading: covered pixels' indices, width x height slots (null: one pass)
+    uint2* shade_list;         // two-pass shading: covered pixels' indices and winners, width x height slots (null: one pass)
     // bin-scan waits: polls of one flag before a wait gives up (0: the
     // library's bound), and 1 + the index of a tile that publishes nothing
     // (0: none) -- the test hook that makes a bounded wait run out
@@ -254,6 +268,7 @@ struct __align__(16) FrameDev {
     uint32_t px_begin, px_end;
     uint32_t rec_tma;          // raster: setup records staged by bulk asynchronous copies (1) or loads (0)
     uint32_t raster_lanes;     // raster: the small-triangle variant (a lane per triangle; phases >= kLanePhase)
+    uint32_t fused_scan;       // the fill pass scans the bins' counts itself (no scan kernel)
     uint32_t block_threads;    // block raster: threads per CTA, 128 or 512
     // two-pass shading of a sparse frame: one byte per bin, "may hold drawn
     // pixels".  dirty_rd: after the last frame; dirty_wr: this frame's, zeroed
@@ -556,7 +571,8 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 // latency, so several must be in flight per lane.
 // Mode 0: count (atomicAdd on the walk's sub-counter of the bin; its return,
 // the pair's rank there, is kept in the walk's rank slots), 1: fill (entry
-// at the sub-counter's list start + rank: no atomics), 2: predicted fill (append within the bin's predicted
+// at the sub-counter's list start + rank: no atomics; 4: at the bin's offset
+// in `s_off` + rank), 2: predicted fill (append within the bin's predicted
 // capacity), 3: pre-pass count (atomicAdd on the first feature slot).  A
 // walk is identified by `walk` (its first triangle slot / 32), so the count
 // and fill passes of the same triangles meet the same slots.  One atomic per
@@ -569,7 +585,8 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 constexpr uint32_t kPairsPerLane = GBR_PAIRS_PER_LANE;
 
 template <int MODE>
-__device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t entry, bool valid, uint32_t walk) {
+__device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t entry, bool valid, uint32_t walk,
+                                         const uint32_t* s_off = nullptr) {
     __shared__ uint4 s_tab[8][32];   // per warp: (first pair, width, bx0 | by0 << 16, entry) of each lane
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t bx0 = rect.x & 0xFFFFu, bx1 = rect.x >> 16;
@@ -598,7 +615,7 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
             F.walk_base[walk] = wb;
         }
         wb = __shfl_sync(0xFFFFFFFFu, wb, 0);
-    } else if (MODE == 1) {
+    } else if (MODE == 1 || MODE == 4) {
         wb = __ldg(&F.walk_base[walk]);
     }
     s_tab[warp][lane] = make_uint4(excl, w, bx0 | (by0 << 16), entry);
@@ -644,14 +661,14 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
                 const unsigned long long slot = (unsigned long long)wb + base + u * 32u + lane;
                 if (act[u] && slot < F.rank_cap) F.ranks[slot] = rank[u];
             }
-        } else if (MODE == 1) {
+        } else if (MODE == 1 || MODE == 4) {
             // fill: the sub-counter's list start plus the rank the count pass kept
             uint32_t rank[kPairsPerLane];
 #pragma unroll
             for (uint32_t u = 0; u < kPairsPerLane; ++u) rank[u] = act[u] ? __ldg(&F.ranks[wb + base + u * 32u + lane]) : 0u;
 #pragma unroll
             for (uint32_t u = 0; u < kPairsPerLane; ++u)
-                if (act[u]) F.list[__ldg(&F.sub_base[krow + bin[u]]) + rank[u]] = ent[u];
+                if (act[u]) F.list[(MODE == 4 ? s_off[bin[u]] : __ldg(&F.sub_base[krow + bin[u]])) + rank[u]] = ent[u];
         } else {
             uint32_t pos[kPairsPerLane];
 #pragma unroll

@@ -39,7 +39,7 @@ __global__ void draw_texture_global_kernel(uint32_t* colour, TexDev tex, int str
     if (x >= width || y >= height) return;
     const float u = __fdiv_rn((float)x, (float)(stretch ? width : tex.w));
     const float v = __fdiv_rn((float)y, (float)(stretch ? height : tex.h));
-    const F3 c = sample == 1u ? sample_linear(tex, u, v) : sample == 2u ? sample_bilinear(tex, u, v) : sample_point(tex, u, v);
+    const F3 c = sample_tex(tex, u, v, sample);
     colour[x + y * width] = rgba_from_colour(c);
 }
 

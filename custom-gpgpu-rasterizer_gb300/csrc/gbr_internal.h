@@ -87,7 +87,7 @@ struct gbr_renderer {
     float* d_depth = nullptr;
     uint32_t* d_ids = nullptr;
     unsigned long long* d_gvis = nullptr;
-    uint32_t* d_shade_list = nullptr;   // two-pass shading queue, W x H (allocated on first use)
+    uint2* d_shade_list = nullptr;      // two-pass shading queue, W x H (allocated on first use)
 
     uint32_t* d_counts = nullptr;     // kCountSplit x bins
     uint32_t* d_sub_base = nullptr;   // kCountSplit x bins
@@ -121,6 +121,7 @@ struct gbr_renderer {
     gbr::Ctl* h_ctl = nullptr;
 
     gbr::LightDev* d_lights = nullptr;   // kMaxLights records
+    gbr::LightDev lights[gbr::kMaxLights] = {};   // the same on the host
     uint32_t num_lights = 0;
 
     bool have_frame = false;

@@ -214,23 +214,120 @@ __global__ void __launch_bounds__(256) setup_kernel(FrameDev F) {
     pdl_release();
 }
 
+// The bin scan inside the fill pass (F.fused_scan): every block scans all the
+// bins' counts in its shared memory instead of waiting for a scan kernel's
+// launch, its tiles' look-back and the offsets' way through memory.  A warp
+// takes a contiguous range of 32-bin rows; row r's
+// offsets and work items are written by block r mod grid, the totals by block
+// 0.  Returns false for a frame that exceeds the storage (flagged, not
+// filled).  The counts stay as they are, for the other blocks: the raster
+// zeroes them.
+template <uint32_t THREADS>
+__device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
+    constexpr uint32_t kWarps = THREADS / 32u;
+    __shared__ unsigned long long s_a[kWarps], s_b[kWarps];
+    const uint32_t nb = F.num_bins, lane = lane_id(), warp = threadIdx.x >> 5, chunk = F.chunk;
+    const uint32_t rows = (nb + 31u) / 32u, per = (rows + kWarps - 1u) / kWarps;
+    const uint32_t r0 = min(warp * per, rows), r1 = min(r0 + per, rows);
+    unsigned long long a = 0, b = 0;   // entries, work items
+#pragma unroll 4
+    for (uint32_t r = r0; r < r1; ++r) {
+        const uint32_t i = r * 32u + lane;
+        const uint32_t c = i < nb ? F.counts[i] : 0u;
+        if (i < nb) s_off[i] = c;
+        a += c;
+        b += (c + chunk - 1u) / chunk;
+    }
+#pragma unroll
+    for (uint32_t d = 16; d > 0; d >>= 1) {
+        a += __shfl_xor_sync(0xFFFFFFFFu, a, d);
+        b += __shfl_xor_sync(0xFFFFFFFFu, b, d);
+    }
+    if (lane == 0u) {
+        s_a[warp] = a;
+        s_b[warp] = b;
+    }
+    __syncthreads();
+    unsigned long long total = 0, items = 0, at64 = 0, item64 = 0;
+#pragma unroll 8
+    for (uint32_t w = 0; w < kWarps; ++w) {
+        if (w == warp) {
+            at64 = total;
+            item64 = items;
+        }
+        total += s_a[w];
+        items += s_b[w];
+    }
+    const bool fits = total <= F.list_cap && items <= F.items_cap;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        F.ctl->num_pairs = total;
+        F.ctl->num_items = fits ? (uint32_t)items : 0u;
+        F.ctl->items_alloc = items;
+        F.ctl->item_next = 0u;
+        if (fits) F.offsets[nb] = (uint32_t)total;
+        else F.ctl->overflow = 1u;
+    }
+    if (F.dirty_wr)
+        for (uint32_t i = blockIdx.x * THREADS + threadIdx.x; i < nb; i += gridDim.x * THREADS) F.dirty_wr[i] = 0u;
+    if (!fits) return false;
+    uint32_t at = (uint32_t)at64, item = (uint32_t)item64;   // the totals fit 32 bits
+    for (uint32_t r = r0; r < r1; ++r) {
+        const uint32_t i = r * 32u + lane;
+        const uint32_t c = i < nb ? s_off[i] : 0u, it = (c + chunk - 1u) / chunk;
+        uint32_t x = c, y = it;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, d), u = __shfl_up_sync(0xFFFFFFFFu, y, d);
+            if (lane >= d) {
+                x += t;
+                y += u;
+            }
+        }
+        const uint32_t start = at + x - c;
+        if (i < nb) {
+            s_off[i] = start;
+            if (r % gridDim.x == blockIdx.x) {
+                F.offsets[i] = start;
+                for (uint32_t k = 0; k < it; ++k)
+                    F.items[item + y - it + k] = make_uint4(i, start + k * chunk, min(chunk, c - k * chunk), it);
+            }
+        }
+        at += __shfl_sync(0xFFFFFFFFu, x, 31);
+        item += __shfl_sync(0xFFFFFFFFu, y, 31);
+    }
+    __syncthreads();
+    return true;
+}
+
 // The list entry of triangle `prim` with rectangle `rect`, in a fill pass.
 __device__ __forceinline__ uint32_t rect_entry(const FrameDev& F, uint32_t prim, uint2 rect, bool in_range) {
     return list_entry(prim, in_range && F.key_mask ? F.keys[prim] : 0u, (rect.y & 0x80000000u) != 0u, F.key_mask);
 }
 
 // Second pass of exact binning for triangle `prim`.  Called by whole warps.
-__device__ __forceinline__ void fill_tri(const FrameDev& F, uint32_t prim, uint32_t walk) {
+// s_off: the bins' offsets of a fused scan (MODE 4).
+template <int MODE>
+__device__ __forceinline__ void fill_tri(const FrameDev& F, uint32_t prim, uint32_t walk, const uint32_t* s_off = nullptr) {
     const bool in_range = prim < F.num_tris;
     const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-    bin_walk<1>(F, rect, rect_entry(F, prim, rect, in_range), in_range, walk);
+    bin_walk<MODE>(F, rect, rect_entry(F, prim, rect, in_range), in_range, walk, s_off);
 }
 
 __global__ void __launch_bounds__(256) fill_kernel(FrameDev F) {
     pdl_wait();
     if (F.ctl->overflow || (F.exact_guard && !F.ctl->pred_overflow)) return;
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x)
-        fill_tri(F, base + threadIdx.x, (base + threadIdx.x) >> 5);
+        fill_tri<1>(F, base + threadIdx.x, (base + threadIdx.x) >> 5);
+    pdl_release();
+}
+
+// The same with the scan in it (at most kFusedBins bins, one counter a bin).
+__global__ void __launch_bounds__(256) fill_fused_kernel(FrameDev F) {
+    __shared__ uint32_t s_off[kFusedBins];
+    pdl_wait();
+    if (!fused_scan<256>(F, s_off)) return;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x)
+        fill_tri<4>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, s_off);
     pdl_release();
 }
 
@@ -301,10 +398,15 @@ __global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F) 
 __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
     extern __shared__ uint32_t s_row[];
     pdl_wait();
-    if (F.ctl->overflow) return;
     const uint32_t nb = F.num_bins;
     const uint32_t* const row = F.row_base + (size_t)blockIdx.x * nb;
-    for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] = __ldg(F.offsets + b) + __ldg(row + b);
+    if (F.fused_scan) {
+        if (!fused_scan<kRowThreads>(F, s_row)) return;
+        for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] += __ldg(row + b);
+    } else {
+        if (F.ctl->overflow) return;
+        for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] = __ldg(F.offsets + b) + __ldg(row + b);
+    }
     __syncthreads();
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x) {
         const uint32_t prim = base + threadIdx.x;
@@ -577,16 +679,12 @@ __device__ __forceinline__ void clear_pixel(const FrameDev& F, size_t gi) {
 // or by depth.
 enum ShadeKind { kShadeFull, kShadeFlat, kShadeFlatOne, kShadeDepth };
 
-// Pixel (x, y) with raster result v: the winner's weights and depth as the
-// raster computed them, its colour, and the three outputs.
+// Pixel (x, y), won by `prim`: the winner's weights and depth as the raster
+// computed them, its colour, and the three outputs.  ONE: the frame's only
+// mesh and its lights (null: looked up).
 template <ShadeKind KIND>
-__device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, unsigned long long v) {
+__device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, uint32_t prim, const ShadeOne* one = nullptr) {
     const size_t gi = (size_t)y * F.width + (size_t)x;
-    if (v == kEmptyVis) {
-        clear_pixel(F, gi);
-        return;
-    }
-    const uint32_t prim = (uint32_t)(v & 0xFFFFFFFFull);
     const uint4* rp = reinterpret_cast<const uint4*>(F.setup) + 3u * (size_t)prim;
     const uint4 a = __ldg(rp), b = __ldg(rp + 1), c = __ldg(rp + 2);
     TriSetup t;
@@ -601,9 +699,12 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
         F.colour[gi] = shade_flat(F.one, prim, w);
     } else if (KIND == kShadeDepth) {
         F.colour[gi] = shade_depth(z);
+    } else if (one) {
+        F.colour[gi] = shade_fragment(F, one->mesh, one->lights, prim, w, z);
     } else {
         const MeshDev& m = F.meshes[t.mesh & kMeshMask];
-        F.colour[gi] = KIND == kShadeFlat ? shade_flat(flat_mesh(m), prim - m.prim_base, w) : shade_fragment(F, m, prim, w, z);
+        F.colour[gi] = KIND == kShadeFlat ? shade_flat(flat_mesh(m), prim - m.prim_base, w)
+                                          : shade_fragment(F, m, F.lights, prim, w, z);
     }
     F.depth[gi] = z;
     F.ids[gi] = prim;
@@ -622,8 +723,9 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
     pdl_wait();
     Ctl* const Q = F.ctl;
     const uint4* const items = F.items;
-    if (Q->overflow) return;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    zero_counts(F);
+    if (Q->overflow) return;
     const uint32_t num_items = Q->num_items;
     const uint32_t phase = F.phase == 0u ? kPhase : min(F.phase, kMaxPhase);
     const uint32_t pass = F.stage == 0u ? kEntries : min(F.stage, kEntries);   // entries per raster pass
@@ -851,8 +953,13 @@ __device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint3
     for (uint32_t k = 0; k < 2u; ++k) {
         const uint32_t yk = y + k * (kTileH / 2u);
         if (yk >= y1) break;
-        if (v[k] != kEmptyVis) F.gvis[(size_t)yk * F.width + x] = kEmptyVis;
-        resolve_pixel<KIND>(F, (int)x, (int)yk, v[k]);
+        const size_t i = (size_t)yk * F.width + x;
+        if (v[k] == kEmptyVis) {
+            clear_pixel(F, i);
+            continue;
+        }
+        F.gvis[i] = kEmptyVis;
+        resolve_pixel<KIND>(F, (int)x, (int)yk, (uint32_t)v[k]);
     }
 }
 
@@ -938,10 +1045,12 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
         if (!__any_sync(0xFFFFFFFFu, live)) return;   // the warp's 128 pixels already hold the clear values
     }
     uint32_t covered = 0;   // bit k: pixel i0 + k has a winner
+    uint32_t won[4] = {0u, 0u, 0u, 0u};
     if (!live) {
     } else if (aligned && i0 + 4u <= n) {
-        const ulonglong2* g = reinterpret_cast<const ulonglong2*>(F.gvis + i0);
+        ulonglong2* g = reinterpret_cast<ulonglong2*>(F.gvis + i0);
         const ulonglong2 a = g[0], b = g[1];
+        won[0] = (uint32_t)a.x; won[1] = (uint32_t)a.y; won[2] = (uint32_t)b.x; won[3] = (uint32_t)b.y;
         covered = (a.x != kEmptyVis ? 1u : 0u) | (a.y != kEmptyVis ? 2u : 0u) | (b.x != kEmptyVis ? 4u : 0u) |
                   (b.y != kEmptyVis ? 8u : 0u);
         if (covered == 0u) {
@@ -949,14 +1058,24 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
             *reinterpret_cast<uint4*>(F.colour + i0) = make_uint4(c, c, c, c);
             *reinterpret_cast<float4*>(F.depth + i0) = make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<uint4*>(F.ids + i0) = make_uint4(kInvalidPrim, kInvalidPrim, kInvalidPrim, kInvalidPrim);
-        } else {
+        } else {   // the merge words are left empty for the next frame
+            g[0] = g[1] = make_ulonglong2(kEmptyVis, kEmptyVis);
+#pragma unroll
             for (uint32_t k = 0; k < 4u; ++k)
                 if (!((covered >> k) & 1u)) clear_pixel(F, i0 + k);
         }
     } else {
-        for (uint32_t k = 0; k < 4u && i0 + k < n; ++k) {
-            if (F.gvis[i0 + k] != kEmptyVis) covered |= 1u << k;
-            else clear_pixel(F, i0 + k);
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            if (i0 + k >= n) break;
+            const unsigned long long v = F.gvis[i0 + k];
+            if (v == kEmptyVis) {
+                clear_pixel(F, i0 + k);
+                continue;
+            }
+            covered |= 1u << k;
+            won[k] = (uint32_t)v;
+            F.gvis[i0 + k] = kEmptyVis;
         }
     }
     // the warp's covered pixels go to the queue in one run
@@ -973,24 +1092,30 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
         if (lane == 31u) base = atomicAdd(&F.ctl->shade_count, total);
         base = __shfl_sync(0xFFFFFFFFu, base, 31);
         uint32_t at = base + incl - c;
+#pragma unroll
         for (uint32_t k = 0; k < 4u; ++k)
-            if ((covered >> k) & 1u) F.shade_list[at++] = i0 + k;
+            if ((covered >> k) & 1u) F.shade_list[at++] = make_uint2(i0 + k, won[k]);
     }
     pdl_release();
 }
 
-// 4 blocks per SM (<= 64 registers): the heavy pass is bound by the latency
-// of its dependent loads, and a 4K frame's covered pixels then fit in one
-// resident wave (3 blocks per SM at 80 registers: 71.7 -> 63.5 us with 4).
-__global__ void __launch_bounds__(256, 4) shade_list_kernel(FrameDev F) {
+// 2 blocks per SM (<= 128 registers): the heavy pass is bound by the latency
+// of a pixel's chain of dependent loads, and the registers keep the four
+// maps' texels in flight (640x480 sphere frame 36.8 us with 4 blocks, 36.5
+// with 3, 35.0 with 2; lit 4K icosphere-6 74.8, 75.8, 72.8; before the maps
+// were fetched together, with the mesh looked up: 39.1 and 74.4).
+// A pixel's chain is queue -> record and indices -> vertices -> texels: the
+// queue holds the winner, a frame's only mesh comes by value (ONE), and the
+// four maps are fetched together.
+template <bool ONE>
+__global__ void __launch_bounds__(256, 2) shade_list_kernel(FrameDev F, const __grid_constant__ ShadeOne one) {
     pdl_wait();
     if (F.ctl->overflow) return;
     const uint32_t count = F.ctl->shade_count;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
-        const uint32_t i = __ldg(F.shade_list + j);
-        const unsigned long long v = F.gvis[i];
-        F.gvis[i] = kEmptyVis;
-        resolve_pixel<kShadeFull>(F, (int)(i % F.width), (int)(i / F.width), v);
+        const uint2 e = __ldg(F.shade_list + j);
+        const uint32_t y = e.x / F.width;
+        resolve_pixel<kShadeFull>(F, (int)(e.x - y * F.width), (int)y, e.y, ONE ? &one : nullptr);
     }
 }
 
@@ -1073,7 +1198,7 @@ __global__ void __launch_bounds__(256) batch_fill_kernel(BatchDev B) {
     __shared__ __align__(16) FrameDev sF;
     const uint32_t sc = __ldg(B.tri_scene + blockIdx.x);
     load_scene(B, sc, sF);
-    fill_tri(sF, (blockIdx.x - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x, (blockIdx.x * 256u + threadIdx.x) >> 5);
+    fill_tri<1>(sF, (blockIdx.x - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x, (blockIdx.x * 256u + threadIdx.x) >> 5);
 }
 
 // KIND: every scene of the batch shades flat (B.all_flat), from one mesh, and
@@ -1163,7 +1288,7 @@ cudaError_t launch_fill(const FrameDev& F, cudaStream_t s) {
     }
     const uint32_t blocks = triangle_blocks(F.num_tris);
     if (blocks == 0) return cudaSuccess;
-    return launch_pdl(fill_kernel, dim3(blocks), dim3(256), 0, s, F);
+    return launch_pdl(F.fused_scan ? fill_fused_kernel : fill_kernel, dim3(blocks), dim3(256), 0, s, F);
 }
 
 static size_t record_smem(uint32_t bw, uint32_t bh) {
@@ -1207,7 +1332,7 @@ cudaError_t launch_raster(const FrameDev& F, const RasterGrid& per_sm, cudaStrea
                                (uint32_t)(sm_count() * per_sm.block(F.block_threads)), s);
 }
 
-cudaError_t launch_shade(const FrameDev& F, cudaStream_t s) {
+cudaError_t launch_shade(const FrameDev& F, const ShadeOne* one, cudaStream_t s) {
     const dim3 b(256);
     if (!F.flat_shade && F.shade_list) {
         const uint32_t npx = (F.px_end ? F.px_end : F.width * F.height) - F.px_begin;
@@ -1216,11 +1341,15 @@ cudaError_t launch_shade(const FrameDev& F, cudaStream_t s) {
         // one resident wave: the queue is a few pixels per thread at most
         static int per_sm = 0;
         if (per_sm <= 0 &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shade_list_kernel, 256, 0) != cudaSuccess) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shade_list_kernel<true>, 256, 0) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 2;
         }
-        return launch_pdl(shade_list_kernel, dim3((uint32_t)std::max(per_sm, 1) * (uint32_t)sm_count()), b, 0, s, F);
+        const dim3 g((uint32_t)std::max(per_sm, 1) * (uint32_t)sm_count());
+        if (one) return launch_pdl(shade_list_kernel<true>, g, b, 0, s, F, *one);
+        ShadeOne none;
+        memset(&none, 0, sizeof none);
+        return launch_pdl(shade_list_kernel<false>, g, b, 0, s, F, none);
     }
     const uint32_t y0 = F.row1 ? F.row0 * F.bh : 0u, y1 = F.row1 ? std::min(F.row1 * F.bh, F.height) : F.height;
     if (y0 >= y1) return cudaSuccess;   // a band below the screen

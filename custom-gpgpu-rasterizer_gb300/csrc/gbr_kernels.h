@@ -57,7 +57,8 @@ cudaError_t launch_fill(const FrameDev& F, cudaStream_t s);
 constexpr unsigned long long kListTouchMinPairs = 1ull << 20;
 cudaError_t launch_list_touch(const FrameDev& F, cudaStream_t s);
 cudaError_t launch_raster(const FrameDev& F, const RasterGrid& per_sm, cudaStream_t s);
-cudaError_t launch_shade(const FrameDev& F, cudaStream_t s);
+// one: the mesh and lights of a frame of one mesh (null otherwise)
+cudaError_t launch_shade(const FrameDev& F, const ShadeOne* one, cudaStream_t s);
 cudaError_t launch_clear(const FrameDev& F, cudaStream_t s);
 
 // Grid sizes of a batch frame (see BatchDev).

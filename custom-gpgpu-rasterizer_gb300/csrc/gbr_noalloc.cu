@@ -164,6 +164,8 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     F.num_tris = (uint32_t)tris;
     F.key_mask = key_mask_for(tris);
     F.chunk = kMaxChunk;      // work items: the library's split
+    F.fused_scan = tris > 0u ? 1u : 0u;   // the scratch's limits are the fused scan's
+    static_assert(kNaMaxBins <= kFusedBins && kNaMaxTris <= kFusedTris, "fused scan limits");
     F.stage = queue_chunk;    // entries per raster pass
     F.block_threads = block_threads_for(nb, (uint32_t)slot.num_sms);
     for (int k = 0; k < 3; ++k) { F.cam_pos[k] = cam->pos[k]; F.cam_fwd[k] = cam->fwd[k]; }
@@ -216,10 +218,10 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     if (e == cudaSuccess && ((uint64_t)num_bins_x * bin_w < width || (uint64_t)num_bins_y * bin_h < height))
         e = launch_clear(F, s);
     if (e == cudaSuccess) e = launch_setup(F, false, s);
-    if (e == cudaSuccess) e = launch_scan(scan_of(F, kScanExact), s);
+    if (e == cudaSuccess && !F.fused_scan) e = launch_scan(scan_of(F, kScanExact), s);
     if (e == cudaSuccess) e = launch_fill(F, s);
     if (e == cudaSuccess) e = launch_raster(F, per_sm, s);
-    if (e == cudaSuccess) e = launch_shade(F, s);
+    if (e == cudaSuccess) e = launch_shade(F, nullptr, s);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
     // the frame is only valid if its bin entries fitted the static storage
     e = cudaStreamSynchronize(s);

@@ -17,4 +17,11 @@ __device__ __forceinline__ void fetch_item(uint4* dst, const uint4* items, uint3
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(items + idx) : "memory");
 }
 
+// After a fill pass with the scan in it, the raster leaves the bins' counts
+// zero for the next frame.
+__device__ __forceinline__ void zero_counts(const FrameDev& F) {
+    if (F.fused_scan)
+        for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < F.num_bins; b += gridDim.x * blockDim.x) F.counts[b] = 0u;
+}
+
 }  // namespace gbr

@@ -77,75 +77,98 @@ __device__ __forceinline__ F3 rgb_of(uint32_t c) {   // byte / 255 per channel
     return f3(over255(c & 0xFFu), over255((c >> 8) & 0xFFu), over255((c >> 16) & 0xFFu));
 }
 
-// SamplePoint (CUDATextureSampler.cuh:87-104): u = int(uv.x*w + 0.5);
-// out of range samples magenta.
-__device__ __forceinline__ F3 sample_point(const TexDev& t, float u, float v) {
-    const int x = cvt_s32(__fmaf_rn(u, (float)t.w, 0.5f));
-    const int y = cvt_s32(__fmaf_rn(v, (float)t.h, 0.5f));
-    if (x < 0 || y < 0 || (uint32_t)x >= t.w || (uint32_t)y >= t.h) return f3(1.f, 0.f, 1.f);
-    return rgb_of(__ldg(t.px + (uint32_t)x + (uint32_t)y * t.w));
-}
+// A texture lookup in two halves, so that a pixel's four maps are all on
+// their way before the first texel is converted: fetch() loads the texels
+// (and keeps the bilinear fractions), colour() combines them.  SS: the
+// sample state.
+template <uint32_t SS>
+struct Lookup {
+    static constexpr int kTaps = SS == 0u ? 1 : SS == 1u ? 5 : 4;
+    uint32_t c[kTaps];
+    float ax, ay;
+    bool in;
 
-// SampleLinear (CUDATextureSampler.cuh:112-190): centre at 1/2 plus the four
-// row-major neighbours at 1/8 each (wrapping across rows, clamped at the
-// buffer ends).
-__device__ __forceinline__ F3 sample_linear(const TexDev& t, float u, float v) {
-    const int x = cvt_s32(__fmaf_rn(u, (float)t.w, 0.5f));
-    const int y = cvt_s32(__fmaf_rn(v, (float)t.h, 0.5f));
-    if (x < 0 || y < 0 || (uint32_t)x >= t.w || (uint32_t)y >= t.h) return f3(1.f, 0.f, 1.f);
-    const int size = (int)(t.w * t.h);
-    const int o = x + y * (int)t.w;
-    int nb[4];
-    nb[0] = o - 1; if (nb[0] < 0) nb[0] = o;
-    nb[1] = o + 1; if (nb[1] >= size) nb[1] = o;
-    nb[2] = o + (int)t.w; if (nb[2] >= size) nb[2] = o;
-    nb[3] = o - (int)t.w; if (nb[3] < 0) nb[3] = o;
-    const float wt = __fdiv_rn(1.f, 8.f);
-    float r = 0.f, g = 0.f, b = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t c = __ldg(t.px + nb[i]);
-        r = __fmaf_rn((float)(c & 0xFFu), wt, r);
-        g = __fmaf_rn((float)((c >> 8) & 0xFFu), wt, g);
-        b = __fmaf_rn((float)((c >> 16) & 0xFFu), wt, b);
+    __device__ __forceinline__ void fetch(const TexDev& t, float u, float v) {
+        in = true;
+        if (SS == 2u) {
+            // bilinear filtering (the build's extension, GBR_SAMPLE_BILINEAR):
+            // texel centres at (i + 1/2) / size, the four nearest texels
+            // weighted by the fractional offsets, addresses clamped to the
+            // texture
+            const float x = __fmaf_rn(u, (float)t.w, -0.5f), y = __fmaf_rn(v, (float)t.h, -0.5f);
+            const float fx = floorf(x), fy = floorf(y);
+            ax = __fsub_rn(x, fx);
+            ay = __fsub_rn(y, fy);
+            const int w = (int)t.w, h = (int)t.h;
+            int xi = cvt_s32(fx), yi = cvt_s32(fy);
+            xi = xi < -1 ? -1 : (xi > w - 1 ? w - 1 : xi);
+            yi = yi < -1 ? -1 : (yi > h - 1 ? h - 1 : yi);
+            const uint32_t x0 = (uint32_t)(xi < 0 ? 0 : xi), x1 = (uint32_t)(xi + 1 > w - 1 ? w - 1 : xi + 1);
+            const uint32_t y0 = (uint32_t)(yi < 0 ? 0 : yi), y1 = (uint32_t)(yi + 1 > h - 1 ? h - 1 : yi + 1);
+            c[0] = __ldg(t.px + x0 + y0 * t.w);
+            c[1 % kTaps] = __ldg(t.px + x1 + y0 * t.w);
+            c[2 % kTaps] = __ldg(t.px + x0 + y1 * t.w);
+            c[3 % kTaps] = __ldg(t.px + x1 + y1 * t.w);
+            return;
+        }
+        // SamplePoint (CUDATextureSampler.cuh:87-104): u = int(uv.x*w + 0.5);
+        // out of range samples magenta
+        const int x = cvt_s32(__fmaf_rn(u, (float)t.w, 0.5f));
+        const int y = cvt_s32(__fmaf_rn(v, (float)t.h, 0.5f));
+        in = !(x < 0 || y < 0 || (uint32_t)x >= t.w || (uint32_t)y >= t.h);
+        if (!in) return;
+        if (SS == 0u) {
+            c[0] = __ldg(t.px + (uint32_t)x + (uint32_t)y * t.w);
+            return;
+        }
+        // SampleLinear (CUDATextureSampler.cuh:112-190): the centre and its
+        // four row-major neighbours (wrapping across rows, clamped at the
+        // buffer ends)
+        const int size = (int)(t.w * t.h);
+        const int o = x + y * (int)t.w;
+        c[0] = __ldg(t.px + (o - 1 < 0 ? o : o - 1));
+        c[1 % kTaps] = __ldg(t.px + (o + 1 >= size ? o : o + 1));
+        c[2 % kTaps] = __ldg(t.px + (o + (int)t.w >= size ? o : o + (int)t.w));
+        c[3 % kTaps] = __ldg(t.px + (o - (int)t.w < 0 ? o : o - (int)t.w));
+        c[4 % kTaps] = __ldg(t.px + o);
     }
-    const uint32_t c = __ldg(t.px + o);
-    r = __fadd_rn(r, __fdiv_rn((float)(c & 0xFFu), 2.f));
-    g = __fadd_rn(g, __fdiv_rn((float)((c >> 8) & 0xFFu), 2.f));
-    b = __fadd_rn(b, __fdiv_rn((float)((c >> 16) & 0xFFu), 2.f));
-    const float rev = __fdiv_rn(1.0f, 255.f);
-    return f3(__fmul_rn(r, rev), __fmul_rn(g, rev), __fmul_rn(b, rev));
-}
 
-// Bilinear filtering (the build's extension, GBR_SAMPLE_BILINEAR): texel
-// centres at (i + 1/2) / size, the four nearest texels weighted by the
-// fractional offsets, addresses clamped to the texture.
-__device__ __forceinline__ F3 sample_bilinear(const TexDev& t, float u, float v) {
-    const float x = __fmaf_rn(u, (float)t.w, -0.5f), y = __fmaf_rn(v, (float)t.h, -0.5f);
-    const float fx = floorf(x), fy = floorf(y);
-    const float ax = __fsub_rn(x, fx), ay = __fsub_rn(y, fy);
-    const int w = (int)t.w, h = (int)t.h;
-    int xi = cvt_s32(fx), yi = cvt_s32(fy);
-    xi = xi < -1 ? -1 : (xi > w - 1 ? w - 1 : xi);
-    yi = yi < -1 ? -1 : (yi > h - 1 ? h - 1 : yi);
-    const uint32_t x0 = (uint32_t)(xi < 0 ? 0 : xi), x1 = (uint32_t)(xi + 1 > w - 1 ? w - 1 : xi + 1);
-    const uint32_t y0 = (uint32_t)(yi < 0 ? 0 : yi), y1 = (uint32_t)(yi + 1 > h - 1 ? h - 1 : yi + 1);
-    const uint32_t c00 = __ldg(t.px + x0 + y0 * t.w), c10 = __ldg(t.px + x1 + y0 * t.w);
-    const uint32_t c01 = __ldg(t.px + x0 + y1 * t.w), c11 = __ldg(t.px + x1 + y1 * t.w);
-    float out[3];
+    __device__ __forceinline__ F3 colour() const {
+        if (!in) return f3(1.f, 0.f, 1.f);
+        float out[3];
+        if (SS == 0u) {
+            const F3 p = rgb_of(c[0]);
+            out[0] = p.x; out[1] = p.y; out[2] = p.z;
+        } else
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float a = (float)((c00 >> (8 * k)) & 0xFFu), b = (float)((c10 >> (8 * k)) & 0xFFu);
-        const float c = (float)((c01 >> (8 * k)) & 0xFFu), d = (float)((c11 >> (8 * k)) & 0xFFu);
-        const float top = __fmaf_rn(ax, __fsub_rn(b, a), a), bottom = __fmaf_rn(ax, __fsub_rn(d, c), c);
-        out[k] = __fmul_rn(__fmaf_rn(ay, __fsub_rn(bottom, top), top), __fdiv_rn(1.0f, 255.f));
+        for (int k = 0; k < 3; ++k) {
+            const float a = (float)((c[0] >> (8 * k)) & 0xFFu), b = (float)((c[1 % kTaps] >> (8 * k)) & 0xFFu);
+            const float d = (float)((c[2 % kTaps] >> (8 * k)) & 0xFFu), f = (float)((c[3 % kTaps] >> (8 * k)) & 0xFFu);
+            if (SS == 2u) {
+                const float top = __fmaf_rn(ax, __fsub_rn(b, a), a), bottom = __fmaf_rn(ax, __fsub_rn(f, d), d);
+                out[k] = __fmul_rn(__fmaf_rn(ay, __fsub_rn(bottom, top), top), 1.0f / 255.f);
+            } else {   // the neighbours at 1/8 each, the centre at 1/2
+                const float wt = 0.125f;
+                float s = __fmaf_rn(a, wt, 0.f);
+                s = __fmaf_rn(b, wt, s);
+                s = __fmaf_rn(d, wt, s);
+                s = __fmaf_rn(f, wt, s);
+                s = __fadd_rn(s, __fmul_rn((float)((c[4 % kTaps] >> (8 * k)) & 0xFFu), 0.5f));
+                out[k] = __fmul_rn(s, 1.0f / 255.f);
+            }
+        }
+        return f3(out[0], out[1], out[2]);
     }
-    return f3(out[0], out[1], out[2]);
-}
+};
 
+template <uint32_t SS>
+__device__ __forceinline__ F3 sample_as(const TexDev& t, float u, float v) {
+    Lookup<SS> l;
+    l.fetch(t, u, v);
+    return l.colour();
+}
 __device__ __forceinline__ F3 sample_tex(const TexDev& t, float u, float v, uint32_t ss) {
-    if (ss == 2u) return sample_bilinear(t, u, v);
-    return ss == 1u ? sample_linear(t, u, v) : sample_point(t, u, v);
+    return ss == 2u ? sample_as<2>(t, u, v) : ss == 1u ? sample_as<1>(t, u, v) : sample_as<0>(t, u, v);
 }
 
 // Lambert + Phong over the scene lights (the build's extension, used when
@@ -157,13 +180,13 @@ __device__ __forceinline__ F3 sample_tex(const TexDev& t, float u, float v, uint
 // colour * clamp(dot(vd, reflect(L, N)), 0, 1)^(gloss * 25); then ambient +
 // diffuse + specular and MaxToOne (CUDAROPs.cu:452-455), or the diffuse
 // term alone without the specular and gloss maps (:459-462).
-__device__ __forceinline__ F3 shade_lit(const FrameDev& F, F3 diffuse, F3 fn, F3 vd, F3 P, bool has_spec, F3 spec,
+__device__ __forceinline__ F3 shade_lit(const LightDev* lights, uint32_t num_lights, F3 diffuse, F3 fn, F3 vd, F3 P, bool has_spec, F3 spec,
                                         F3 gloss) {
     F3 dacc = f3(0.f, 0.f, 0.f), sacc = f3(0.f, 0.f, 0.f);
     const F3 nfn = f3(-fn.x, -fn.y, -fn.z);
-    const uint32_t nl = F.num_lights < kMaxLights ? F.num_lights : kMaxLights;
+    const uint32_t nl = num_lights < kMaxLights ? num_lights : kMaxLights;
     for (uint32_t k = 0; k < nl; ++k) {
-        const LightDev lt = F.lights[k];
+        const LightDev& lt = lights[k];
         F3 L;
         float E;
         if (lt.type == 1u) {
@@ -210,24 +233,32 @@ __device__ __forceinline__ uint32_t rgba_from_colour(F3 c) {
 }
 
 // ShadePixelSafe (CUDAROPs.cu:411-470).
-__device__ __forceinline__ F3 shade_pixel_safe(const FrameDev& F, const MeshDev& m, float u, float v, F3 n, F3 tan,
-                                               F3 vd, F3 P, uint32_t ss) {
+template <uint32_t SS>
+__device__ __forceinline__ F3 shade_pixel_safe(const LightDev* lights, uint32_t num_lights, const MeshDev& m, float u,
+                                               float v, F3 n, F3 tan, F3 vd, F3 P) {
     const F3 L = f3(0.577f, -0.577f, -0.577f);
-    const F3 diffuse = sample_tex(m.tex[0], u, v, ss);
+    const bool has_spec = m.tex[1].px && m.tex[2].px && m.tex[3].px;
+    Lookup<SS> ld, ln, ls, lg;
+    ld.fetch(m.tex[0], u, v);
+    if (m.tex[1].px) ln.fetch(m.tex[1], u, v);
+    if (has_spec) {
+        ls.fetch(m.tex[2], u, v);
+        lg.fetch(m.tex[3], u, v);
+    }
+    const F3 diffuse = ld.colour();
     if (!m.tex[1].px) return diffuse;
-    const F3 ns = sample_tex(m.tex[1], u, v, ss);
+    const F3 ns = ln.colour();
     const F3 cr = cross3(tan, n);
     const F3 bin = f3(-cr.x, -cr.y, -cr.z);
     const F3 fn0 = f3(__fmaf_rn(2.f, ns.x, -1.f), __fmaf_rn(2.f, ns.y, -1.f), __fmaf_rn(2.f, ns.z, -1.f));
     const F3 fn = f3(__fmaf_rn(n.x, fn0.z, __fmaf_rn(tan.x, fn0.x, __fmul_rn(bin.x, fn0.y))),
                      __fmaf_rn(n.y, fn0.z, __fmaf_rn(tan.y, fn0.x, __fmul_rn(bin.y, fn0.y))),
                      __fmaf_rn(n.z, fn0.z, __fmaf_rn(tan.z, fn0.x, __fmul_rn(bin.z, fn0.y))));
-    if (F.num_lights) {
-        const bool has_spec = m.tex[2].px && m.tex[3].px;
+    if (num_lights) {
         const F3 zero = f3(0.f, 0.f, 0.f);
-        const F3 spec = has_spec ? sample_tex(m.tex[2], u, v, ss) : zero;
-        const F3 gloss = has_spec ? sample_tex(m.tex[3], u, v, ss) : zero;
-        return shade_lit(F, diffuse, fn, vd, P, has_spec, spec, gloss);
+        const F3 spec = has_spec ? ls.colour() : zero;
+        const F3 gloss = has_spec ? lg.colour() : zero;
+        return shade_lit(lights, num_lights, diffuse, fn, vd, P, has_spec, spec, gloss);
     }
     float obs = dot3(f3(-fn.x, -fn.y, -fn.z), L);
     {   // ClampFast(obs, 0, obs) (CUDAROPs.cu:439) leaves negative values as they are
@@ -237,9 +268,8 @@ __device__ __forceinline__ F3 shade_pixel_safe(const FrameDev& F, const MeshDev&
     obs = __fdiv_rn(obs, 3.14159265358979323846f);
     obs = __fmul_rn(obs, 7.0f);
     const F3 dcol = f3(__fmul_rn(diffuse.x, obs), __fmul_rn(diffuse.y, obs), __fmul_rn(diffuse.z, obs));
-    if (!(m.tex[2].px && m.tex[3].px)) return dcol;
-    const F3 spec = sample_tex(m.tex[2], u, v, ss);
-    const F3 gloss = sample_tex(m.tex[3], u, v, ss);
+    if (!has_spec) return dcol;
+    const F3 spec = ls.colour(), gloss = lg.colour();
     const float s2 = __fmul_rn(2.f, dot3(L, fn));
     const F3 refl = f3(__fmaf_rn(fn.x, s2, -L.x), __fmaf_rn(fn.y, s2, -L.y), __fmaf_rn(fn.z, s2, -L.z));
     float ang = dot3(vd, refl);
@@ -300,8 +330,8 @@ __device__ __forceinline__ uint32_t shade_depth(float z) {
 }
 
 // Colour of the fragment of primitive `prim` with weights w and depth z.
-__device__ __forceinline__ uint32_t shade_fragment(const FrameDev& F, const MeshDev& m, uint32_t prim,
-                                                   const float w[3], float z) {
+__device__ __forceinline__ uint32_t shade_fragment(const FrameDev& F, const MeshDev& m, const LightDev* lights,
+                                                   uint32_t prim, const float w[3], float z) {
     if (F.vis == 1u) return shade_depth(z);
     if (F.vis == 0u && !m.tex[0].px) return shade_flat(flat_mesh(m), prim - m.prim_base, w);
     uint32_t vid[3];
@@ -329,7 +359,11 @@ __device__ __forceinline__ uint32_t shade_fragment(const FrameDev& F, const Mesh
                __fmul_rn(GBR_INTERP(v0.wp.y, v1.wp.y, v2.wp.y), winterp),
                __fmul_rn(GBR_INTERP(v0.wp.z, v1.wp.z, v2.wp.z), winterp));
 #undef GBR_INTERP
-    return rgba_from_colour(shade_pixel_safe(F, m, u, vv, n, tan, vd, P, F.sample));
+    const uint32_t nl = F.num_lights;
+    const F3 c = F.sample == 2u   ? shade_pixel_safe<2>(lights, nl, m, u, vv, n, tan, vd, P)
+                 : F.sample == 1u ? shade_pixel_safe<1>(lights, nl, m, u, vv, n, tan, vd, P)
+                                  : shade_pixel_safe<0>(lights, nl, m, u, vv, n, tan, vd, P);
+    return rgba_from_colour(c);
 }
 
 }  // namespace gbr
