@@ -244,8 +244,12 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     // per-mesh descriptors with the matrices of this frame
     std::vector<MeshDev> md(r->meshes.size());
     if (!md.empty()) build_mesh_table(r, cam, md.data());
-    const bool same = md.size() == r->last_uploaded.size() &&
-                      (md.empty() || memcmp(md.data(), r->last_uploaded.data(), md.size() * sizeof(MeshDev)) == 0);
+    const bool predicted = r->binning == GBR_BINNING_PREDICTED && r->predictor_ready && !r->collect;
+    // a frame of one mesh carries it in its launches' arguments; the
+    // pre-pass reads the table
+    const bool table = md.size() > 1u || predicted || r->collect;
+    const bool same = !table || (md.size() == r->last_uploaded.size() &&
+                                 (md.empty() || memcmp(md.data(), r->last_uploaded.data(), md.size() * sizeof(MeshDev)) == 0));
     if (!same && !md.empty()) {
         GBR_CUDA(cudaEventSynchronize(r->meshes_evt));  // previous copy out of the staging buffer is done
         memcpy(r->h_meshes, md.data(), md.size() * sizeof(MeshDev));
@@ -287,7 +291,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     }
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;
-    if (md.size() == 1u) F.one = flat_mesh(md[0]);
+    const MeshDev* const only = md.size() == 1u ? md.data() : nullptr;
+    if (only) F.one = flat_mesh(*only);
     F.setup = r->d_setup; F.rects = r->d_rects; F.keys = r->d_keys;
     F.counts = r->d_counts; F.sub_base = r->d_sub_base; F.count_stride = nb; F.offsets = r->d_offsets;
     F.cursors = r->d_cursors; F.capacity = r->d_capacity;
@@ -308,7 +313,6 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         F.px_end = std::min(F.row1 * r->bh, r->H) * r->W;
     }
     F.scan_silent_tile1 = r->scan_silent_tile1;
-    const bool predicted = r->binning == GBR_BINNING_PREDICTED && r->predictor_ready && !r->collect;
     F.feat = r->d_feat;
     F.mlp_w = r->sampled_rule ? nullptr : r->d_mlp_w;   // null: capacities from the sampled counts alone
     F.features_out = r->collect ? r->d_features_out : nullptr;
@@ -354,7 +358,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.fused_scan = !predicted && nb <= kFusedBins && F.count_split == 1u && !F.scan_silent_tile1 && !F.scan_spin_limit &&
                    (F.row_blocks || (F.num_tris > 0u && F.num_tris <= kFusedTris && !touch));
     if (r->timing) GBR_CUDA(cudaEventRecord(r->ev[0], s));
-    GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
+    if (!F.fused_scan || !r->ctl_clean) GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
+    r->ctl_clean = false;
     if (predicted) {
         // coarse pre-pass -> capacities -> one fused setup + fill pass; the
         // exact kernels behind it only run if a bin overflowed.  The fused
@@ -369,10 +374,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         GBR_CUDA(launch_prepass(F, s));
         GBR_CUDA(launch_capacity(F, true, s));
         GBR_CUDA(launch_scan(scan_of(F, kScanCapacity), s));
-        GBR_CUDA(launch_setup(P, true, s));
+        GBR_CUDA(launch_setup(P, only, true, s));
         if (stages) GBR_CUDA(cudaEventRecord(r->ev[1], s));
         GBR_CUDA(launch_scan(scan_of(F, kScanPredictedItems), s));
-        GBR_CUDA(launch_setup(F, false, s));
+        GBR_CUDA(launch_setup(F, only, false, s));
         GBR_CUDA(launch_scan(scan_of(F, kScanExactAfterPredicted), s));
         GBR_CUDA(launch_fill(F, s));
     } else {
@@ -381,7 +386,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
             GBR_CUDA(launch_capacity(F, false, s));
             GBR_CUDA(launch_feat_reset(F, s));
         }
-        GBR_CUDA(launch_setup(F, false, s));
+        GBR_CUDA(launch_setup(F, only, false, s));
         if (stages) GBR_CUDA(cudaEventRecord(r->ev[1], s));
         if (!F.fused_scan) GBR_CUDA(launch_scan(scan_of(F, kScanExact), s));
         if (touch && !F.row_blocks) GBR_CUDA(launch_list_touch(F, s));
@@ -390,13 +395,14 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     r->last_predicted = predicted;
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[2], s));
     GBR_CUDA(launch_raster(F, r->raster_grid, s));
+    r->ctl_clean = true;
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[4], s));
     ShadeOne one;
-    if (md.size() == 1u) {
-        one.mesh = md[0];
+    if (only) {
+        one.mesh = *only;
         memcpy(one.lights, r->lights, sizeof one.lights);
     }
-    GBR_CUDA(launch_shade(F, md.size() == 1u ? &one : nullptr, s));
+    GBR_CUDA(launch_shade(F, only ? &one : nullptr, s));
     if (r->timing) {
         GBR_CUDA(cudaEventRecord(r->ev[3], s));
         r->ev_recorded = true;

@@ -179,7 +179,11 @@ struct __align__(16) TriSetup {
 };
 static_assert(sizeof(TriSetup) == 48, "setup record is 48 bytes");
 
-// Device-side control block of one frame.
+// Device-side control block of one frame.  `visible`, `float_path` and
+// `rank_next` add up during the count pass and are zero between frames: the
+// raster hands the first two on and clears all three (close_counters), and a
+// frame whose fill pass holds the scan writes every other field, so it needs
+// no clearing pass of its own.
 struct Ctl {
     unsigned long long num_pairs;
     uint32_t num_visible;
@@ -194,8 +198,10 @@ struct Ctl {
     unsigned long long items_alloc;   // batch: work items requested by all scenes
     uint32_t rank_next;        // exact binning: rank slots reserved by the count pass
     uint32_t shade_count;      // two-pass shading: covered pixels queued by the light pass
+    uint32_t visible, float_path;   // the count pass's running num_visible and num_float_path
+    uint32_t pad[2];
 };
-static_assert(sizeof(Ctl) == 64, "control block is 64 bytes");
+static_assert(sizeof(Ctl) == 80, "control block is 80 bytes");
 
 // Everything a kernel of the frame needs, passed by value.
 struct __align__(16) FrameDev {

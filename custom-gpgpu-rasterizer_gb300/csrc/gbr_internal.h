@@ -119,6 +119,7 @@ struct gbr_renderer {
 
     gbr::Ctl* d_ctl = nullptr;
     gbr::Ctl* h_ctl = nullptr;
+    bool ctl_clean = false;   // d_ctl's counters are zero (the last frame's raster was launched)
 
     gbr::LightDev* d_lights = nullptr;   // kMaxLights records
     gbr::LightDev lights[gbr::kMaxLights] = {};   // the same on the host

@@ -91,16 +91,17 @@ __device__ __forceinline__ uint32_t hiz_key(const TriSetup& t) {
 // block's shared-memory row `s_row` (MODE 2).  Called by whole warps.
 // Returns the warp's visible and float-path triangle counts (bits 0-15 and
 // 16-31), for the block's statistics.
+// `one`: the frame's only mesh (null: looked up).
 template <int MODE>
-__device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, uint32_t walk,
+__device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, uint32_t walk, const MeshDev* one,
                                               uint32_t* s_row = nullptr) {
     const bool in_range = prim < F.num_tris;
     uint2 rect = empty_rect();
     bool visible = false, fpath = false, no_raster = true;
     uint32_t key = 0u;
     if (in_range) {
-        const uint32_t mi = find_mesh(F, prim);
-        const MeshDev& m = F.meshes[mi];
+        const uint32_t mi = one ? 0u : find_mesh(F, prim);
+        const MeshDev& m = one ? *one : F.meshes[mi];
         uint32_t vid[3];
         tri_vertex_ids(m, prim - m.prim_base, vid);
         float nx[3], ny[3], nz[3];
@@ -189,24 +190,27 @@ __device__ __forceinline__ void add_block_stats(Ctl* ctl, uint32_t warp_vis, uin
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (s_vis) atomicAdd(&ctl->num_visible, s_vis);
-        if (s_fp) atomicAdd(&ctl->num_float_path, s_fp);
+        if (s_vis) atomicAdd(&ctl->visible, s_vis);
+        if (s_fp) atomicAdd(&ctl->float_path, s_fp);
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) setup_kernel(FrameDev F) {
+template <int MODE, bool ONE>
+__global__ void __launch_bounds__(256) setup_kernel(FrameDev F, const __grid_constant__ MeshDev one) {
     pdl_wait();
     // predicted binning: the exact pass only runs after an overflow, and the
     // predicted pass stops once an overflow is known; neither runs after a
-    // scan of the frame gave up (Ctl::overflow)
-    if (F.ctl->overflow) return;
-    if (MODE == 0 ? (F.exact_guard && !F.ctl->pred_overflow) : (F.ctl->pred_overflow != 0u)) return;
+    // scan of the frame gave up (Ctl::overflow).  An exact frame starts here,
+    // with nothing to check
+    if (MODE == 1 || F.exact_guard) {
+        if (F.ctl->overflow) return;
+        if (MODE == 0 ? !F.ctl->pred_overflow : F.ctl->pred_overflow != 0u) return;
+    }
     // a resident grid strides over the triangles, so that a guarded launch
     // that does not run costs one wave of early exits
     uint32_t vis = 0, fp = 0;
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x) {
-        const uint32_t c = setup_tri<MODE>(F, base + threadIdx.x, (base + threadIdx.x) >> 5);
+        const uint32_t c = setup_tri<MODE>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, ONE ? &one : nullptr);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -264,8 +268,10 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
         F.ctl->num_items = fits ? (uint32_t)items : 0u;
         F.ctl->items_alloc = items;
         F.ctl->item_next = 0u;
+        F.ctl->overflow = fits ? 0u : 1u;
+        F.ctl->pred_overflow = F.ctl->error = F.ctl->num_sampled = F.ctl->shade_count = 0u;
+        F.ctl->pred_capacity = 0ull;
         if (fits) F.offsets[nb] = (uint32_t)total;
-        else F.ctl->overflow = 1u;
     }
     if (F.dirty_wr)
         for (uint32_t i = blockIdx.x * THREADS + threadIdx.x; i < nb; i += gridDim.x * THREADS) F.dirty_wr[i] = 0u;
@@ -364,16 +370,16 @@ __device__ __forceinline__ void reserve_runs(const uint32_t* counts, uint32_t nb
     }
 }
 
-__global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F) {
+template <bool ONE>
+__global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F, const __grid_constant__ MeshDev one) {
     extern __shared__ uint32_t s_row[];
-    pdl_wait();
-    if (F.ctl->overflow) return;
     const uint32_t nb = F.num_bins;
     for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] = 0u;
     __syncthreads();
+    pdl_wait();
     uint32_t vis = 0, fp = 0;
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x) {
-        const uint32_t c = setup_tri<2>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, s_row);
+        const uint32_t c = setup_tri<2>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, ONE ? &one : nullptr, s_row);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -429,7 +435,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
 // one per (block, bin).  A block whose run does not fit raises
 // Ctl::pred_overflow and writes nothing (the exact kernels queued behind
 // re-bin the frame); the other blocks' runs lie inside their capacities.
-__global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev F) {
+template <bool ONE>
+__global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev F, const __grid_constant__ MeshDev one) {
     extern __shared__ uint32_t s_row[];
     __shared__ uint32_t s_ovf;
     pdl_wait();
@@ -440,7 +447,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
     __syncthreads();
     uint32_t vis = 0, fp = 0;
     for (uint32_t base = blockIdx.x * kRowThreads; base < F.num_tris; base += gridDim.x * kRowThreads) {
-        const uint32_t c = setup_tri<2>(F, base + tid, (base + tid) >> 5, s_row);
+        const uint32_t c = setup_tri<2>(F, base + tid, (base + tid) >> 5, ONE ? &one : nullptr, s_row);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -725,6 +732,7 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
     const uint4* const items = F.items;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     zero_counts(F);
+    if (blockIdx.x == 0u && tid == 0u) close_counters(Q);
     if (Q->overflow) return;
     const uint32_t num_items = Q->num_items;
     const uint32_t phase = F.phase == 0u ? kPhase : min(F.phase, kMaxPhase);
@@ -938,7 +946,8 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
 // and vertices (2M soup at 4K: one pixel a thread 96 us, two 92, two with
 // eight blocks an SM 82).
 template <ShadeKind KIND>
-__device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint32_t ty, uint32_t y1) {
+__device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint32_t ty, uint32_t y1,
+                                           const uint32_t* skip = nullptr) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t x = tx * kTileW + (warp & 3u) * 8u + (lane & 7u);
     const uint32_t y = ty + (warp >> 2) * 4u + (lane >> 3);
@@ -949,6 +958,7 @@ __device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint3
         const uint32_t yk = y + k * (kTileH / 2u);
         v[k] = yk < y1 ? F.gvis[(size_t)yk * F.width + x] : kEmptyVis;
     }
+    if (skip && *skip) return;   // a frame that was not rasterised
 #pragma unroll
     for (uint32_t k = 0; k < 2u; ++k) {
         const uint32_t yk = y + k * (kTileH / 2u);
@@ -970,8 +980,7 @@ template <ShadeKind KIND>
 __global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : KIND == kShadeFlat ? 6 : 8) shade_kernel(FrameDev F, uint32_t y0,
                                                                                                       uint32_t y1) {
     pdl_wait();
-    if (F.ctl->overflow) return;
-    shade_tile<KIND>(F, blockIdx.x, y0 + blockIdx.y * kTileH, y1);
+    shade_tile<KIND>(F, blockIdx.x, y0 + blockIdx.y * kTileH, y1, &F.ctl->overflow);
 }
 
 // Two-pass shading, for frames that shade through the full vertex stage
@@ -1184,7 +1193,7 @@ __global__ void __launch_bounds__(256) batch_setup_kernel(BatchDev B, uint32_t c
         }
         enter_scene(B, sc, loaded, sF);
         const uint32_t c = setup_tri<0>(sF, (v - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x,
-                                        (v * 256u + threadIdx.x) >> 5);
+                                        (v * 256u + threadIdx.x) >> 5, nullptr);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -1250,33 +1259,34 @@ static cudaError_t row_smem(const FrameDev& F, size_t* bytes) {
     const uint64_t bit = dev < 64 ? (1ull << dev) : 0ull;
     if (!(opted & bit)) {
         const int most = (int)(kMaxRowBins * sizeof(uint32_t));
-        e = cudaFuncSetAttribute(setup_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fill_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(predicted_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        e = cudaFuncSetAttribute(fill_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        for (auto* k : {setup_rows_kernel<true>, setup_rows_kernel<false>, predicted_rows_kernel<true>, predicted_rows_kernel<false>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
         opted |= bit;
     }
     return cudaSuccess;
 }
 
-cudaError_t launch_setup(const FrameDev& F, bool predicted, cudaStream_t s) {
-    if (predicted && F.row_blocks) {
+template <bool ONE>
+static cudaError_t launch_setup(const FrameDev& F, const MeshDev& one, bool predicted, cudaStream_t s) {
+    if (F.row_blocks) {
         size_t smem = 0;
         const cudaError_t e = row_smem(F, &smem);
         if (e != cudaSuccess) return e;
-        return launch_pdl(predicted_rows_kernel, dim3(F.row_blocks), dim3(kRowThreads), smem, s, F);
-    }
-    if (!predicted && F.row_blocks) {
-        size_t smem = 0;
-        const cudaError_t e = row_smem(F, &smem);
-        if (e != cudaSuccess) return e;
-        return launch_pdl(setup_rows_kernel, dim3(F.row_blocks), dim3(kRowThreads), smem, s, F);
+        return launch_pdl(predicted ? predicted_rows_kernel<ONE> : setup_rows_kernel<ONE>, dim3(F.row_blocks),
+                          dim3(kRowThreads), smem, s, F, one);
     }
     const uint32_t blocks = triangle_blocks(F.num_tris);
     if (blocks == 0) return cudaSuccess;
-    return predicted ? launch_pdl(setup_kernel<1>, dim3(blocks), dim3(256), 0, s, F)
-                     : launch_pdl(setup_kernel<0>, dim3(blocks), dim3(256), 0, s, F);
+    return launch_pdl(predicted ? setup_kernel<1, ONE> : setup_kernel<0, ONE>, dim3(blocks), dim3(256), 0, s, F, one);
+}
+
+cudaError_t launch_setup(const FrameDev& F, const MeshDev* one, bool predicted, cudaStream_t s) {
+    if (one) return launch_setup<true>(F, *one, predicted, s);
+    MeshDev none;
+    memset(&none, 0, sizeof none);
+    return launch_setup<false>(F, none, predicted, s);
 }
 
 cudaError_t launch_fill(const FrameDev& F, cudaStream_t s) {

@@ -46,7 +46,8 @@ cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_
                                    int* blocks_per_sm);
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,
                                 uint32_t bw, uint32_t bh, uint32_t grid, cudaStream_t s);
-cudaError_t launch_setup(const FrameDev& F, bool predicted, cudaStream_t s);
+// one: the mesh of a frame of one mesh (null otherwise)
+cudaError_t launch_setup(const FrameDev& F, const MeshDev* one, bool predicted, cudaStream_t s);
 // The bin scan of a frame (mode: kScanExact, ...), one launch.
 ScanDev scan_of(const FrameDev& F, uint32_t mode);
 uint32_t scan_blocks(uint32_t num_bins);   // tiles of 1024 bins

@@ -217,7 +217,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     e = cudaGetLastError();
     if (e == cudaSuccess && ((uint64_t)num_bins_x * bin_w < width || (uint64_t)num_bins_y * bin_h < height))
         e = launch_clear(F, s);
-    if (e == cudaSuccess) e = launch_setup(F, false, s);
+    if (e == cudaSuccess) e = launch_setup(F, &desc, false, s);
     if (e == cudaSuccess && !F.fused_scan) e = launch_scan(scan_of(F, kScanExact), s);
     if (e == cudaSuccess) e = launch_fill(F, s);
     if (e == cudaSuccess) e = launch_raster(F, per_sm, s);

@@ -283,7 +283,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
     pdl_wait();
     Ctl* const Q = BATCH ? B.ctl : F.ctl;
     const uint4* const items = BATCH ? B.items : F.items;
-    if (!BATCH) zero_counts(F);
+    if (!BATCH) {
+        zero_counts(F);
+        if (blockIdx.x == 0u && tid == 0u) close_counters(Q);
+    } else {
+        for (uint32_t i = blockIdx.x * THREADS + tid; i < B.num_scenes; i += gridDim.x * THREADS)
+            close_counters(B.scenes[i].ctl);
+    }
     if (Q->overflow) return;
     const uint32_t num_items = Q->num_items;
     const uint32_t stage_req = BATCH ? B.stage : F.stage;

@@ -17,6 +17,14 @@ __device__ __forceinline__ void fetch_item(uint4* dst, const uint4* items, uint3
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(items + idx) : "memory");
 }
 
+// The count pass's counters of a frame (Ctl): handed on, and left zero for
+// the next frame.
+__device__ __forceinline__ void close_counters(Ctl* c) {
+    c->num_visible = c->visible;
+    c->num_float_path = c->float_path;
+    c->visible = c->float_path = c->rank_next = 0u;
+}
+
 // After a fill pass with the scan in it, the raster leaves the bins' counts
 // zero for the next frame.
 __device__ __forceinline__ void zero_counts(const FrameDev& F) {

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
     if (!scan_runs(S)) return;
     if (S.mode == kScanPredictedItems) {
         if (S.ctl->pred_overflow) {   // the exact pass that follows counts again
-            if (blockIdx.x == 0 && threadIdx.x == 0) { S.ctl->num_visible = 0u; S.ctl->num_float_path = 0u; }
+            if (blockIdx.x == 0 && threadIdx.x == 0) { S.ctl->visible = 0u; S.ctl->float_path = 0u; }
             return;
         }
     }
