@@ -263,12 +263,12 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.nbx = r->nbx; F.nby = r->nby; F.bw = r->bw; F.bh = r->bh; F.num_bins = nb;
     // raster work: once a frame has been seen, items hold about half of a
     // raster CTA's share of the pairs (so a few crowded bins do not
-    // serialise the frame), within [kMinChunk, kMaxChunk]; queue_chunk is
-    // the pass size (entries depth-sorted and rasterised at a time); with the
-    // library's phase, triangles spanning under 4 bins on average (little
-    // overdraw per bin) refresh the tile's depth bound every kSparsePhase
-    // triangles rather than every kPhase (every kMaxPhase with the
-    // small-triangle variant, below)
+    // serialise the frame), within [kMinBlockChunk, kMaxChunk]; queue_chunk
+    // is the pass size (entries depth-sorted and rasterised at a time).
+    // Bulk-copy staging: at least kMinChunk, and with the library's phase,
+    // triangles spanning under 4 bins on average (little overdraw per bin)
+    // refresh the tile's depth bound every kSparsePhase triangles rather than
+    // every kPhase
     F.chunk = kMaxChunk;
     F.stage = r->chunk;   // queue_chunk: entries per raster pass
     F.phase = r->raster_phase;
@@ -276,18 +276,14 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     if (r->seen_pairs) {
         if (F.phase == 0u) F.phase = r->seen_pairs < 4u * r->seen_visible ? kSparsePhase : kPhase;
         // small triangles: about (pairs per visible triangle - 1) x the bin
-        // side of width + height each; with the library's phase the
-        // small-triangle variant runs phases of the whole record ring, so
-        // that every warp of the CTA takes a share of each phase
-        if (F.phase >= kLanePhase && r->seen_visible) {
+        // side of width + height each
+        if (F.phase >= kDirectPhase && r->seen_visible && !r->rec_tma) {
             const double extent = ((double)r->seen_pairs / (double)r->seen_visible - 1.0) * 0.5 * (r->bw + r->bh);
-            F.raster_lanes = extent < kLaneExtentPx ? 1u : 0u;
-            if (F.raster_lanes && r->raster_phase == 0u) F.phase = kMaxPhase;
+            F.direct = extent < kDirectExtentPx ? 1u : 0u;
         }
-        const bool record = F.raster_lanes || r->rec_tma;
-        const uint64_t grid = (uint64_t)r->num_sms * (uint64_t)(record ? r->raster_grid.record : r->raster_grid.block128 / 2);
+        const uint64_t grid = (uint64_t)r->num_sms * (uint64_t)(r->rec_tma ? r->raster_grid.record : r->raster_grid.block128 / 2);
         const uint64_t share = r->seen_pairs / (2u * grid);
-        F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), record ? kMinChunk : kMinBlockChunk);
+        F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), r->rec_tma ? kMinChunk : kMinBlockChunk);
     }
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;
@@ -296,7 +292,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.setup = r->d_setup; F.rects = r->d_rects; F.keys = r->d_keys;
     F.counts = r->d_counts; F.sub_base = r->d_sub_base; F.count_stride = nb; F.offsets = r->d_offsets;
     F.cursors = r->d_cursors; F.capacity = r->d_capacity;
-    F.count_split = count_split_for(r->seen_pairs, nb);   // 1 until a frame has been seen
+    F.count_split = std::max(count_split_for(r->seen_pairs, nb), F.direct ? 2u : 1u);   // 1 until a frame has been seen
     F.bin_end = r->d_bin_end;
     F.items = r->d_items; F.items_cap = r->items_cap;
     F.list = r->d_list; F.list_cap = r->list_cap;
@@ -321,14 +317,14 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.exact_guard = predicted ? 1u : 0u;
     // exact binning of a dense frame: block-private counter rows
     const uint32_t rows = std::min<uint32_t>((F.num_tris + kRowThreads - 1u) / kRowThreads, (uint32_t)r->num_sms);
-    if (!predicted && r->d_row_base && use_count_rows(r->seen_pairs, nb, rows)) {
+    if (!predicted && !F.direct && r->d_row_base && use_count_rows(r->seen_pairs, nb, rows)) {
         F.row_base = r->d_row_base;
         F.row_blocks = rows;
         F.count_split = 1u;
     }
     r->last_row_blocks = F.row_blocks;
     r->last_key_mask = F.key_mask;
-    r->last_raster_lanes = F.raster_lanes;
+    r->last_raster_lanes = F.direct;
     // frames shaded through the full vertex stage shade their covered
     // pixels in a second, densely packed pass
     if (!F.flat_shade && vis != GBR_VIS_DEPTH) {
@@ -355,7 +351,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         F.touch_words = (uint32_t)((std::min<uint64_t>(r->list_cap, r->seen_pairs + r->seen_pairs / 16u) + 3u) / 4u);
     // the fill pass scans the bins itself (not where a test hook silences a
     // tile of the scan kernel)
-    F.fused_scan = !predicted && nb <= kFusedBins && F.count_split == 1u && !F.scan_silent_tile1 && !F.scan_spin_limit &&
+    F.fused_scan = !predicted && nb <= kFusedBins && F.count_split == (F.direct ? 2u : 1u) && !F.scan_silent_tile1 && !F.scan_spin_limit &&
                    (F.row_blocks || (F.num_tris > 0u && F.num_tris <= kFusedTris && !touch));
     if (r->timing) GBR_CUDA(cudaEventRecord(r->ev[0], s));
     if (!F.fused_scan || !r->ctl_clean) GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));

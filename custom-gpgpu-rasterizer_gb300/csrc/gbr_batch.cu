@@ -331,7 +331,7 @@ gbr_status capture_graph(gbr_batch* b) {
     memset(&L.scan, 0, sizeof L.scan);
     L.scan.counts = b->d_counts;
     L.scan.sub_base = b->d_sub_base;
-    L.scan.split = b->count_split;
+    L.scan.split = L.scan.raster_split = b->count_split;
     L.scan.offsets = b->d_offsets;
     L.scan.cursors = b->d_cursors;
     L.scan.items = b->d_items;

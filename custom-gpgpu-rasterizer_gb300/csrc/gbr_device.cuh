@@ -14,8 +14,8 @@
 namespace gbr {
 
 constexpr uint32_t kInvalidPrim = 0xFFFFFFFFu;
-// A bin-list entry: the primitive, kNoRasterBit if it cannot cover a pixel,
-// and in frames of at most 2^kKeyedIdBits triangles the top 8 bits of its
+// A bin-list entry: the primitive, kNoRasterBit if the raster need not read
+// it (it cannot cover a pixel, or the set-up pass has rasterised it), and in frames of at most 2^kKeyedIdBits triangles the top 8 bits of its
 // depth-key bound (bits 23-30, where they sit in the key), by which the
 // raster sorts.  Sorting a bin then reads nothing but its list: gathering
 // the bounds of 980 entries a bin took 16 L1 wavefronts a load.  Larger
@@ -75,16 +75,21 @@ constexpr uint32_t kWideItemsPerSm = 6;
 __host__ __device__ inline uint32_t block_threads_for(unsigned long long items, uint32_t sms) {
     return items < (unsigned long long)kWideItemsPerSm * sms ? 512u : 128u;
 }
-// The raster's small-triangle variant: in phases of at least kLanePhase
-// triangles a warp takes kLaneGrab sorted triangles at once and each lane
-// rasterises its own when its pixel box holds at most kLanePixels pixels.
-// The library picks it for sparse frames whose triangles span less than
-// kLaneExtentPx (width + height, estimated from the last frame's
-// (triangle, bin) pairs per visible triangle).
-constexpr uint32_t kLanePhase = 32;
-constexpr uint32_t kLaneGrab = 16;
-constexpr int kLanePixels = 16;
-constexpr double kLaneExtentPx = 16.0;
+// Frames of small triangles (FrameDev::direct): the set-up pass rasterises
+// every triangle whose pixel box holds at most kDirectPixels pixels itself, a
+// lane per triangle, straight into the merge buffer; its list entries are
+// marked as the raster need not read them, and come after the others in their
+// bins (exact binning; predicted capacities keep them together).  A sub-pixel
+// triangle covers a pixel or none, and bringing it to a raster CTA through its
+// bin's list cost more than that (4K icosphere-7: set-up 18.3 -> 20.8 us,
+// raster 25.2 -> 2.9).  The library takes it for sparse
+// frames whose triangles span less than kDirectExtentPx (width + height,
+// estimated from the last frame's (triangle, bin) pairs per visible
+// triangle), and not where an explicit phase below kDirectPhase asks for depth
+// refreshes.
+constexpr uint32_t kDirectPhase = 32;
+constexpr int kDirectPixels = 16;
+constexpr double kDirectExtentPx = 16.0;
 // Exact binning with block-private counter rows: one block of kRowThreads
 // per SM counts its pairs per bin in shared memory (num_bins <=
 // kMaxRowBins), then takes its run of every bin it touched with one global
@@ -252,7 +257,8 @@ struct __align__(16) FrameDev {
     uint32_t* rank_next;       // slot reservation counter (a Ctl's rank_next)
     unsigned long long rank_cap;
     uint32_t count_stride;     // bins between sub-counter rows (the scan's bin count)
-    uint32_t count_split;      // sub-counters per bin in use: 1, 2, 4 or 8
+    uint32_t count_split;      // sub-counters per bin in use: 1, 2, 4 or 8 (direct: the first half for entries the
+                               // raster reads, which come first in the list)
     // exact binning with block-private counter rows (row_blocks > 0)
     uint32_t* row_base;        // row_blocks x num_bins: a block's first entry in each bin it touched, bin-relative
     uint32_t row_blocks;       // blocks of the count and fill passes (0: sub-counters)
@@ -273,12 +279,13 @@ struct __align__(16) FrameDev {
     uint32_t row0, row1;
     uint32_t px_begin, px_end;
     uint32_t rec_tma;          // raster: setup records staged by bulk asynchronous copies (1) or loads (0)
-    uint32_t raster_lanes;     // raster: the small-triangle variant (a lane per triangle; phases >= kLanePhase)
+    uint32_t direct;           // the set-up pass rasterises small triangles itself (kDirectPixels)
     uint32_t fused_scan;       // the fill pass scans the bins' counts itself (no scan kernel)
     uint32_t block_threads;    // block raster: threads per CTA, 128 or 512
     // two-pass shading of a sparse frame: one byte per bin, "may hold drawn
-    // pixels".  dirty_rd: after the last frame; dirty_wr: this frame's, zeroed
-    // by its first scan and set by the raster for every bin it draws.  The
+    // pixels".  dirty_rd: after the last frame; dirty_wr: this frame's, set by
+    // the scan for every bin with entries (predicted binning: by the raster for
+    // every bin it draws).  The
     // light pass leaves the quads of bins clean in both untouched: their
     // pixels already hold the clear values.  (null: every pixel is written)
     uint8_t* dirty_rd;
@@ -321,6 +328,7 @@ struct ScanDev {
     uint32_t* counts;              // exact sub-counts (kCountSplit rows of stride n), zeroed for the next frame
     uint32_t* sub_base;            // exact modes: list start of each sub-count (same layout)
     uint32_t split;                // sub-counters per bin in use
+    uint32_t raster_split;         // those whose entries the raster reads (the first ones): work items cover them alone
     const uint32_t* capacity;      // predicted capacities
     uint32_t* offsets;             // n + 1
     uint32_t* cursors;
@@ -336,7 +344,8 @@ struct ScanDev {
     uint32_t mode;
     uint32_t spin_limit;           // polls of one flag before a look-back wait gives up (0: kScanSpinLimit)
     uint32_t silent_tile1;         // 1 + a tile that publishes nothing (0: none; test hook)
-    uint8_t* dirty;                // the frame's per-bin drawn flags to zero (FrameDev::dirty_wr; null: none)
+    uint8_t* dirty;                // the frame's per-bin drawn flags (FrameDev::dirty_wr; null: none): set for the bins
+                                   // with entries, or zeroed by the capacity scan (the raster then sets them)
 };
 
 // Many scenes rendered as one batch frame.  Each scene keeps its own frame
@@ -497,7 +506,8 @@ __device__ __forceinline__ int4 bin_rect(float2 s0, float2 s1, float2 s2, const 
     return r;
 }
 
-// Packed bin rectangle: x = bx0 | bx1 << 16, y = by0 | by1 << 16 | noRaster << 31.
+// Packed bin rectangle: x = bx0 | bx1 << 16, y = by0 | by1 << 16 | noRaster
+// << 31 (the raster need not read the entry).
 __device__ __forceinline__ uint2 pack_rect(int4 r, bool no_raster) {
     uint2 p;
     p.x = (uint32_t)r.x | ((uint32_t)r.z << 16);
@@ -577,8 +587,8 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 // latency, so several must be in flight per lane.
 // Mode 0: count (atomicAdd on the walk's sub-counter of the bin; its return,
 // the pair's rank there, is kept in the walk's rank slots), 1: fill (entry
-// at the sub-counter's list start + rank: no atomics; 4: at the bin's offset
-// in `s_off` + rank), 2: predicted fill (append within the bin's predicted
+// at the sub-counter's list start + rank: no atomics; 4: at its start in
+// `s_off` + rank), 2: predicted fill (append within the bin's predicted
 // capacity), 3: pre-pass count (atomicAdd on the first feature slot).  A
 // walk is identified by `walk` (its first triangle slot / 32), so the count
 // and fill passes of the same triangles meet the same slots.  One atomic per
@@ -590,7 +600,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
 #endif
 constexpr uint32_t kPairsPerLane = GBR_PAIRS_PER_LANE;
 
-template <int MODE>
+template <int MODE, bool DIRECT = false>
 __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t entry, bool valid, uint32_t walk,
                                          const uint32_t* s_off = nullptr) {
     __shared__ uint4 s_tab[8][32];   // per warp: (first pair, width, bx0 | by0 << 16, entry) of each lane
@@ -614,7 +624,10 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
     // exact binning: the walk's rank slots, reserved by the count pass and
     // found again by the fill pass (same triangles, same enumeration)
     uint32_t wb = 0;
-    const uint32_t krow = (walk & (F.count_split - 1u)) * F.count_stride;   // the walk's sub-counter row
+    // the walk's sub-counter row, and (DIRECT) that of entries the raster
+    // does not read
+    const uint32_t half = DIRECT ? F.count_split >> 1 : F.count_split;
+    const uint32_t krow = (walk & (half - 1u)) * F.count_stride, skipped = half * F.count_stride;
     if (MODE == 0) {
         if (lane == 0) {
             wb = atomicAdd(F.rank_next, total);
@@ -624,12 +637,12 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
     } else if (MODE == 1 || MODE == 4) {
         wb = __ldg(&F.walk_base[walk]);
     }
-    s_tab[warp][lane] = make_uint4(excl, w, bx0 | (by0 << 16), entry);
+    s_tab[warp][lane] = make_uint4(excl, w, bx0 | (by0 << 16) | (DIRECT ? rect.y & 0x80000000u : 0u), entry);
     __syncwarp();
     const uint32_t nonempty = __ballot_sync(0xFFFFFFFFu, n != 0u);
     const uint32_t upto = lane == 31u ? 0xFFFFFFFFu : ((2u << lane) - 1u);   // bits 0..lane
     for (uint32_t base = 0; base < total; base += 32u * kPairsPerLane) {   // warp-uniform
-        uint32_t bin[kPairsPerLane], ent[kPairsPerLane];
+        uint32_t bin[kPairsPerLane], ent[kPairsPerLane];   // modes 0, 1 and 4: bin is the pair's sub-counter
         bool act[kPairsPerLane];
 #pragma unroll
         for (uint32_t u = 0; u < kPairsPerLane; ++u) {
@@ -649,7 +662,8 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
             act[u] = k < total;
             const uint32_t j = k - d.x;
             const uint32_t q = act[u] ? j / d.y : 0u;
-            bin[u] = ((d.z & 0xFFFFu) + (j - q * d.y)) + ((d.z >> 16) + q) * F.nbx;
+            bin[u] = ((d.z & 0xFFFFu) + (j - q * d.y)) + ((DIRECT ? (d.z >> 16) & 0x7FFFu : d.z >> 16) + q) * F.nbx;
+            if (MODE == 0 || MODE == 1 || MODE == 4) bin[u] += krow + (DIRECT && (d.z & 0x80000000u) ? skipped : 0u);
             ent[u] = d.w;
         }
         if (MODE == 3) {
@@ -661,7 +675,7 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
             // storage are dropped: that frame overflows and is not filled)
             uint32_t rank[kPairsPerLane];
 #pragma unroll
-            for (uint32_t u = 0; u < kPairsPerLane; ++u) rank[u] = act[u] ? atomicAdd(&F.counts[krow + bin[u]], 1u) : 0u;
+            for (uint32_t u = 0; u < kPairsPerLane; ++u) rank[u] = act[u] ? atomicAdd(&F.counts[bin[u]], 1u) : 0u;
 #pragma unroll
             for (uint32_t u = 0; u < kPairsPerLane; ++u) {
                 const unsigned long long slot = (unsigned long long)wb + base + u * 32u + lane;
@@ -674,7 +688,7 @@ __device__ __forceinline__ void bin_walk(const FrameDev& F, uint2 rect, uint32_t
             for (uint32_t u = 0; u < kPairsPerLane; ++u) rank[u] = act[u] ? __ldg(&F.ranks[wb + base + u * 32u + lane]) : 0u;
 #pragma unroll
             for (uint32_t u = 0; u < kPairsPerLane; ++u)
-                if (act[u]) F.list[(MODE == 4 ? s_off[bin[u]] : __ldg(&F.sub_base[krow + bin[u]])) + rank[u]] = ent[u];
+                if (act[u]) F.list[(MODE == 4 ? s_off[bin[u]] : __ldg(&F.sub_base[bin[u]])) + rank[u]] = ent[u];
         } else {
             uint32_t pos[kPairsPerLane];
 #pragma unroll

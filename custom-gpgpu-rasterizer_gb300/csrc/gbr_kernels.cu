@@ -18,9 +18,9 @@
 //                  slots from shared-memory cursors).
 //   block_raster_kernel (gbr_raster.cu): persistent CTAs pull work items,
 //                  depth-sort the chunk by the key bounds and rasterise it
-//                  front to back, a warp to 8x4 pixels; raster_kernel, here,
-//                  takes frames of small triangles (a lane per triangle) and
-//                  the bulk-copy staging on request.
+//                  front to back, a warp to 8x4 pixels (frames of small
+//                  triangles: the set-up pass has rasterised those itself);
+//                  raster_kernel, here, takes the bulk-copy staging on request.
 //   shade_kernel : each pixel's winner shaded once: colour, depth and id.
 //
 // Reference stages replaced: VS_Kernel, TA_Kernel, TB_Kernel,
@@ -85,19 +85,50 @@ __device__ __forceinline__ uint32_t hiz_key(const TriSetup& t) {
     return (uint32_t)__float2int_rz(__fmul_rn(zb, 2147483648.0f));
 }
 
+// One lane's raster of a small triangle with bin rectangle r, straight into
+// the merge buffer: the raster's pixel box, exact edge functions, weights,
+// depth and (key, id) minimum.  Returns false, having done nothing, for a box
+// of more than kDirectPixels pixels.
+__device__ __forceinline__ bool raster_direct(const FrameDev& F, const TriSetup& t, uint32_t prim, int4 r, int X0, int Y0,
+                                              int X1, int Y1, int X2, int Y2) {
+    // covered pixels lie in [ceil(min), floor(max)] of the snapped triangle,
+    // and only those of its bins are rasterised
+    const int px0 = max((min(X0, min(X1, X2)) + 0xFFFF) >> kFxBits, r.x * (int)F.bw);
+    const int px1 = min(max(X0, max(X1, X2)) >> kFxBits, min((r.z + 1) * (int)F.bw, (int)F.width) - 1);
+    const int py0 = max((min(Y0, min(Y1, Y2)) + 0xFFFF) >> kFxBits, r.y * (int)F.bh);
+    const int py1 = min(max(Y0, max(Y1, Y2)) >> kFxBits, min((r.w + 1) * (int)F.bh, (int)F.height) - 1);
+    if (px0 > px1 || py0 > py1) return true;
+    if ((px1 - px0 + 1) * (py1 - py0 + 1) > kDirectPixels) return false;
+    for (int y = py0; y <= py1; ++y)
+        for (int x = px0; x <= px1; ++x) {
+            const int fx = x << kFxBits, fy = y << kFxBits;
+            if ((edge_fx(fx, fy, X0, Y0, X1 - X0, Y1 - Y0) | edge_fx(fx, fy, X1, Y1, X2 - X1, Y2 - Y1) |
+                 edge_fx(fx, fy, X2, Y2, X0 - X2, Y0 - Y2)) < 0)
+                continue;
+            float w[3];
+            weights_fixed(t, x, y, w);
+            const float z = interp_z(w[0], w[1], w[2], t.z0, t.z1, t.z2);
+            if (!(z >= 0.f && z < 1.f)) continue;   // as the raster rejects it
+            const uint32_t key = (uint32_t)__float2int_rz(__fmul_rn(z, 2147483648.0f));
+            atomicMin(F.gvis + ((size_t)y * F.width + (size_t)x), ((unsigned long long)key << 32) | prim);
+        }
+    return true;
+}
+
 // Vertex stage (positions), triangle assembly, cull, frustum reject, raster
 // setup record, depth-key bound and bin rectangle of triangle `prim`, then the count pass
 // (MODE 0), the predicted-capacity fill (MODE 1) or the count into the
 // block's shared-memory row `s_row` (MODE 2).  Called by whole warps.
 // Returns the warp's visible and float-path triangle counts (bits 0-15 and
 // 16-31), for the block's statistics.
-// `one`: the frame's only mesh (null: looked up).
-template <int MODE>
+// `one`: the frame's only mesh (null: looked up).  DIRECT: small triangles
+// are rasterised here (a variant of its own, for the registers).
+template <int MODE, bool DIRECT = false>
 __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, uint32_t walk, const MeshDev* one,
                                               uint32_t* s_row = nullptr) {
     const bool in_range = prim < F.num_tris;
     uint2 rect = empty_rect();
-    bool visible = false, fpath = false, no_raster = true;
+    bool visible = false, fpath = false, skip = true;   // skip: the raster need not read the triangle's entries
     uint32_t key = 0u;
     if (in_range) {
         const uint32_t mi = one ? 0u : find_mesh(F, prim);
@@ -136,9 +167,10 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
                                 fabsf(s1.y) < kGuardPx && fabsf(s2.x) < kGuardPx && fabsf(s2.y) < kGuardPx;
             float inv_area = 0.f;
             uint32_t flags;
+            int X0 = 0, Y0 = 0, X1 = 0, Y1 = 0, X2 = 0, Y2 = 0;
             if (inside) {
-                const int X0 = snap_fx(s0.x), Y0 = snap_fx(s0.y), X1 = snap_fx(s1.x);
-                const int Y1 = snap_fx(s1.y), X2 = snap_fx(s2.x), Y2 = snap_fx(s2.y);
+                X0 = snap_fx(s0.x); Y0 = snap_fx(s0.y); X1 = snap_fx(s1.x);
+                Y1 = snap_fx(s1.y); X2 = snap_fx(s2.x); Y2 = snap_fx(s2.y);
                 // S = cross(v0 - v1, v2 - v1) of the snapped triangle: > 0 for the
                 // covered winding (the three edge functions sum to S)
                 const long long S = (long long)(X0 - X1) * (long long)(Y2 - Y1) -
@@ -146,12 +178,12 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
                 // the float area the reference divides its weights by (CUDAROPs.cu:336)
                 const float area = fabsf(__fmaf_rn(__fsub_rn(s0.x, s1.x), __fsub_rn(s0.y, s2.y),
                                                    -__fmul_rn(__fsub_rn(s0.y, s1.y), __fsub_rn(s0.x, s2.x))));
-                no_raster = !(S > 0 && area > 0.f);
-                inv_area = no_raster ? 0.f : __fdiv_rn(1.0f, area);
-                flags = no_raster ? 0u : kFlagRaster;
+                skip = !(S > 0 && area > 0.f);
+                inv_area = skip ? 0.f : __fdiv_rn(1.0f, area);
+                flags = skip ? 0u : kFlagRaster;
             } else {
                 fpath = true;
-                no_raster = false;
+                skip = false;
                 flags = kFlagFloat;
             }
             // the raster depth-sorts a bin's triangles by this bound before it
@@ -164,16 +196,17 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
             rec[0] = make_uint4(__float_as_uint(s0.x), __float_as_uint(s0.y), __float_as_uint(s1.x), __float_as_uint(s1.y));
             rec[1] = make_uint4(__float_as_uint(s2.x), __float_as_uint(s2.y), __float_as_uint(nz[0]), __float_as_uint(nz[1]));
             rec[2] = make_uint4(__float_as_uint(nz[2]), __float_as_uint(inv_area), key, mi | flags);
-            rect = pack_rect(r, no_raster);
+            if (DIRECT && !skip && inside) skip = raster_direct(F, t, prim, r, X0, Y0, X1, Y1, X2, Y2);
+            rect = pack_rect(r, skip);
             F.keys[prim] = key;
         }
         F.rects[prim] = rect;
     }
     const uint32_t counts = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, visible)) |
                             ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, fpath)) << 16);
-    if (MODE == 0) bin_walk<0>(F, rect, 0u, visible, walk);
+    if (MODE == 0) bin_walk<0, DIRECT>(F, rect, 0u, visible, walk);
     else if (MODE == 2) count_rect(s_row, visible ? rect : empty_rect(), F.nbx, F.nby);
-    else bin_walk<2>(F, rect, list_entry(prim, key, no_raster, F.key_mask), visible, walk);
+    else bin_walk<2>(F, rect, list_entry(prim, key, skip, F.key_mask), visible, walk);
     return counts;
 }
 
@@ -195,7 +228,7 @@ __device__ __forceinline__ void add_block_stats(Ctl* ctl, uint32_t warp_vis, uin
     }
 }
 
-template <int MODE, bool ONE>
+template <int MODE, bool ONE, bool DIRECT = false>
 __global__ void __launch_bounds__(256) setup_kernel(FrameDev F, const __grid_constant__ MeshDev one) {
     pdl_wait();
     // predicted binning: the exact pass only runs after an overflow, and the
@@ -210,7 +243,7 @@ __global__ void __launch_bounds__(256) setup_kernel(FrameDev F, const __grid_con
     // that does not run costs one wave of early exits
     uint32_t vis = 0, fp = 0;
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x) {
-        const uint32_t c = setup_tri<MODE>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, ONE ? &one : nullptr);
+        const uint32_t c = setup_tri<MODE, DIRECT>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, ONE ? &one : nullptr);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -226,7 +259,7 @@ __global__ void __launch_bounds__(256) setup_kernel(FrameDev F, const __grid_con
 // 0.  Returns false for a frame that exceeds the storage (flagged, not
 // filled).  The counts stay as they are, for the other blocks: the raster
 // zeroes them.
-template <uint32_t THREADS>
+template <uint32_t THREADS, bool DIRECT>
 __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
     constexpr uint32_t kWarps = THREADS / 32u;
     __shared__ unsigned long long s_a[kWarps], s_b[kWarps];
@@ -237,9 +270,14 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
 #pragma unroll 4
     for (uint32_t r = r0; r < r1; ++r) {
         const uint32_t i = r * 32u + lane;
-        const uint32_t c = i < nb ? F.counts[i] : 0u;
-        if (i < nb) s_off[i] = c;
-        a += c;
+        // c: entries the raster reads; c1 (DIRECT): the others
+        const uint32_t c = i < nb ? F.counts[i] : 0u, c1 = i < nb && DIRECT ? F.counts[nb + i] : 0u;
+        if (i < nb) {
+            s_off[i] = c;
+            if (DIRECT) s_off[nb + i] = c1;
+            if (F.dirty_wr && r % gridDim.x == blockIdx.x) F.dirty_wr[i] = c + c1 ? 1u : 0u;
+        }
+        a += (unsigned long long)c + c1;
         b += (c + chunk - 1u) / chunk;
     }
 #pragma unroll
@@ -273,14 +311,13 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
         F.ctl->pred_capacity = 0ull;
         if (fits) F.offsets[nb] = (uint32_t)total;
     }
-    if (F.dirty_wr)
-        for (uint32_t i = blockIdx.x * THREADS + threadIdx.x; i < nb; i += gridDim.x * THREADS) F.dirty_wr[i] = 0u;
     if (!fits) return false;
     uint32_t at = (uint32_t)at64, item = (uint32_t)item64;   // the totals fit 32 bits
     for (uint32_t r = r0; r < r1; ++r) {
         const uint32_t i = r * 32u + lane;
-        const uint32_t c = i < nb ? s_off[i] : 0u, it = (c + chunk - 1u) / chunk;
-        uint32_t x = c, y = it;
+        const uint32_t c = i < nb ? s_off[i] : 0u, c1 = i < nb && DIRECT ? s_off[nb + i] : 0u;
+        const uint32_t it = (c + chunk - 1u) / chunk;
+        uint32_t x = c + c1, y = it;
 #pragma unroll
         for (uint32_t d = 1; d < 32; d <<= 1) {
             const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, d), u = __shfl_up_sync(0xFFFFFFFFu, y, d);
@@ -289,9 +326,10 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
                 y += u;
             }
         }
-        const uint32_t start = at + x - c;
+        const uint32_t start = at + x - c - c1;
         if (i < nb) {
             s_off[i] = start;
+            if (DIRECT) s_off[nb + i] = start + c;
             if (r % gridDim.x == blockIdx.x) {
                 F.offsets[i] = start;
                 for (uint32_t k = 0; k < it; ++k)
@@ -312,28 +350,31 @@ __device__ __forceinline__ uint32_t rect_entry(const FrameDev& F, uint32_t prim,
 
 // Second pass of exact binning for triangle `prim`.  Called by whole warps.
 // s_off: the bins' offsets of a fused scan (MODE 4).
-template <int MODE>
+template <int MODE, bool DIRECT>
 __device__ __forceinline__ void fill_tri(const FrameDev& F, uint32_t prim, uint32_t walk, const uint32_t* s_off = nullptr) {
     const bool in_range = prim < F.num_tris;
     const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-    bin_walk<MODE>(F, rect, rect_entry(F, prim, rect, in_range), in_range, walk, s_off);
+    bin_walk<MODE, DIRECT>(F, rect, rect_entry(F, prim, rect, in_range), in_range, walk, s_off);
 }
 
+template <bool DIRECT>
 __global__ void __launch_bounds__(256) fill_kernel(FrameDev F) {
     pdl_wait();
     if (F.ctl->overflow || (F.exact_guard && !F.ctl->pred_overflow)) return;
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x)
-        fill_tri<1>(F, base + threadIdx.x, (base + threadIdx.x) >> 5);
+        fill_tri<1, DIRECT>(F, base + threadIdx.x, (base + threadIdx.x) >> 5);
     pdl_release();
 }
 
-// The same with the scan in it (at most kFusedBins bins, one counter a bin).
+// The same with the scan in it (at most kFusedBins bins, one counter a bin,
+// or two in direct frames).
+template <bool DIRECT>
 __global__ void __launch_bounds__(256) fill_fused_kernel(FrameDev F) {
-    __shared__ uint32_t s_off[kFusedBins];
+    __shared__ uint32_t s_off[(DIRECT ? 2u : 1u) * kFusedBins];
     pdl_wait();
-    if (!fused_scan<256>(F, s_off)) return;
+    if (!fused_scan<256, DIRECT>(F, s_off)) return;
     for (uint32_t base = blockIdx.x * blockDim.x; base < F.num_tris; base += gridDim.x * blockDim.x)
-        fill_tri<4>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, s_off);
+        fill_tri<4, DIRECT>(F, base + threadIdx.x, (base + threadIdx.x) >> 5, s_off);
     pdl_release();
 }
 
@@ -407,7 +448,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
     const uint32_t nb = F.num_bins;
     const uint32_t* const row = F.row_base + (size_t)blockIdx.x * nb;
     if (F.fused_scan) {
-        if (!fused_scan<kRowThreads>(F, s_row)) return;
+        if (!fused_scan<kRowThreads, false>(F, s_row)) return;
         for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] += __ldg(row + b);
     } else {
         if (F.ctl->overflow) return;
@@ -435,7 +476,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
 // one per (block, bin).  A block whose run does not fit raises
 // Ctl::pred_overflow and writes nothing (the exact kernels queued behind
 // re-bin the frame); the other blocks' runs lie inside their capacities.
-template <bool ONE>
+template <bool ONE, bool DIRECT>
 __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev F, const __grid_constant__ MeshDev one) {
     extern __shared__ uint32_t s_row[];
     __shared__ uint32_t s_ovf;
@@ -447,7 +488,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
     __syncthreads();
     uint32_t vis = 0, fp = 0;
     for (uint32_t base = blockIdx.x * kRowThreads; base < F.num_tris; base += gridDim.x * kRowThreads) {
-        const uint32_t c = setup_tri<2>(F, base + tid, (base + tid) >> 5, ONE ? &one : nullptr, s_row);
+        const uint32_t c = setup_tri<2, DIRECT>(F, base + tid, (base + tid) >> 5, ONE ? &one : nullptr, s_row);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -610,42 +651,6 @@ __device__ __forceinline__ void raster_fixed(const TriSetup& t, uint32_t prim, u
     }
 }
 
-// One lane's raster of a small triangle: raster_fixed's snapped box,
-// coverage, occlusion test, weights, depth and (key, id) minimum, pixel by
-// pixel (the edge functions evaluated exactly at each pixel equal the
-// stepped ones).  Returns false, having done nothing, for a triangle on the
-// float path or with a box of more than kLanePixels pixels.
-__device__ __forceinline__ bool raster_fixed_lane(const TriSetup& t, uint32_t prim, unsigned long long* tile, int tx0,
-                                                  int ty0, int tw, int th, uint32_t key_bound) {
-    if (t.mesh & kFlagFloat) return false;
-    const int X0 = snap_fx(t.x0), Y0 = snap_fx(t.y0), X1 = snap_fx(t.x1);
-    const int Y1 = snap_fx(t.y1), X2 = snap_fx(t.x2), Y2 = snap_fx(t.y2);
-    const int minx = min(X0, min(X1, X2)), maxx = max(X0, max(X1, X2));
-    const int miny = min(Y0, min(Y1, Y2)), maxy = max(Y0, max(Y1, Y2));
-    const int px0 = max((minx + 0xFFFF) >> kFxBits, tx0), px1 = min(maxx >> kFxBits, tx0 + tw - 1);
-    const int py0 = max((miny + 0xFFFF) >> kFxBits, ty0), py1 = min(maxy >> kFxBits, ty0 + th - 1);
-    if (px0 > px1 || py0 > py1) return true;
-    if ((px1 - px0 + 1) * (py1 - py0 + 1) > kLanePixels) return false;
-    for (int y = py0; y <= py1; ++y)
-        for (int x = px0; x <= px1; ++x) {
-            const int fx = x << kFxBits, fy = y << kFxBits;
-            if (edge_fx(fx, fy, X0, Y0, X1 - X0, Y1 - Y0) < 0 || edge_fx(fx, fy, X1, Y1, X2 - X1, Y2 - Y1) < 0 ||
-                edge_fx(fx, fy, X2, Y2, X0 - X2, Y0 - Y2) < 0)
-                continue;
-            unsigned long long* slot = tile + (y - ty0) * tw + (x - tx0);
-            const unsigned long long cur = *((volatile unsigned long long*)slot);
-            if ((uint32_t)(cur >> 32) < key_bound) continue;   // occluded
-            float w[3];
-            weights_fixed(t, x, y, w);
-            const float z = interp_z(w[0], w[1], w[2], t.z0, t.z1, t.z2);
-            if (!(z >= 0.f && z < 1.f)) continue;
-            const uint32_t key = (uint32_t)__float2int_rz(__fmul_rn(z, 2147483648.0f));
-            const unsigned long long packed = ((unsigned long long)key << 32) | prim;
-            if (packed < cur) atomicMin(slot, packed);
-        }
-    return true;
-}
-
 // Triangles outside the guard band: the reference's float edge functions.
 __device__ __noinline__ void raster_float(const TriSetup& t, uint32_t prim, unsigned long long* tile, int tx0,
                                              int ty0, int tw, int th, uint32_t lane) {
@@ -717,11 +722,10 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& F, int x, int y, u
     F.ids[gi] = prim;
 }
 
-// The record raster: persistent CTAs that stage a phase's setup records in
-// shared memory and merge fragments into a shared tile.  It runs the frames
-// of small triangles (TMA false: a lane per triangle, kLanePhase) and, on
-// request, the bulk-copy staging (TMA); the others take the block raster.
-template <int MIN_CTAS, bool TMA>
+// The record raster, on request (GBR_STAGING_TMA): persistent CTAs that stage
+// a phase's setup records in shared memory by bulk copies and merge
+// fragments into a shared tile, a triangle to a warp.
+template <int MIN_CTAS>
 __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameDev F) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr uint32_t kEntries = kBatch, THREADS = kRasterThreads;
@@ -741,15 +745,12 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
     // an item starts and its descriptor copied to shared memory
     // (asynchronously) while the item is staged
     uint32_t next_idx = 0;
-    constexpr bool tma = TMA;   // setup records staged by bulk copies (a variant for single frames)
     const uint32_t rec_bar0 = smem_addr(&S.rec_bar[0]);
     uint32_t rec_parity = 0;   // bit b: completions of record barrier b seen so far, mod 2
     if (tid == 0) {
-        if (TMA) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rec_bar0) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rec_bar0 + 8u) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rec_bar0) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rec_bar0 + 8u) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         next_idx = atomicAdd(&Q->item_next, 1u);
         fetch_item(&S.item_next, items, next_idx, num_items);
     }
@@ -832,30 +833,20 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
             // between phases.  A triangle whose key bound exceeds it cannot win
             // a pixel; once a whole bucket's lower bound does, the rest of the
             // batch is skipped.
-            // TMA staging: phases of at most kMaxPhase / 2 triangles prefetch
+            // phases of at most kMaxPhase / 2 triangles prefetch
             // the next phase's records into the other half of the ring
-            const bool ahead = tma && phase <= kMaxPhase / 2u;
+            const bool ahead = phase <= kMaxPhase / 2u;
             for (uint32_t p0 = 0, ph = 0; p0 < total; p0 += phase, ph ^= 1u) {
                 __syncthreads();   // the order, or the previous phase's records and tile
                 const uint32_t pn = min(phase, total - p0);
                 const uint32_t bar = rec_bar0 + 8u * ph, bar_next = rec_bar0 + 8u * (ph ^ 1u);
                 const bool next = ahead && p0 + phase < total;   // this phase prefetches the next one's records
-                if (tma) {
-                    if (warp == 0) {
-                        if (p0 == 0u || !ahead)   // this phase's records were not prefetched
-                            issue_records(S.rec, setup, S.prim, S.order, p0, pn, bar, lane, key_mask);
-                        if (next)
-                            issue_records(S.rec, setup, S.prim, S.order, p0 + phase, min(phase, total - p0 - phase),
-                                          bar_next, lane, key_mask);
-                    }
-                } else {
-                    // 16 bytes per thread (triangle k's record goes to slot k
-                    // mod kMaxPhase: phase <= kMaxPhase)
-                    for (uint32_t r = tid; r < 3u * pn; r += THREADS) {
-                        const uint32_t q = r / 3u, k = p0 + q;
-                        const uint4* rp = reinterpret_cast<const uint4*>(setup) + 3u * (size_t)list_id(S.prim[S.order[k]], key_mask);
-                        reinterpret_cast<uint4*>(&S.rec[k & (kMaxPhase - 1u)])[r - 3u * q] = __ldg(rp + (r - 3u * q));
-                    }
+                if (warp == 0) {
+                    if (p0 == 0u || !ahead)   // this phase's records were not prefetched
+                        issue_records(S.rec, setup, S.prim, S.order, p0, pn, bar, lane, key_mask);
+                    if (next)
+                        issue_records(S.rec, setup, S.prim, S.order, p0 + phase, min(phase, total - p0 - phase), bar_next,
+                                      lane, key_mask);
                 }
                 if (b0 > 0 || p0 > 0) {
                     uint32_t m = 0;
@@ -869,10 +860,8 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
                 // every thread sees this phase's records land before any phase
                 // decision; a phase that ends the batch early also waits for
                 // the records it prefetched, so no copy is ever left in flight
-                if (tma) {
-                    if (!rec_wait(bar, (rec_parity >> ph) & 1u) && tid == 0) atomicOr(&Q->error, 8u);
-                    rec_parity ^= 1u << ph;
-                }
+                if (!rec_wait(bar, (rec_parity >> ph) & 1u) && tid == 0) atomicOr(&Q->error, 8u);
+                rec_parity ^= 1u << ph;
                 uint32_t tile_max = 0xFFFFFFFFu;
                 if (b0 > 0 || p0 > 0) {
                     tile_max = 0;
@@ -889,38 +878,16 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
                     break;
                 }
                 const uint32_t p1 = min(limit, p0 + phase);
-                // a warp takes one sorted triangle at a time; the
-                // small-triangle variant takes kLaneGrab in phases of at least
-                // kLanePhase triangles, each lane rasterises its own when its
-                // pixel box holds at most kLanePixels pixels, and the warp the
-                // others
-                const bool lanes = !TMA && phase >= kLanePhase;
-                for (;;) {
+                for (;;) {   // a warp takes one sorted triangle at a time
                     int kb = 0;
-                    if (lane == 0) kb = atomicAdd(&S.next, lanes ? (int)kLaneGrab : 1);
+                    if (lane == 0) kb = atomicAdd(&S.next, 1);
                     kb = __shfl_sync(0xFFFFFFFFu, kb, 0);
                     if (kb >= (int)p1) break;
-                    uint32_t m;   // bit l: triangle kb + l goes to the whole warp
-                    if (lanes) {
-                        const uint32_t k = (uint32_t)kb + lane;
-                        bool big = false;
-                        if (lane < kLaneGrab && k < p1) {
-                            const uint32_t i = S.order[k];
-                            const TriSetup& t = S.rec[k & (kMaxPhase - 1u)];
-                            if (t.key <= tile_max)
-                                big = !raster_fixed_lane(t, list_id(S.prim[i], key_mask), tile, tx0, ty0, tw, th, t.key);
-                        }
-                        m = __ballot_sync(0xFFFFFFFFu, big);
-                    } else {
-                        m = S.rec[(uint32_t)kb & (kMaxPhase - 1u)].key <= tile_max ? 1u : 0u;
-                    }
-                    for (; m; m &= m - 1u) {
-                        const uint32_t k = (uint32_t)kb + (uint32_t)(__ffs(m) - 1), i = S.order[k];
-                        const TriSetup& t = S.rec[k & (kMaxPhase - 1u)];
-                        const uint32_t prim = list_id(S.prim[i], key_mask);
-                        if (t.mesh & kFlagFloat) raster_float(t, prim, tile, tx0, ty0, tw, th, lane);
-                        else raster_fixed(t, prim, tile, tx0, ty0, tw, th, lane, t.key);
-                    }
+                    const TriSetup& t = S.rec[(uint32_t)kb & (kMaxPhase - 1u)];
+                    if (t.key > tile_max) continue;
+                    const uint32_t prim = list_id(S.prim[S.order[kb]], key_mask);
+                    if (t.mesh & kFlagFloat) raster_float(t, prim, tile, tx0, ty0, tw, th, lane);
+                    else raster_fixed(t, prim, tile, tx0, ty0, tw, th, lane, t.key);
                 }
             }
         }
@@ -958,7 +925,11 @@ __device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint3
         const uint32_t yk = y + k * (kTileH / 2u);
         v[k] = yk < y1 ? F.gvis[(size_t)yk * F.width + x] : kEmptyVis;
     }
-    if (skip && *skip) return;   // a frame that was not rasterised
+    if (skip && *skip) {   // a frame that was not rasterised, but for the set-up pass's small triangles
+        for (uint32_t k = 0; k < 2u && F.direct; ++k)
+            if (v[k] != kEmptyVis) F.gvis[(size_t)(y + k * (kTileH / 2u)) * F.width + x] = kEmptyVis;
+        return;
+    }
 #pragma unroll
     for (uint32_t k = 0; k < 2u; ++k) {
         const uint32_t yk = y + k * (kTileH / 2u);
@@ -997,6 +968,8 @@ __global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : KIND == kShadeFl
 // queues its covered pixels with one atomic.  Buffers not 16-byte aligned
 // take per-pixel accesses.
 __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
+    // pixels [px_begin, px_end) (px_begin a multiple of 4)
+    const uint32_t n = F.px_end ? F.px_end : F.width * F.height;
     pdl_wait();
     if (F.ctl->overflow) {
         // not rasterised: the buffers keep the last frame's pixels, and the
@@ -1004,10 +977,13 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
         if (F.dirty_rd)
             for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < F.num_bins; b += gridDim.x * blockDim.x)
                 F.dirty_wr[b] |= F.dirty_rd[b];
+        // what the set-up pass has drawn goes
+        if (F.direct)
+            for (uint32_t i = F.px_begin + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+                F.gvis[i] = kEmptyVis;
         return;
     }
-    // pixels [px_begin, px_end) (px_begin a multiple of 4)
-    const uint32_t n = F.px_end ? F.px_end : F.width * F.height, lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t i0 = F.px_begin + (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
     const bool aligned = ((reinterpret_cast<uintptr_t>(F.gvis) | reinterpret_cast<uintptr_t>(F.colour) |
                            reinterpret_cast<uintptr_t>(F.depth) | reinterpret_cast<uintptr_t>(F.ids)) & 15u) == 0u;
@@ -1207,7 +1183,7 @@ __global__ void __launch_bounds__(256) batch_fill_kernel(BatchDev B) {
     __shared__ __align__(16) FrameDev sF;
     const uint32_t sc = __ldg(B.tri_scene + blockIdx.x);
     load_scene(B, sc, sF);
-    fill_tri<1>(sF, (blockIdx.x - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x, (blockIdx.x * 256u + threadIdx.x) >> 5);
+    fill_tri<1, false>(sF, (blockIdx.x - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x, (blockIdx.x * 256u + threadIdx.x) >> 5);
 }
 
 // KIND: every scene of the batch shades flat (B.all_flat), from one mesh, and
@@ -1260,7 +1236,9 @@ static cudaError_t row_smem(const FrameDev& F, size_t* bytes) {
     if (!(opted & bit)) {
         const int most = (int)(kMaxRowBins * sizeof(uint32_t));
         e = cudaFuncSetAttribute(fill_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        for (auto* k : {setup_rows_kernel<true>, setup_rows_kernel<false>, predicted_rows_kernel<true>, predicted_rows_kernel<false>})
+        for (auto* k : {setup_rows_kernel<true>, setup_rows_kernel<false>, predicted_rows_kernel<true, true>,
+                        predicted_rows_kernel<true, false>, predicted_rows_kernel<false, true>,
+                        predicted_rows_kernel<false, false>})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
         opted |= bit;
@@ -1274,12 +1252,16 @@ static cudaError_t launch_setup(const FrameDev& F, const MeshDev& one, bool pred
         size_t smem = 0;
         const cudaError_t e = row_smem(F, &smem);
         if (e != cudaSuccess) return e;
-        return launch_pdl(predicted ? predicted_rows_kernel<ONE> : setup_rows_kernel<ONE>, dim3(F.row_blocks),
-                          dim3(kRowThreads), smem, s, F, one);
+        return launch_pdl(!predicted ? setup_rows_kernel<ONE>
+                          : F.direct ? predicted_rows_kernel<ONE, true>
+                                     : predicted_rows_kernel<ONE, false>,
+                          dim3(F.row_blocks), dim3(kRowThreads), smem, s, F, one);
     }
     const uint32_t blocks = triangle_blocks(F.num_tris);
     if (blocks == 0) return cudaSuccess;
-    return launch_pdl(predicted ? setup_kernel<1, ONE> : setup_kernel<0, ONE>, dim3(blocks), dim3(256), 0, s, F, one);
+    return launch_pdl(predicted ? (F.direct ? setup_kernel<1, ONE, true> : setup_kernel<1, ONE>)
+                                : (F.direct ? setup_kernel<0, ONE, true> : setup_kernel<0, ONE>),
+                      dim3(blocks), dim3(256), 0, s, F, one);
 }
 
 cudaError_t launch_setup(const FrameDev& F, const MeshDev* one, bool predicted, cudaStream_t s) {
@@ -1298,7 +1280,9 @@ cudaError_t launch_fill(const FrameDev& F, cudaStream_t s) {
     }
     const uint32_t blocks = triangle_blocks(F.num_tris);
     if (blocks == 0) return cudaSuccess;
-    return launch_pdl(F.fused_scan ? fill_fused_kernel : fill_kernel, dim3(blocks), dim3(256), 0, s, F);
+    return launch_pdl(F.direct ? (F.fused_scan ? fill_fused_kernel<true> : fill_kernel<true>)
+                               : (F.fused_scan ? fill_fused_kernel<false> : fill_kernel<false>),
+                      dim3(blocks), dim3(256), 0, s, F);
 }
 
 static size_t record_smem(uint32_t bw, uint32_t bh) {
@@ -1307,35 +1291,31 @@ static size_t record_smem(uint32_t bw, uint32_t bh) {
 
 using RecordRaster = void (*)(FrameDev);
 
-template <bool TMA>
 static RecordRaster record_variant(uint32_t ctas) {
     switch (ctas ? ctas : kDefaultRasterCtas) {
-        case 2: return raster_kernel<2, TMA>;
-        case 3: return raster_kernel<3, TMA>;
-        case 5: return raster_kernel<5, TMA>;
-        case 6: return raster_kernel<6, TMA>;
-        default: return raster_kernel<4, TMA>;
+        case 2: return raster_kernel<2>;
+        case 3: return raster_kernel<3>;
+        case 5: return raster_kernel<5>;
+        case 6: return raster_kernel<6>;
+        default: return raster_kernel<4>;
     }
 }
 
 cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid* per_sm) {
     const size_t smem = record_smem(bw, bh);
-    for (const RecordRaster k : {record_variant<true>(ctas), record_variant<false>(ctas)}) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm->record, k, kRasterThreads, smem);
-        if (e != cudaSuccess) return e;
-    }
-    cudaError_t e = block_raster_configure(bw, bh, false, 128u, ctas, &per_sm->block128);
+    const RecordRaster k = record_variant(ctas);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm->record, k, kRasterThreads, smem);
+    if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, 128u, ctas, &per_sm->block128);
     if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, 512u, ctas, &per_sm->block512);
     for (int* n : {&per_sm->record, &per_sm->block128, &per_sm->block512}) *n = std::max(*n, 1);
     return e;
 }
 
 cudaError_t launch_raster(const FrameDev& F, const RasterGrid& per_sm, cudaStream_t s) {
-    if (F.rec_tma || F.raster_lanes)
-        return launch_pdl(F.rec_tma ? record_variant<true>(F.raster_ctas) : record_variant<false>(F.raster_ctas),
-                          dim3((uint32_t)(sm_count() * per_sm.record)), dim3(kRasterThreads), record_smem(F.bw, F.bh), s,
-                          F);
+    if (F.rec_tma)
+        return launch_pdl(record_variant(F.raster_ctas), dim3((uint32_t)(sm_count() * per_sm.record)),
+                          dim3(kRasterThreads), record_smem(F.bw, F.bh), s, F);
     BatchDev none;
     memset(&none, 0, sizeof none);
     return launch_block_raster(F, none, false, F.block_threads, F.raster_ctas, F.bw, F.bh,

@@ -461,14 +461,16 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
         }
         if (count == 0u) __syncthreads();   // the tile's initial values
         // publish: one chunk owns its pixels (plain stores); the chunks of a
-        // longer bin merge with 64-bit atomicMin
+        // longer bin merge with 64-bit atomicMin, among themselves and with
+        // what the set-up pass has drawn
+        const bool own = nchunks == 1u && !G.direct;
         for (uint32_t blk = warp; blk < nblk; blk += kWarps) {
             const uint32_t by = blk * inv >> 10, bx = blk - by * nbw;
             const int x = (int)bx * kBlockW + lx, y = (int)by * kBlockH + ly;
             const unsigned long long best = tile[blk * 32u + lane];
             if (x >= tw || y >= th || best == kEmptyVis) continue;
             unsigned long long* g = &G.gvis[(size_t)(ty0 + y) * G.width + (size_t)(tx0 + x)];
-            if (nchunks == 1u) *g = best;
+            if (own) *g = best;
             else atomicMin(g, best);
         }
     }

@@ -29,7 +29,8 @@ __device__ __forceinline__ void close_counters(Ctl* c) {
 // zero for the next frame.
 __device__ __forceinline__ void zero_counts(const FrameDev& F) {
     if (F.fused_scan)
-        for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < F.num_bins; b += gridDim.x * blockDim.x) F.counts[b] = 0u;
+        for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < F.count_split * F.num_bins; b += gridDim.x * blockDim.x)
+            F.counts[b] = 0u;
 }
 
 }  // namespace gbr

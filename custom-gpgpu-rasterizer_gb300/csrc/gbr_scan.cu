@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
     __shared__ unsigned long long s_excl[2];
     __shared__ uint32_t s_tile, s_tag;
     pdl_wait();
-    if (S.dirty)   // before any wait: a scan that gives up has still cleared them
+    if (S.dirty && S.mode == kScanCapacity)   // before any wait: a scan that gives up has still cleared them
         for (uint32_t b = blockIdx.x * 1024u + threadIdx.x; b < S.n; b += gridDim.x * 1024u) S.dirty[b] = 0u;
     if (S.mode == kScanPredictedItems && S.feat) {
         // the pre-pass accumulators start the next frame empty (also when
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
     if (tile >= ntiles) return;
     const uint32_t b = tile * 1024u + threadIdx.x;
     const bool exact = S.mode == kScanExact || S.mode == kScanExactAfterPredicted;
-    uint32_t c = 0, it = 0;
+    uint32_t c = 0, cr = 0, it = 0;   // entries, those the raster reads (the first ones), work items
     uint32_t sub[kCountSplit];   // exact modes: the bin's sub-counts (zeroed for the next frame)
     if (b < S.n) {
         if (exact) {
@@ -207,12 +207,14 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
                     sub[k] = S.counts[k * S.n + b];
                     S.counts[k * S.n + b] = 0u;
                     c += sub[k];
+                    if (k < S.raster_split) cr += sub[k];
                 }
             }
+            if (S.dirty) S.dirty[b] = c ? 1u : 0u;
         } else {
-            c = predicted_size(S, b);
+            c = cr = predicted_size(S, b);
         }
-        it = bin_items(c, S.chunk);
+        it = bin_items(cr, S.chunk);
     }
     unsigned long long ia = c, ib = it, ta, tb;
     block_scan2(ia, ib, s_a, s_b, ta, tb);
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
                 const uint32_t start = exact ? (uint32_t)run : S.offsets[b];
                 const uint32_t chunk = S.chunk;
                 for (uint32_t k = 0; k < it; ++k)
-                    S.items[item + k] = make_uint4(b, start + k * chunk, min(chunk, c - min(c, k * chunk)), it);
+                    S.items[item + k] = make_uint4(b, start + k * chunk, min(chunk, cr - min(cr, k * chunk)), it);
             }
         }
     }
@@ -286,6 +288,7 @@ ScanDev scan_of(const FrameDev& F, uint32_t mode) {
     S.counts = F.counts;
     S.sub_base = F.sub_base;
     S.split = F.count_split;
+    S.raster_split = F.direct ? F.count_split >> 1 : F.count_split;
     S.capacity = F.capacity;
     S.offsets = F.offsets;
     S.cursors = F.cursors;
@@ -301,9 +304,9 @@ ScanDev scan_of(const FrameDev& F, uint32_t mode) {
     S.mode = mode;
     S.spin_limit = F.scan_spin_limit;
     S.silent_tile1 = F.scan_silent_tile1;
-    // the frame's first scan (exact, or the predicted capacities) clears
-    // the drawn flags the raster sets
-    S.dirty = mode == kScanExact || mode == kScanCapacity ? F.dirty_wr : nullptr;
+    // the scan that places a frame's exact lists flags its bins; the
+    // capacity scan clears the flags for the raster
+    S.dirty = mode == kScanPredictedItems ? nullptr : F.dirty_wr;
     return S;
 }
 

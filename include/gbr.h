@@ -79,8 +79,8 @@ typedef struct {
     float ms_shade;              /* the shade pass (included in ms_total, not in ms_raster) */
     uint32_t count_blocks;       /* blocks with private counter rows in the last frame's exact
                                     count pass (0: per-bin counters in global memory) */
-    uint32_t raster_lanes;       /* 1: the last frame's raster took its small-triangle variant (a lane
-                                    per triangle; picked for sparse frames of small triangles) */
+    uint32_t raster_lanes;       /* 1: the last frame's small triangles were rasterised a lane per triangle, by
+                                    the set-up pass (picked for sparse frames of small triangles) */
     uint32_t reserved;
 } gbr_stats;
 
@@ -222,10 +222,9 @@ gbr_status gbr_set_lights(gbr_renderer *r, const gbr_light *lights, uint32_t n);
 /* Binning method for the following frames. */
 gbr_status gbr_set_binning(gbr_renderer *r, uint32_t method);
 /* Raster tuning (no counterpart in the reference; used by the autotuner):
- * phase = triangles the small-triangle and bulk-copy raster variants rasterise between hierarchical-z
- * refreshes, 0..128 (0: the library's choice: 16, 64 for frames of small triangles, 128 with the
- * small-triangle variant; below 32 the small-triangle variant is not taken; the block raster refreshes after
- * every triangle), ctas_per_sm = occupancy variant of the raster kernel in CTAs of 256 threads, 2..6 (0: the
+ * phase = triangles the raster with bulk-copy staging rasterises between hierarchical-z refreshes, 0..128
+ * (0: the library's choice: 16, 64 for frames of small triangles); the default raster refreshes after every
+ * triangle, and with a phase of 1..31 leaves no triangle to the set-up pass; ctas_per_sm = occupancy variant of the raster kernel in CTAs of 256 threads, 2..6 (0: the
  * library's choice). */
 gbr_status gbr_set_raster_params(gbr_renderer *r, uint32_t phase, uint32_t ctas_per_sm);
 /* How the raster stages triangle-setup records into shared memory (no

@@ -4,11 +4,13 @@ blocks than a CTA has warps and of many times more, items around one phase
 (32 triangles) and around one sorted pass (1024 and 2048 entries), triangles
 around and far above the extent that keeps 32-bit edge values, and triangles
 on the float path.  Winners and depth bit-exact, colour within 1 LSB."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import scenes
-from oracle import oracle
+from oracle import mlp_oracle, oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +93,84 @@ def test_list_entries_with_and_without_depth(gbr_lib, cuda_device, n):
             offsets, bins = r.get_bins()
             assert np.array_equal(offsets, o["offsets"]) and np.array_equal(bins, o["bins"])
             assert np.array_equal(r.readback_ids(), o["ids"])
+
+
+def small_beside_large(w, h, vertex_colours, px=3.5):
+    rng = np.random.default_rng(3)
+    n = 9000
+    c = rng.uniform(-0.95, 0.95, (n, 1, 2))
+    size = rng.uniform(0.2, px, (n, 1, 1)) * 2.0 / np.array([w, h])
+    ang = rng.uniform(0, 2 * np.pi, (n, 1)) - np.arange(3) * (2 * np.pi / 3)
+    v = np.zeros(3 * n, scenes.IVERTEX56)
+    p = v["p"].reshape(-1, 3, 3)
+    p[:, :, :2] = c + size * np.stack([np.cos(ang), -np.sin(ang)], -1)
+    p[:, :, 2] = rng.uniform(0.05, 0.95, (n, 1))
+    p[::1500, 0, :2] += rng.uniform(0.1, 0.5, (6, 2))
+    p[5, 0, 0] = 60.0
+    p[5, 2] = p[5, 0] + (0.0, 0.02, 0.0)
+    v["p"] = p.reshape(-1, 3)
+    v["uv"] = rng.uniform(0, 1, (3 * n, 2))
+    v["n"] = (0, 0, 1)
+    v["tan"] = (1, 0, 0)
+    v["c"] = rng.uniform(0, 1, (3 * n, 3))
+    m = scenes.Mesh(vertices=v)
+    if not vertex_colours:
+        m.textures = [scenes.checker_texture(64, 8), scenes.flat_texture(64, (128, 128, 255)), None, None]
+    return m
+
+
+@pytest.mark.parametrize("vertex_colours", [True, False])
+@pytest.mark.parametrize("w,h,bw,bh", [(640, 480, 16, 16), (333, 250, 24, 20), (1024, 600, 8, 8)])
+def test_direct_small_triangles_beside_large_ones(gbr_lib, cuda_device, w, h, bw, bh, vertex_colours):
+    """A frame of small triangles, drawn by the set-up pass, around boxes of
+    16 pixels (its limit) and among them a few large, very large and float-path
+    triangles, drawn by the raster: lists, winners and depth are the oracle's
+    (flat- and texture-shaded frames, one and two passes)."""
+    m = small_beside_large(w, h, vertex_colours)
+    s = scenes.Scene("direct", w, h, bw, bh, scenes.identity_camera(), [m], cull=scenes.CULL_NONE)
+    o = oracle.render(s, oracle.RASTER_FIXED)
+    assert o["stats"]["num_float_path"] == 1
+    with gbr_lib.Renderer(w, h) as r:
+        r.load_scene(s)
+        for frame in range(3):
+            r.render_scene(s)
+            colour, depth = r.readback()
+            offsets, bins = r.get_bins()
+            assert np.array_equal(offsets, o["offsets"]) and np.array_equal(bins, o["bins"]), f"frame {frame}: lists"
+            assert np.array_equal(r.readback_ids(), o["ids"]), f"frame {frame}: winners"
+            assert np.array_equal(depth.view(np.uint32), o["depth"].view(np.uint32)), f"frame {frame}: depth"
+            c0, c1 = colour.astype(np.int64), o["colour"].astype(np.int64)
+            assert max(np.abs(((c0 >> k) & 255) - ((c1 >> k) & 255)).max() for k in (0, 8, 16)) <= 1
+            assert r.stats()["raster_lanes"] == (1 if frame else 0)
+
+
+@pytest.mark.parametrize("per_bin", [29.0, 3.0])
+@pytest.mark.parametrize("w,h,bin_size,px", [(640, 480, 16, 3.5), (2048, 1088, 8, 2.5)])   # bins within and beyond shared memory's rows
+def test_direct_small_triangles_with_predicted_capacities(gbr_lib, cuda_device, w, h, bin_size, px, per_bin):
+    """The same under predicted binning: capacities that hold every bin (the
+    lists carry drawn and undrawn entries together), and capacities that
+    overflow (the exact pass draws the small triangles once more)."""
+    m = small_beside_large(w, h, True, px)
+    s = scenes.Scene("direct", w, h, bin_size, bin_size, scenes.identity_camera(), [m], cull=scenes.CULL_NONE)
+    o = oracle.render(s, oracle.RASTER_FIXED)
+    most = int(np.diff(o["offsets"].astype(np.int64)).max())
+    assert 4 < most <= 29
+    weights = np.zeros(mlp_oracle.NUM_PARAMS, np.float32)
+    weights[mlp_oracle.OFF_B3] = per_bin
+    w16 = mlp_oracle.f32_to_bf16(weights)
+    with gbr_lib.Renderer(w, h) as r:
+        r.load_scene(s)
+        r.render_scene(s)
+        r.stats()
+        gbr_lib.check(r._lib.gbr_set_predictor(r.h, w16.ctypes.data_as(C.c_void_p), len(w16), C.c_float(0.0),
+                                               C.c_float(0.0), C.c_float(0.0)))
+        r.set_binning(gbr_lib.BINNING_PREDICTED)
+        for frame in range(3):
+            r.render_scene(s)
+            _, depth = r.readback()
+            st = r.stats()
+            assert st["raster_lanes"] == 1 and st["predicted_overflow"] == (per_bin < most)
+            offsets, bins = r.get_bins()
+            assert np.array_equal(offsets, o["offsets"]) and np.array_equal(bins, o["bins"]), f"frame {frame}: lists"
+            assert np.array_equal(r.readback_ids(), o["ids"]), f"frame {frame}: winners"
+            assert np.array_equal(depth.view(np.uint32), o["depth"].view(np.uint32)), f"frame {frame}: depth"

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("w,h,bin_size,n", [
-    (16, 16, 16, 40),            # one bin
+    (16, 16, 16, 40),            # one bin (and a pair a triangle: taken for small triangles)
     (31 * 4, 4, 4, 300),         # one row of bins short of 32, whole, and one over
     (32 * 4, 4, 4, 300),
     (33 * 4, 4, 4, 300),
@@ -35,8 +35,9 @@ def test_fused_scan_against_the_oracle(gbr_lib, cuda_device, w, h, bin_size, n):
             assert np.array_equal(r.readback_ids(), o["ids"]), f"frame {frame}"
             st = r.stats()
             assert st["num_pairs"] == o["stats"]["num_pairs"] and st["num_visible"] == o["stats"]["num_visible"]
-            # later frames count in block rows: the first frame showed at
-            # least a pair per (block, bin)
+            # later frames count in block rows (the first frame showed at
+            # least a pair per (block, bin)), but for one of small triangles,
+            # whose lists keep apart what the set-up pass has drawn
             blocks = min((n + 1023) // 1024, torch.cuda.get_device_properties(0).multi_processor_count)
             assert st["num_pairs"] >= s.num_bins_x * s.num_bins_y * blocks
-            assert st["count_blocks"] == (blocks if frame else 0)
+            assert st["count_blocks"] == (blocks if frame and not st["raster_lanes"] else 0)
