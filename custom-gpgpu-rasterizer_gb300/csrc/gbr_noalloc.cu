@@ -25,6 +25,7 @@
 // the same device) race on it and must be serialised by the caller.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -147,9 +148,13 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
         }
         slot = s;
     }
+    // the one raster variant that the frame launches
+    const uint32_t block_threads = block_threads_for(nb, (uint32_t)slot.num_sms);
     RasterGrid per_sm;
-    e = raster_configure(bin_w, bin_h, 0u, &per_sm);
+    int& ctas = block_threads == 512u ? per_sm.block512 : per_sm.block128;
+    e = block_raster_configure(bin_w, bin_h, false, block_threads, 0u, &ctas);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
+    ctas = std::max(ctas, 1);
 
     unsigned char* b = slot.base;
     FrameDev F;
@@ -167,7 +172,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     F.fused_scan = tris > 0u ? 1u : 0u;   // the scratch's limits are the fused scan's
     static_assert(kNaMaxBins <= kFusedBins && kNaMaxTris <= kFusedTris, "fused scan limits");
     F.stage = queue_chunk;    // entries per raster pass
-    F.block_threads = block_threads_for(nb, (uint32_t)slot.num_sms);
+    F.block_threads = block_threads;
     for (int k = 0; k < 3; ++k) { F.cam_pos[k] = cam->pos[k]; F.cam_fwd[k] = cam->fwd[k]; }
     F.meshes = reinterpret_cast<const MeshDev*>(b + kOffMesh);
     F.setup = reinterpret_cast<TriSetup*>(b + kOffSetup);
@@ -224,10 +229,9 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     if (e == cudaSuccess) e = launch_shade(F, nullptr, s);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
     // the frame is only valid if its bin entries fitted the static storage
-    e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
     Ctl ctl;
-    e = cudaMemcpy(&ctl, b + kOffCtl, sizeof ctl, cudaMemcpyDeviceToHost);
+    e = cudaMemcpyAsync(&ctl, b + kOffCtl, sizeof ctl, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
     if (ctl.overflow) return na_fail(GBR_ERR_OUT_OF_MEMORY, "frame needs more than 2^20 bin entries");
     if (ctl.error) return na_fail(GBR_ERR_TIMEOUT, "bin scan wait timed out; the frame is invalid");
