@@ -119,9 +119,11 @@ __device__ __forceinline__ void reduce_triangle(const TriSetup* setup, uint32_t 
         qa = bin_edge(fx, fy, X0, Y0, dxa, dya);
         qb = bin_edge(fx, fy, X1, Y1, dxb, dyb);
         qc = bin_edge(fx, fy, X2, Y2, dxc, dyc);
-        // steps across the bin: at most (tw + th) times the extent
+        // steps across the bin's blocks, which may reach past its last pixels:
+        // at most their width + height times the extent
         kind = kTriWide;
-        if ((long long)max(maxx - minx, maxy - miny) * (tw + th) < kEdgeClamp) {
+        const int span = ((tw + kBlockW - 1) & -kBlockW) + ((th + kBlockH - 1) & -kBlockH);
+        if ((long long)max(maxx - minx, maxy - miny) * span < kEdgeClamp) {
             kind = kTriNarrow;
             qa = narrow_edge(qa);
             qb = narrow_edge(qb);

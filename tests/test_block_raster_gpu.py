@@ -24,6 +24,12 @@ def triangles(kind, n, width, height, seed):
         return v
     rng = np.random.default_rng(seed)
     p = v["p"].reshape(-1, 3, 3)
+    if kind == "vast":     # screen-filling triangles of 3000 to 8000 px
+        reach = rng.uniform(1500.0, 4000.0, (n, 1, 1)) * 2.0 / np.array([width, height])
+        angle = rng.uniform(0, 2 * np.pi, (n, 1)) - np.arange(3) * (2 * np.pi / 3)
+        p[:, :, :2] = rng.uniform(-0.5, 0.5, (n, 1, 2)) + reach * np.stack([np.cos(angle), -np.sin(angle)], -1)
+        v["p"] = p.reshape(-1, 3)
+        return v
     # every fourth triangle's first vertex thrown out to the given distance:
     # extents around 128 to 1024 px (the 32-bit limit is 2^14 px over the
     # bin's width + height), thousands of px, or beyond the guard band
@@ -38,6 +44,9 @@ def triangles(kind, n, width, height, seed):
 
 @pytest.mark.parametrize("bw,bh,w,h,n,kind", [
     (1, 1, 40, 24, 60, "small"),           # one pixel a bin, eight warps on one block
+    (1, 1, 40, 24, 60, "vast"),            # blocks that reach far past their bins
+    (2, 3, 40, 24, 200, "vast"),
+    (9, 5, 90, 61, 500, "vast"),
     (8, 4, 96, 60, 400, "small"),          # one block a bin
     (7, 5, 100, 61, 600, "wide"),          # ragged blocks, ragged last bins
     (8, 8, 128, 96, 33, "huge"),           # items of at most a phase
