@@ -69,7 +69,8 @@ constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
 // The block raster's CTAs in a single frame: 128 threads where the items
 // outnumber the SMs several times (fewer warps wait at each of an item's
 // barriers than in CTAs of 256: 1M soup 78 us against 88, 2M soup at 4K 201
-// against 285; of 64: 94 and 195), 512 where they don't and the longest item
+// against 285; frames in CTAs of 64: 198 against 176, and 430 against 442),
+// 512 where they don't and the longest item
 // decides.
 constexpr uint32_t kWideItemsPerSm = 6;
 __host__ __device__ inline uint32_t block_threads_for(unsigned long long items, uint32_t sms) {

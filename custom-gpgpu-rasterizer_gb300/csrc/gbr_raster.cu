@@ -5,13 +5,14 @@
 // them in phases of 32 triangles (128 in CTAs of 512 threads):
 //   - a thread each, the phase's triangles are loaded, snapped and reduced to
 //     three 32-bit edge values at the bin's first pixel (reduce_triangle);
-//   - each warp owns blocks of 8x4 pixels of the bin, a pixel a lane, whose
+//   - each warp owns blocks of 8x4 pixels of the bin, a pixel a lane (in CTAs
+//     of 128 and 256 threads pairs of them, two pixels a lane), whose
 //     best (depth key, primitive) it keeps in registers.  It tests 32
-//     triangles at once, a lane each, against the block (depth bound, box,
-//     edges), then takes the ones that meet it one after another, every lane
-//     testing its own pixel.
+//     triangles at once, a lane each, against the blocks (depth bound, box,
+//     edges), then takes the ones that meet them one after another, every lane
+//     testing its own pixels.
 // A warp is done once the next triangle's depth bucket lies behind its
-// block's farthest key, the item once every warp is.
+// blocks' farthest key, the item once every warp is.
 //
 // Why: a warp that sweeps a whole triangle over the bin pays the triangle's
 // set-up (some 120 instructions) in all 32 lanes, steps 64-bit edge values
@@ -55,12 +56,17 @@ struct PhaseTris {
 
 // CTAs of 128 or 256 threads fill the SM; those of 512 run frames of few
 // items, whose time is that of their longest one: several warps share a
-// block's triangles and a phase holds more of them.
+// block's triangles and a phase holds more of them.  Two pixels a lane read a
+// triangle and step its edges once for both, and a pair of blocks goes
+// through the tests and the tile's loads once (batch of 32 uneven soups,
+// 32x32 bins: 394M -> 335M instructions, frame 1005 -> 982 us; 2M soup at 4K,
+// 16x16: 449 -> 443; phases of 64: 457).
 template <int THREADS>
 struct BlockShared {
     static constexpr uint32_t kWarps = THREADS / 32u;
     static constexpr uint32_t kEntries = THREADS == 128 ? 1024u : 2048u;   // entries depth-sorted at once
     static constexpr uint32_t kPhase = THREADS == 512 ? 128u : 32u;        // triangles reduced at once
+    static constexpr int kPixels = THREADS == 512 ? 1 : 2;                 // a lane's pixels, blocks below one another
     PhaseTris<kPhase> tri;
     uint32_t sorted[kEntries];              // staged entries, front to back by bucket
     uint32_t hist[2][kSortBuckets];         // entries per bucket; passes alternate, each zeroed after its scan
@@ -122,7 +128,7 @@ __device__ __forceinline__ void reduce_triangle(const TriSetup* setup, uint32_t 
         // steps across the bin's blocks, which may reach past its last pixels:
         // at most their width + height times the extent
         kind = kTriWide;
-        const int span = ((tw + kBlockW - 1) & -kBlockW) + ((th + kBlockH - 1) & -kBlockH);
+        const int span = ((tw + kBlockW - 1) & -kBlockW) + ((th + 2 * kBlockH - 1) & (-2 * kBlockH));
         if ((long long)max(maxx - minx, maxy - miny) * span < kEdgeClamp) {
             kind = kTriNarrow;
             qa = narrow_edge(qa);
@@ -160,25 +166,35 @@ __device__ __forceinline__ int edges_at(uint4 q, uint4 d, uint4 c, const PhaseTr
     return (int)(e >> 32);
 }
 
-// Does phase triangle `k` meet the block of pixels [bx, bx + 7] x [by,
-// by + 3] of the bin, with a fragment possibly at or before key `far`?  Its
-// box overlaps the block's, and no edge is negative on the whole block.
-template <uint32_t P>
-__device__ __forceinline__ bool meets_block(const PhaseTris<P>& tri, uint32_t k, int bx, int by, uint32_t far,
-                                            uint32_t& kind, uint32_t& key) {
+// Which of the R blocks of pixels [bx, bx + 7] x [by + 4 r, by + 4 r + 3] of
+// the bin does phase triangle `k` meet, with a fragment possibly at or before
+// key far[r]?  Its box overlaps the block's, and no edge is negative on the
+// whole block.
+template <int R, uint32_t P>
+__device__ __forceinline__ void meets_blocks(const PhaseTris<P>& tri, uint32_t k, int bx, int by, const uint32_t (&far)[R],
+                                             uint32_t& kind, uint32_t& key, bool (&hit)[R]) {
     const uint4 c = tri.c[k];
     key = c.z;
     const int x0 = (int)(c.w & 63u), x1 = (int)((c.w >> 8) & 63u), y0 = (int)((c.w >> 16) & 63u), y1 = (int)(c.w >> 24);
     kind = (c.w >> 6) & 3u;
-    const int ex = bx + kBlockW - 1, ey = by + kBlockH - 1;
-    if (c.z > far || x0 > ex || x1 < bx || y0 > ey || y1 < by) return false;
-    if (kind == kTriFloat) return true;
+    const int ex = bx + kBlockW - 1;
+    bool some = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        hit[r] = c.z <= far[r] && x0 <= ex && x1 >= bx && y0 <= by + kBlockH * (r + 1) - 1 && y1 >= by + kBlockH * r;
+        some |= hit[r];
+    }
+    if (!some || kind == kTriFloat) return;
     const uint4 q = tri.a[k], d = tri.b[k];
-    const int xa = (int)d.x > 0 ? ex : bx, ya = (int)d.y > 0 ? ey : by;
-    const int xb = (int)d.z > 0 ? ex : bx, yb = (int)d.w > 0 ? ey : by;
-    const int xc = (int)c.x > 0 ? ex : bx, yc = (int)c.y > 0 ? ey : by;
-    if (kind == kTriNarrow) return edges_at<false>(q, d, c, tri, k, xa, ya, xb, yb, xc, yc) >= 0;
-    return edges_at<true>(q, d, c, tri, k, xa, ya, xb, yb, xc, yc) >= 0;
+    const int xa = (int)d.x > 0 ? ex : bx, ya = (int)d.y > 0 ? by + kBlockH - 1 : by;
+    const int xb = (int)d.z > 0 ? ex : bx, yb = (int)d.w > 0 ? by + kBlockH - 1 : by;
+    const int xc = (int)c.x > 0 ? ex : bx, yc = (int)c.y > 0 ? by + kBlockH - 1 : by;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int dy = kBlockH * r;
+        hit[r] = hit[r] && (kind == kTriNarrow ? edges_at<false>(q, d, c, tri, k, xa, ya + dy, xb, yb + dy, xc, yc + dy)
+                                               : edges_at<true>(q, d, c, tri, k, xa, ya + dy, xb, yb + dy, xc, yc + dy)) >= 0;
+    }
 }
 
 template <uint32_t P>
@@ -213,19 +229,23 @@ __device__ __forceinline__ void take(unsigned long long& best, uint32_t key, uin
     if (packed < best) best = packed;
 }
 
-// The triangles `mask` of the phase (all narrow or all wide) against the
-// lane's pixel (x, y), (lx, ly) in the bin; `best` the nearest (depth key,
-// primitive) so far, `far` the block's farthest key.  `key`: the bound of the
-// lane's own triangle -- as the block closes, the triangles behind `far` are
-// dropped from the mask, which most of a phase's are (1M soup: 73 of 91 a
-// bin).
+// The triangles of the phase (all narrow or all wide) that meet the warp's
+// blocks, meet[r] those of block r, against the lane's pixels (x, y + 4 r),
+// (lx, ly + 4 r) in the bin; best[r] the nearest (depth key, primitive) so
+// far, far[r] the block's farthest key.  `key`: the bound of the
+// lane's own triangle -- as a block closes, the triangles behind its `far` are
+// dropped, which most of a phase's are (1M soup: 73 of 91 a bin).
 // U triangles a turn: a turn is one chain of dependent operations, and two
 // triangles' run side by side where few warps are there to fill the gaps.
-template <int U, bool WIDE, uint32_t P>
-__device__ __forceinline__ void raster_fixed_tris(const PhaseTris<P>& tri, uint32_t k0, uint32_t mask, uint32_t key,
-                                                  int x, int y, int lx, int ly, unsigned long long& best, uint32_t& far) {
+template <int U, bool WIDE, int R, uint32_t P>
+__device__ __forceinline__ void raster_fixed_tris(const PhaseTris<P>& tri, uint32_t k0, const uint32_t (&meet)[R], uint32_t key,
+                                                  int x, int y, int lx, int ly, unsigned long long (&best)[R],
+                                                  uint32_t (&far)[R]) {
+    uint32_t mask = meet[0];
+#pragma unroll
+    for (int r = 1; r < R; ++r) mask |= meet[r];
     while (mask) {   // warp-uniform
-        bool cov[U], some = false;
+        bool cov[U][R], covers[U], some = false;
         uint32_t i[U], prim[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -234,24 +254,40 @@ __device__ __forceinline__ void raster_fixed_tris(const PhaseTris<P>& tri, uint3
             mask &= mask - 1u;
             const uint4 q = tri.a[i[u]], d = tri.b[i[u]], c = tri.c[i[u]];
             prim[u] = q.w;
-            // a stored key below the triangle's bound: no fragment of it can win
-            cov[u] = any && edges_at<WIDE>(q, d, c, tri, i[u], lx, ly, lx, ly, lx, ly) >= 0 && c.z <= (uint32_t)(best >> 32);
-            some |= cov[u];
+            covers[u] = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int yr = ly + kBlockH * r;
+                // a stored key below the triangle's bound: no fragment of it can win
+                cov[u][r] = any && edges_at<WIDE>(q, d, c, tri, i[u], lx, yr, lx, yr, lx, yr) >= 0 &&
+                            c.z <= (uint32_t)(best[r] >> 32);
+                covers[u] |= cov[u][r];
+            }
+            some |= covers[u];
         }
         if (!__any_sync(0xFFFFFFFFu, some)) continue;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (!cov[u]) continue;
+            if (!covers[u]) continue;
             const TriSetup t = load_record(tri, i[u]);
-            float w[3];
-            weights_fixed(t, x, y, w);
-            const float z = interp_z(w[0], w[1], w[2], t.z0, t.z1, t.z2);
-            // the reference rejects z < 0 or z > 1; z == 1 saturates the key to
-            // INT_MAX and can never win the depth test (CUDAROPs.cu:343-345, 386)
-            if (z >= 0.f && z < 1.f) take(best, (uint32_t)__float2int_rz(__fmul_rn(z, 2147483648.0f)), prim[u]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (!cov[u][r]) continue;
+                float w[3];
+                weights_fixed(t, x, y + kBlockH * r, w);
+                const float z = interp_z(w[0], w[1], w[2], t.z0, t.z1, t.z2);
+                // the reference rejects z < 0 or z > 1; z == 1 saturates the key to
+                // INT_MAX and can never win the depth test (CUDAROPs.cu:343-345, 386)
+                if (z >= 0.f && z < 1.f) take(best[r], (uint32_t)__float2int_rz(__fmul_rn(z, 2147483648.0f)), prim[u]);
+            }
         }
-        far = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best >> 32));
-        mask &= __ballot_sync(0xFFFFFFFFu, key <= far);
+        uint32_t keep = 0u;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            far[r] = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best[r] >> 32));
+            keep |= meet[r] & __ballot_sync(0xFFFFFFFFu, key <= far[r]);
+        }
+        mask &= keep;
     }
 }
 
@@ -277,7 +313,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using Shared = BlockShared<THREADS>;
     constexpr uint32_t kWarps = Shared::kWarps, kEntries = Shared::kEntries, kPhase = Shared::kPhase;
-    constexpr int U = THREADS == 512 ? 2 : 1;
+    constexpr int U = THREADS == 512 ? 2 : 1, R = Shared::kPixels;
     Shared& S = *reinterpret_cast<Shared*>(smem_raw);
     unsigned long long* const tile = reinterpret_cast<unsigned long long*>(smem_raw + sizeof(Shared));
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -351,16 +387,19 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
         const uint32_t* const keys = G.keys;
         const uint32_t key_mask = G.key_mask;
         const uint32_t nbw = (uint32_t)(tw + kBlockW - 1) / kBlockW;
-        const uint32_t nblk = nbw * ((uint32_t)(th + kBlockH - 1) / kBlockH);
+        const uint32_t nblk = nbw * ((uint32_t)(th + R * kBlockH - 1) / (R * kBlockH));   // R blocks as one
         const uint32_t inv = kInvBlocks[nbw];
         // a bin of fewer blocks than warps: `groups` warps share a block,
         // taking its triangles in turn and merging in the shared tile
         const uint32_t groups = nblk < kWarps ? kWarps / nblk : 1u, jobs = nblk * groups;
         for (uint32_t blk = warp; blk < nblk; blk += kWarps) {
             const uint32_t by = blk * inv >> 10, bx = blk - by * nbw;
-            // pixels outside the bin: 0, which nothing beats
-            const bool inside = (int)bx * kBlockW + lx < tw && (int)by * kBlockH + ly < th;
-            tile[blk * 32u + lane] = inside ? kEmptyVis : 0ull;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                // pixels outside the bin: 0, which nothing beats
+                const bool inside = (int)bx * kBlockW + lx < tw && (int)by * (R * kBlockH) + kBlockH * r + ly < th;
+                tile[(blk * R + r) * 32u + lane] = inside ? kEmptyVis : 0ull;
+            }
         }
         const bool direct = count <= min(kPhase, pass);   // one phase: nothing to sort
         for (uint32_t b0 = 0; b0 < count; b0 += pass) {
@@ -427,33 +466,54 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
                 for (uint32_t w = warp; w < jobs; w += kWarps) {
                     const uint32_t group = groups > 1u ? w / nblk : 0u, blk = w - group * nblk;
                     const uint32_t brow = blk * inv >> 10;
-                    const int bx = (int)(blk - brow * nbw) * kBlockW, by = (int)brow * kBlockH;
+                    const int bx = (int)(blk - brow * nbw) * kBlockW, by = (int)brow * (R * kBlockH);
                     const int px = bx + lx, py = by + ly;
-                    unsigned long long* const slot = tile + blk * 32u + lane;
-                    unsigned long long best = *(volatile unsigned long long*)slot;
-                    uint32_t far = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best >> 32));
-                    uint32_t limit = total;   // sorted entries from `limit` on lie in buckets behind `far`
+                    unsigned long long* const slot = tile + blk * (R * 32u) + lane;
+                    unsigned long long best[R];
+                    uint32_t far[R];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        best[r] = *(volatile unsigned long long*)(slot + r * 32);
+                        far[r] = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best[r] >> 32));
+                    }
+                    uint32_t limit = total;   // sorted entries from `limit` on lie in buckets behind every block's `far`
                     for (uint32_t c = 0; c < kPhase; c += 32u) {
-                        if (!direct && far < 0x80000000u) limit = S.start[(far >> kSortShift) + 1u];
+                        const uint32_t farthest = R == 1 ? far[0] : max(far[0], far[R - 1]);
+                        if (!direct && farthest < 0x80000000u) limit = S.start[(farthest >> kSortShift) + 1u];
                         if (c >= pn || p0 + c >= limit) break;
-                        uint32_t kind = kTriNarrow, key = 0u;
-                        const bool hit = c + lane < pn && meets_block(S.tri, c + lane, bx, by, far, kind, key);
+                        uint32_t kind = kTriNarrow, key = 0u, meet[R], narrow[R], any = 0u;
+                        bool hit[R] = {};
+                        if (c + lane < pn) meets_blocks<R>(S.tri, c + lane, bx, by, far, kind, key, hit);
                         // a group's share of the chunk, the same whatever its own `far`
-                        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, hit && (groups == 1u || lane % groups == group));
-                        if (!mask) continue;
-                        const uint32_t other = __ballot_sync(0xFFFFFFFFu, kind != kTriNarrow) & mask;
-                        raster_fixed_tris<U, false>(S.tri, c, mask & ~other, key, tx0 + px, ty0 + py, px, py, best, far);
-                        if (other) {
-                            const uint32_t wide = __ballot_sync(0xFFFFFFFFu, kind == kTriWide) & other;
-                            raster_fixed_tris<1, true>(S.tri, c, wide, key, tx0 + px, ty0 + py, px, py, best, far);
-                            if (other != wide)
-                                best = raster_float_tris(S.tri, c, other & ~wide, tx0 + px, ty0 + py, best);
-                            far = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best >> 32));
+                        const bool mine = groups == 1u || lane % groups == group;
+#pragma unroll
+                        for (int r = 0; r < R; ++r) any |= meet[r] = __ballot_sync(0xFFFFFFFFu, hit[r] && mine);
+                        if (!any) continue;
+                        const uint32_t other = __ballot_sync(0xFFFFFFFFu, kind != kTriNarrow);
+#pragma unroll
+                        for (int r = 0; r < R; ++r) narrow[r] = meet[r] & ~other;
+                        raster_fixed_tris<U, false, R>(S.tri, c, narrow, key, tx0 + px, ty0 + py, px, py, best, far);
+                        if (other & any) {
+                            const uint32_t wide = __ballot_sync(0xFFFFFFFFu, kind == kTriWide);
+#pragma unroll
+                            for (int r = 0; r < R; ++r) narrow[r] = meet[r] & wide;
+                            raster_fixed_tris<1, true, R>(S.tri, c, narrow, key, tx0 + px, ty0 + py, px, py, best, far);
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+                                const uint32_t rest = meet[r] & other & ~wide;
+                                if (rest)
+                                    best[r] = raster_float_tris(S.tri, c, rest, tx0 + px, ty0 + py + kBlockH * r, best[r]);
+                                far[r] = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best[r] >> 32));
+                            }
                         }
                     }
-                    if (!direct && far < 0x80000000u) limit = S.start[(far >> kSortShift) + 1u];
-                    if (groups > 1u) atomicMin(slot, best);
-                    else *slot = best;
+                    const uint32_t farthest = R == 1 ? far[0] : max(far[0], far[R - 1]);
+                    if (!direct && farthest < 0x80000000u) limit = S.start[(farthest >> kSortShift) + 1u];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        if (groups > 1u) atomicMin(slot + r * 32, best[r]);
+                        else slot[r * 32] = best[r];
+                    }
                     more |= p0 + kPhase < limit;
                 }
                 // the phase's triangles are done with; on while some block is
@@ -468,12 +528,15 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
         const bool own = nchunks == 1u && !G.direct;
         for (uint32_t blk = warp; blk < nblk; blk += kWarps) {
             const uint32_t by = blk * inv >> 10, bx = blk - by * nbw;
-            const int x = (int)bx * kBlockW + lx, y = (int)by * kBlockH + ly;
-            const unsigned long long best = tile[blk * 32u + lane];
-            if (x >= tw || y >= th || best == kEmptyVis) continue;
-            unsigned long long* g = &G.gvis[(size_t)(ty0 + y) * G.width + (size_t)(tx0 + x)];
-            if (own) *g = best;
-            else atomicMin(g, best);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int x = (int)bx * kBlockW + lx, y = (int)by * (R * kBlockH) + kBlockH * r + ly;
+                const unsigned long long best = tile[(blk * R + r) * 32u + lane];
+                if (x >= tw || y >= th || best == kEmptyVis) continue;
+                unsigned long long* g = &G.gvis[(size_t)(ty0 + y) * G.width + (size_t)(tx0 + x)];
+                if (own) *g = best;
+                else atomicMin(g, best);
+            }
         }
     }
 }
@@ -484,7 +547,8 @@ size_t block_raster_smem(uint32_t bw, uint32_t bh, uint32_t threads) {
     const size_t shared = threads == 128u   ? sizeof(BlockShared<128>)
                           : threads == 256u ? sizeof(BlockShared<256>)
                                             : sizeof(BlockShared<512>);
-    const size_t blocks = (size_t)((bw + kBlockW - 1) / kBlockW) * ((bh + kBlockH - 1) / kBlockH);
+    // an even number of rows: warps of the narrower CTAs own two blocks
+    const size_t blocks = (size_t)((bw + kBlockW - 1) / kBlockW) * (((bh + kBlockH - 1) / kBlockH + 1u) & ~1u);
     return shared + blocks * 32u * sizeof(unsigned long long);
 }
 
