@@ -918,41 +918,44 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
     }
 }
 
-// Shades the thread's two pixels of tile (tx, ty), above row y1: the winners
-// the raster left in the merge buffer (or the clear colour), and leaves the
-// buffer empty for the next frame.  Both merge words are loaded before
-// either pixel is shaded: the pass waits on the chain merge word -> record
-// and vertices (2M soup at 4K: one pixel a thread 96 us, two 92, two with
-// eight blocks an SM 82).
-template <ShadeKind KIND>
-__device__ __forceinline__ void shade_tile(const FrameDev& F, uint32_t tx, uint32_t ty, uint32_t y1,
-                                           const uint32_t* skip = nullptr) {
+// The thread's two pixels of tile (tx, ty): columns by 8 lanes, the second
+// pixel half a tile below the first.
+struct TilePixels {
+    uint32_t x, y;
+    unsigned long long v[2];   // their merge words
+};
+__device__ __forceinline__ TilePixels load_tile(const FrameDev& F, uint32_t tx, uint32_t ty, uint32_t y1) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint32_t x = tx * kTileW + (warp & 3u) * 8u + (lane & 7u);
-    const uint32_t y = ty + (warp >> 2) * 4u + (lane >> 3);
-    if (x >= F.width) return;
-    unsigned long long v[2];
+    TilePixels p;
+    p.x = tx * kTileW + (warp & 3u) * 8u + (lane & 7u);
+    p.y = ty + (warp >> 2) * 4u + (lane >> 3);
 #pragma unroll
     for (uint32_t k = 0; k < 2u; ++k) {
-        const uint32_t yk = y + k * (kTileH / 2u);
-        v[k] = yk < y1 ? F.gvis[(size_t)yk * F.width + x] : kEmptyVis;
+        const uint32_t yk = p.y + k * (kTileH / 2u);
+        p.v[k] = p.x < F.width && yk < y1 ? F.gvis[(size_t)yk * F.width + p.x] : kEmptyVis;
     }
-    if (skip && *skip) {   // a frame that was not rasterised, but for the set-up pass's small triangles
-        for (uint32_t k = 0; k < 2u && F.direct; ++k)
-            if (v[k] != kEmptyVis) F.gvis[(size_t)(y + k * (kTileH / 2u)) * F.width + x] = kEmptyVis;
-        return;
-    }
+    return p;
+}
+
+// Shades a tile's pixels above row y1: the winners the raster left in the
+// merge buffer (or the clear colour), and leaves the buffer empty for the
+// next frame.  Both merge words are loaded before either pixel is shaded: the
+// pass waits on the chain merge word -> record and vertices (2M soup at 4K:
+// one pixel a thread 96 us, two 92, two with eight blocks an SM 82).
+template <ShadeKind KIND>
+__device__ __forceinline__ void shade_tile(const FrameDev& F, const TilePixels& p, uint32_t y1) {
+    if (p.x >= F.width) return;
 #pragma unroll
     for (uint32_t k = 0; k < 2u; ++k) {
-        const uint32_t yk = y + k * (kTileH / 2u);
+        const uint32_t yk = p.y + k * (kTileH / 2u);
         if (yk >= y1) break;
-        const size_t i = (size_t)yk * F.width + x;
-        if (v[k] == kEmptyVis) {
+        const size_t i = (size_t)yk * F.width + p.x;
+        if (p.v[k] == kEmptyVis) {
             clear_pixel(F, i);
             continue;
         }
         F.gvis[i] = kEmptyVis;
-        resolve_pixel<KIND>(F, (int)x, (int)yk, (uint32_t)v[k]);
+        resolve_pixel<KIND>(F, (int)p.x, (int)yk, (uint32_t)p.v[k]);
     }
 }
 
@@ -963,7 +966,13 @@ template <ShadeKind KIND>
 __global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : KIND == kShadeFlat ? 6 : 8) shade_kernel(FrameDev F, uint32_t y0,
                                                                                                       uint32_t y1) {
     pdl_wait();
-    shade_tile<KIND>(F, blockIdx.x, y0 + blockIdx.y * kTileH, y1, &F.ctl->overflow);
+    const TilePixels p = load_tile(F, blockIdx.x, y0 + blockIdx.y * kTileH, y1);
+    if (F.ctl->overflow) {   // a frame that was not rasterised, but for the set-up pass's small triangles
+        for (uint32_t k = 0; k < 2u && F.direct; ++k)
+            if (p.v[k] != kEmptyVis) F.gvis[(size_t)(p.y + k * (kTileH / 2u)) * F.width + p.x] = kEmptyVis;
+        return;
+    }
+    shade_tile<KIND>(F, p, y1);
 }
 
 // Two-pass shading, for frames that shade through the full vertex stage
@@ -1200,26 +1209,42 @@ __global__ void __launch_bounds__(256) batch_fill_kernel(BatchDev B) {
 
 // KIND: every scene of the batch shades flat (B.all_flat), from one mesh, and
 // the kernel holds only that path's registers; kShadeFull: each scene its own
-// way.
+// way.  The flat kinds were bound by L1 (91% busy: the descriptor's fields
+// read from shared memory over and over, spilled registers); with its fields
+// and the next tile's merge words in registers and four blocks an SM that do
+// not spill, a batch frame of 32 uneven soups (26.3M pixels) takes 900 us
+// (957 before; five blocks 904, six 912, without the words ahead 930).
 template <ShadeKind KIND>
-__global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : 6) batch_shade_kernel(BatchDev B, uint32_t chunks, uint32_t per) {
+__global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : 4) batch_shade_kernel(BatchDev B, uint32_t chunks, uint32_t per) {
     if (B.ctl->overflow) return;
     __shared__ __align__(16) FrameDev sF;
     const uint32_t c0 = blockIdx.x * per, c1 = min(c0 + per, chunks);
     uint32_t loaded = 0xFFFFFFFFu, tx = 0, ty = 0;
+    TilePixels p;
+    bool have = false;
     for (uint32_t v = c0; v < c1; ++v) {
         const uint32_t sc = __ldg(B.px_scene + v);
         if (enter_scene(B, sc, loaded, sF)) {
             const uint32_t tile = v - __ldg(B.px_blocks + sc), across = (sF.width + kTileW - 1u) / kTileW;
             ty = tile / across;
             tx = tile - ty * across;
-        } else if (++tx * kTileW >= sF.width) {   // a range's tiles follow one another
+            have = false;
+        }
+        // what the flat path reads of the descriptor, in registers: from
+        // shared memory it is read again after every store
+        const FrameDev F = sF;
+        if (!have) p = load_tile(F, tx, ty * kTileH, F.height);
+        const TilePixels cur = p;
+        if (++tx * kTileW >= F.width) {   // a range's tiles follow one another
             tx = 0;
             ++ty;
         }
-        if (KIND != kShadeFull) shade_tile<KIND>(sF, tx, ty * kTileH, sF.height);
-        else if (sF.flat_shade) shade_tile<kShadeFlat>(sF, tx, ty * kTileH, sF.height);
-        else shade_tile<kShadeFull>(sF, tx, ty * kTileH, sF.height);
+        // the next tile's merge words are on their way while this one is shaded
+        have = KIND != kShadeFull && v + 1u < c1;
+        if (have) p = load_tile(F, tx, ty * kTileH, F.height);
+        if (KIND != kShadeFull) shade_tile<KIND>(F, cur, F.height);
+        else if (sF.flat_shade) shade_tile<kShadeFlat>(sF, cur, sF.height);
+        else shade_tile<kShadeFull>(sF, cur, sF.height);
     }
 }
 
