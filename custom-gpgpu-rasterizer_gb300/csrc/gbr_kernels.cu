@@ -1182,6 +1182,7 @@ __global__ void __launch_bounds__(256) batch_setup_kernel(BatchDev B, uint32_t c
     __shared__ __align__(16) FrameDev sF;
     const uint32_t c0 = blockIdx.x * per, c1 = min(c0 + per, chunks);
     uint32_t loaded = 0xFFFFFFFFu, vis = 0, fp = 0;
+    pdl_wait();
     for (uint32_t v = c0; v < c1; ++v) {
         const uint32_t sc = __ldg(B.tri_scene + v);
         if (sc != loaded && loaded != 0xFFFFFFFFu) {   // the previous scene's statistics
@@ -1195,16 +1196,19 @@ __global__ void __launch_bounds__(256) batch_setup_kernel(BatchDev B, uint32_t c
         fp += c >> 16;
     }
     if (loaded != 0xFFFFFFFFu) add_block_stats(sF.ctl, vis, fp);
+    pdl_release();
 }
 
 // The fill pass keeps one block per chunk (a range loop measured slower
 // here: 489 -> 653 us for the 256-soup batch, more registers per thread).
 __global__ void __launch_bounds__(256) batch_fill_kernel(BatchDev B) {
+    pdl_wait();
     if (B.ctl->overflow) return;
     __shared__ __align__(16) FrameDev sF;
     const uint32_t sc = __ldg(B.tri_scene + blockIdx.x);
     load_scene(B, sc, sF);
     fill_tri<1, false>(sF, (blockIdx.x - __ldg(B.tri_blocks + sc)) * 256u + threadIdx.x, (blockIdx.x * 256u + threadIdx.x) >> 5);
+    pdl_release();
 }
 
 // KIND: every scene of the batch shades flat (B.all_flat), from one mesh, and
@@ -1216,6 +1220,7 @@ __global__ void __launch_bounds__(256) batch_fill_kernel(BatchDev B) {
 // (957 before; five blocks 904, six 912, without the words ahead 930).
 template <ShadeKind KIND>
 __global__ void __launch_bounds__(256, KIND == kShadeFull ? 3 : 4) batch_shade_kernel(BatchDev B, uint32_t chunks, uint32_t per) {
+    pdl_wait();
     if (B.ctl->overflow) return;
     __shared__ __align__(16) FrameDev sF;
     const uint32_t c0 = blockIdx.x * per, c1 = min(c0 + per, chunks);
@@ -1396,18 +1401,21 @@ cudaError_t launch_batch(const BatchDev& B, const BatchLaunch& L, cudaStream_t s
     const uint32_t tri_per = std::max<uint32_t>(1u, (L.tri_blocks + target - 1u) / target);
     const uint32_t px_per = std::max<uint32_t>(1u, (L.px_blocks + target - 1u) / target);
     const uint32_t tri_grid = (L.tri_blocks + tri_per - 1u) / tri_per, px_grid = (L.px_blocks + px_per - 1u) / px_per;
-    if (L.tri_blocks) batch_setup_kernel<<<tri_grid, 256, 0, s>>>(B, L.tri_blocks, tri_per);
-    cudaError_t e = launch_scan(L.scan, s);
+    cudaError_t e = cudaSuccess;
+    if (L.tri_blocks) e = launch_pdl(batch_setup_kernel, dim3(tri_grid), dim3(256), 0, s, B, L.tri_blocks, tri_per);
+    if (e == cudaSuccess) e = launch_scan(L.scan, s);
+    if (e == cudaSuccess && L.tri_blocks) e = launch_pdl(batch_fill_kernel, dim3(L.tri_blocks), dim3(256), 0, s, B);
     if (e != cudaSuccess) return e;
-    if (L.tri_blocks) batch_fill_kernel<<<L.tri_blocks, 256, 0, s>>>(B);
     FrameDev none;
     memset(&none, 0, sizeof none);
     e = launch_block_raster(none, B, true, L.raster_threads, L.raster_ctas, L.bin_w, L.bin_h, L.raster_grid, s);
     if (e != cudaSuccess) return e;
     if (L.px_blocks) {
-        if (B.all_flat == 2u) batch_shade_kernel<kShadeFlatOne><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
-        else if (B.all_flat) batch_shade_kernel<kShadeFlat><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
-        else batch_shade_kernel<kShadeFull><<<px_grid, 256, 0, s>>>(B, L.px_blocks, px_per);
+        e = launch_pdl(B.all_flat == 2u ? batch_shade_kernel<kShadeFlatOne>
+                       : B.all_flat     ? batch_shade_kernel<kShadeFlat>
+                                        : batch_shade_kernel<kShadeFull>,
+                       dim3(px_grid), dim3(256), 0, s, B, L.px_blocks, px_per);
+        if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
