@@ -5,8 +5,8 @@
 // them in phases of 32 triangles (128 in CTAs of 512 threads):
 //   - a thread each, the phase's triangles are loaded, snapped and reduced to
 //     three 32-bit edge values at the bin's first pixel (reduce_triangle);
-//   - each warp owns blocks of 8x4 pixels of the bin, a pixel a lane (in CTAs
-//     of 128 and 256 threads pairs of them, two pixels a lane), whose
+//   - each warp owns blocks of 8x4 pixels of the bin, a pixel a lane (or
+//     pairs of them, two pixels a lane: pixels_per_lane), whose
 //     best (depth key, primitive) it keeps in registers.  It tests 32
 //     triangles at once, a lane each, against the blocks (depth bound, box,
 //     edges), then takes the ones that meet them one after another, every lane
@@ -56,17 +56,12 @@ struct PhaseTris {
 
 // CTAs of 128 or 256 threads fill the SM; those of 512 run frames of few
 // items, whose time is that of their longest one: several warps share a
-// block's triangles and a phase holds more of them.  Two pixels a lane read a
-// triangle and step its edges once for both, and a pair of blocks goes
-// through the tests and the tile's loads once (batch of 32 uneven soups,
-// 32x32 bins: 394M -> 335M instructions, frame 1005 -> 982 us; 2M soup at 4K,
-// 16x16: 449 -> 443; phases of 64: 457).
+// block's triangles and a phase holds more of them.
 template <int THREADS>
 struct BlockShared {
     static constexpr uint32_t kWarps = THREADS / 32u;
     static constexpr uint32_t kEntries = THREADS == 128 ? 1024u : 2048u;   // entries depth-sorted at once
     static constexpr uint32_t kPhase = THREADS == 512 ? 128u : 32u;        // triangles reduced at once
-    static constexpr int kPixels = THREADS == 512 ? 1 : 2;                 // a lane's pixels, blocks below one another
     PhaseTris<kPhase> tri;
     uint32_t sorted[kEntries];              // staged entries, front to back by bucket
     uint32_t hist[2][kSortBuckets];         // entries per bucket; passes alternate, each zeroed after its scan
@@ -308,12 +303,13 @@ __device__ __noinline__ unsigned long long raster_float_tris(const PhaseTris<P>&
 // and its frame descriptor is copied to shared memory when it differs from
 // the previous item's.  MIN_CTAS counts CTAs of 256 threads: twice as many
 // of 128 threads are resident (of 512, two).
-template <int MIN_CTAS, bool BATCH, int THREADS>
+// R: a lane's pixels, its warp's blocks below one another.
+template <int MIN_CTAS, bool BATCH, int THREADS, int R>
 __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 / THREADS)) block_raster_kernel(FrameDev F, BatchDev B) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using Shared = BlockShared<THREADS>;
     constexpr uint32_t kWarps = Shared::kWarps, kEntries = Shared::kEntries, kPhase = Shared::kPhase;
-    constexpr int U = THREADS == 512 ? 2 : 1, R = Shared::kPixels;
+    constexpr int U = THREADS == 512 ? 2 : 1;
     Shared& S = *reinterpret_cast<Shared*>(smem_raw);
     unsigned long long* const tile = reinterpret_cast<unsigned long long*>(smem_raw + sizeof(Shared));
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -547,7 +543,7 @@ size_t block_raster_smem(uint32_t bw, uint32_t bh, uint32_t threads) {
     const size_t shared = threads == 128u   ? sizeof(BlockShared<128>)
                           : threads == 256u ? sizeof(BlockShared<256>)
                                             : sizeof(BlockShared<512>);
-    // an even number of rows: warps of the narrower CTAs own two blocks
+    // an even number of rows, for pairs of blocks
     const size_t blocks = (size_t)((bw + kBlockW - 1) / kBlockW) * (((bh + kBlockH - 1) / kBlockH + 1u) & ~1u);
     return shared + blocks * 32u * sizeof(unsigned long long);
 }
@@ -556,20 +552,36 @@ namespace {
 
 using BlockRaster = void (*)(FrameDev, BatchDev);
 
-template <bool BATCH, int THREADS>
+template <bool BATCH, int THREADS, int R>
 BlockRaster variant(uint32_t ctas) {
     switch (ctas ? ctas : kDefaultBlockCtas) {
-        case 2: return block_raster_kernel<2, BATCH, THREADS>;
-        case 3: return block_raster_kernel<3, BATCH, THREADS>;
-        case 5: return block_raster_kernel<5, BATCH, THREADS>;
-        case 6: return block_raster_kernel<6, BATCH, THREADS>;
-        default: return block_raster_kernel<4, BATCH, THREADS>;
+        case 2: return block_raster_kernel<2, BATCH, THREADS, R>;
+        case 3: return block_raster_kernel<3, BATCH, THREADS, R>;
+        case 5: return block_raster_kernel<5, BATCH, THREADS, R>;
+        case 6: return block_raster_kernel<6, BATCH, THREADS, R>;
+        default: return block_raster_kernel<4, BATCH, THREADS, R>;
     }
 }
 
-BlockRaster variant(bool batch, uint32_t threads, uint32_t ctas) {
-    if (batch) return threads == 128u ? variant<true, 128>(ctas) : variant<true, 256>(ctas);
-    return threads == 128u ? variant<false, 128>(ctas) : block_raster_kernel<2, false, 512>;
+// A lane's pixels: two where a bin has a pair of blocks for every warp (16x16
+// bins and CTAs of 128 threads, say).  They read a triangle and step its edges
+// once for both, and a pair of blocks goes through the tests and the tile's
+// loads once (batch of 32 uneven soups, 32x32 bins: CTAs of 128 394M -> 335M
+// instructions, frame 1005 -> 982 us, CTAs of 256 950 -> 907; 2M soup at 4K,
+// 16x16 bins: 449 -> 443).  In smaller bins the pairs would leave warps to
+// share one (the batch with CTAs of 256: 16x16 bins 1459 -> 1667, 8x8 4206 ->
+// 4753), as in the frames of few items that CTAs of 512 run.
+int pixels_per_lane(uint32_t bw, uint32_t bh, uint32_t threads) {
+    const uint32_t pairs = ((bw + 7u) / 8u) * ((bh + 7u) / 8u);
+    return threads != 512u && pairs >= threads / 32u ? 2 : 1;
+}
+
+BlockRaster variant(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas) {
+    const bool two = pixels_per_lane(bw, bh, threads) == 2;
+    if (batch && threads != 128u) return two ? variant<true, 256, 2>(ctas) : variant<true, 256, 1>(ctas);
+    if (batch) return two ? variant<true, 128, 2>(ctas) : variant<true, 128, 1>(ctas);
+    if (threads != 128u) return block_raster_kernel<2, false, 512, 1>;
+    return two ? variant<false, 128, 2>(ctas) : variant<false, 128, 1>(ctas);
 }
 
 }  // namespace
@@ -577,7 +589,7 @@ BlockRaster variant(bool batch, uint32_t threads, uint32_t ctas) {
 cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas,
                                    int* blocks_per_sm) {
     const size_t smem = block_raster_smem(bw, bh, threads);
-    const BlockRaster k = variant(batch, threads, ctas);
+    const BlockRaster k = variant(bw, bh, batch, threads, ctas);
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, (int)threads, smem);
@@ -585,7 +597,7 @@ cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_
 
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,
                                 uint32_t bw, uint32_t bh, uint32_t grid, cudaStream_t s) {
-    return launch_pdl(variant(batch, threads, ctas), dim3(grid), dim3(threads), block_raster_smem(bw, bh, threads), s, F,
+    return launch_pdl(variant(bw, bh, batch, threads, ctas), dim3(grid), dim3(threads), block_raster_smem(bw, bh, threads), s, F,
                       B);
 }
 
