@@ -66,15 +66,29 @@ __host__ __device__ inline uint32_t count_split_for(unsigned long long pairs, ui
 }
 constexpr uint32_t kDefaultRasterCtas = 6;    // record raster variant (CTAs per SM) used by default
 constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
-// The block raster's CTAs in a single frame: 128 threads where the items
-// outnumber the SMs several times (fewer warps wait at each of an item's
-// barriers than in CTAs of 256: 1M soup 78 us against 88, 2M soup at 4K 201
-// against 285; frames in CTAs of 64: 198 against 176, and 430 against 442),
-// 512 where they don't and the longest item
-// decides.
+// The block raster's CTAs in a single frame of `items` work items and `pairs`
+// entries (0: none seen yet):
+//   512 threads where the items don't outnumber the SMs several times and the
+//       longest one decides;
+//    64 in bins of one or two 8x4-pixel blocks (warps would only share them:
+//       300k soup at 1080p, 8x8 bins, 256 us with CTAs of 128, 191 with 64),
+//       and in bins of at most four pairs of blocks where there are many items
+//       of few entries, which one warp reduces while the others wait (16x16
+//       bins, 128 against 64 threads: 4K, 75 entries an item, 295 and 268 us,
+//       247 entries 362 and 341; 1080p, 99 entries, 99 and 95, 295 entries 115
+//       and 119; 1440p, 278 entries 181 and 186, 1075 entries 299 and 336);
+//   128 otherwise (fewer warps wait at each of an item's barriers than in CTAs
+//       of 256: 1M soup, raster 78 us against 88, 2M soup at 4K 201 against
+//       285).
 constexpr uint32_t kWideItemsPerSm = 6;
-__host__ __device__ inline uint32_t block_threads_for(unsigned long long items, uint32_t sms) {
-    return items < (unsigned long long)kWideItemsPerSm * sms ? 512u : 128u;
+constexpr uint32_t kShortItem = 256, kShortItemsPerSm = 48;
+__host__ __device__ inline uint32_t block_threads_for(unsigned long long items, unsigned long long pairs, uint32_t sms,
+                                                      uint32_t bw, uint32_t bh) {
+    if (items < (unsigned long long)kWideItemsPerSm * sms) return 512u;
+    const uint32_t across = (bw + 7u) / 8u, blocks = across * ((bh + 3u) / 4u), block_pairs = across * ((bh + 7u) / 8u);
+    const bool brief = block_pairs <= 4u && pairs > 0u && pairs <= (unsigned long long)kShortItem * items &&
+                       items >= (unsigned long long)kShortItemsPerSm * sms;
+    return blocks <= 2u || brief ? 64u : 128u;
 }
 // Frames of small triangles (FrameDev::direct): the set-up pass rasterises
 // every triangle whose pixel box holds at most kDirectPixels pixels itself, a
@@ -282,7 +296,7 @@ struct __align__(16) FrameDev {
     uint32_t rec_tma;          // raster: setup records staged by bulk asynchronous copies (1) or loads (0)
     uint32_t direct;           // the set-up pass rasterises small triangles itself (kDirectPixels)
     uint32_t fused_scan;       // the fill pass scans the bins' counts itself (no scan kernel)
-    uint32_t block_threads;    // block raster: threads per CTA, 128 or 512
+    uint32_t block_threads;    // block raster: threads per CTA, 64, 128 or 512
     // two-pass shading of a sparse frame: one byte per bin, "may hold drawn
     // pixels".  dirty_rd: after the last frame; dirty_wr: this frame's, set by
     // the scan for every bin with entries (predicted binning: by the raster for

@@ -1348,9 +1348,9 @@ cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid
     const RecordRaster k = record_variant(ctas);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm->record, k, kRasterThreads, smem);
-    if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, 128u, ctas, &per_sm->block128);
-    if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, 512u, ctas, &per_sm->block512);
-    for (int* n : {&per_sm->record, &per_sm->block128, &per_sm->block512}) *n = std::max(*n, 1);
+    for (uint32_t threads : {64u, 128u, 512u})
+        if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, threads, ctas, &per_sm->block(threads));
+    for (int* n : {&per_sm->record, &per_sm->block64, &per_sm->block128, &per_sm->block512}) *n = std::max(*n, 1);
     return e;
 }
 

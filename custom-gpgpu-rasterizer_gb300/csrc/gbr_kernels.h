@@ -34,14 +34,15 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // bw x bh pixels.  ctas: the variant compiled for 2..6 CTAs per SM (0:
 // default).
 struct RasterGrid {
-    int block128 = 1, block512 = 1;   // block raster, CTAs of 128 and of 512 threads
+    int block64 = 1, block128 = 1, block512 = 1;   // block raster, by threads a CTA
     int record = 1;                   // record raster (small-triangle and bulk-copy variants)
-    int block(uint32_t threads) const { return threads == 128u ? block128 : block512; }
+    int& block(uint32_t threads) { return threads == 64u ? block64 : threads == 128u ? block128 : block512; }
+    int block(uint32_t threads) const { return threads == 64u ? block64 : threads == 128u ? block128 : block512; }
 };
 cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid* per_sm);
 // The block raster (gbr_raster.cu) for a batch frame (B's scenes) or a single
 // frame (F), in CTAs of 128 or 256 threads (a batch) or of
-// 128 or 512 (a frame).
+// 64, 128 or 512 (a frame).
 cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas,
                                    int* blocks_per_sm);
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,

@@ -149,9 +149,9 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
         slot = s;
     }
     // the one raster variant that the frame launches
-    const uint32_t block_threads = block_threads_for(nb, (uint32_t)slot.num_sms);
+    const uint32_t block_threads = block_threads_for(nb, 0u, (uint32_t)slot.num_sms, bin_w, bin_h);
     RasterGrid per_sm;
-    int& ctas = block_threads == 512u ? per_sm.block512 : per_sm.block128;
+    int& ctas = per_sm.block(block_threads);
     e = block_raster_configure(bin_w, bin_h, false, block_threads, 0u, &ctas);
     if (e != cudaSuccess) return na_fail(GBR_ERR_CUDA, cudaGetErrorString(e));
     ctas = std::max(ctas, 1);

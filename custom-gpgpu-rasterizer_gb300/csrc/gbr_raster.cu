@@ -54,13 +54,13 @@ struct PhaseTris {
     uint2 r2[P], h[P];
 };
 
-// CTAs of 128 or 256 threads fill the SM; those of 512 run frames of few
+// CTAs of 64, 128 or 256 threads fill the SM; those of 512 run frames of few
 // items, whose time is that of their longest one: several warps share a
 // block's triangles and a phase holds more of them.
 template <int THREADS>
 struct BlockShared {
     static constexpr uint32_t kWarps = THREADS / 32u;
-    static constexpr uint32_t kEntries = THREADS == 128 ? 1024u : 2048u;   // entries depth-sorted at once
+    static constexpr uint32_t kEntries = THREADS <= 128 ? 8u * THREADS : 2048u;   // entries depth-sorted at once
     static constexpr uint32_t kPhase = THREADS == 512 ? 128u : 32u;        // triangles reduced at once
     PhaseTris<kPhase> tri;
     uint32_t sorted[kEntries];              // staged entries, front to back by bucket
@@ -540,7 +540,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
 }  // namespace
 
 size_t block_raster_smem(uint32_t bw, uint32_t bh, uint32_t threads) {
-    const size_t shared = threads == 128u   ? sizeof(BlockShared<128>)
+    const size_t shared = threads == 64u    ? sizeof(BlockShared<64>)
+                          : threads == 128u ? sizeof(BlockShared<128>)
                           : threads == 256u ? sizeof(BlockShared<256>)
                                             : sizeof(BlockShared<512>);
     // an even number of rows, for pairs of blocks
@@ -580,7 +581,8 @@ BlockRaster variant(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint
     const bool two = pixels_per_lane(bw, bh, threads) == 2;
     if (batch && threads != 128u) return two ? variant<true, 256, 2>(ctas) : variant<true, 256, 1>(ctas);
     if (batch) return two ? variant<true, 128, 2>(ctas) : variant<true, 128, 1>(ctas);
-    if (threads != 128u) return block_raster_kernel<2, false, 512, 1>;
+    if (threads == 512u) return block_raster_kernel<2, false, 512, 1>;
+    if (threads == 64u) return two ? variant<false, 64, 2>(ctas) : variant<false, 64, 1>(ctas);
     return two ? variant<false, 128, 2>(ctas) : variant<false, 128, 1>(ctas);
 }
 

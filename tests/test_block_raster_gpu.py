@@ -60,6 +60,9 @@ def triangles(kind, n, width, height, seed):
     (64, 64, 64, 64, 1025, "inside"),
     (64, 64, 64, 64, 2049, "inside"),      # one entry past a 256-thread CTA's pass
     (33, 17, 66, 34, 5000, "huge"),
+    (8, 8, 640, 480, 3000, "wide"),        # many bins of two blocks: CTAs of 64 threads
+    (16, 16, 1920, 1080, 2500, "wide"),    # many short items: CTAs of 64 threads, two pixels a lane
+    (10, 12, 960, 1080, 2500, "huge"),     # the same, ragged
 ])
 def test_block_raster_against_the_oracle(gbr_lib, cuda_device, bw, bh, w, h, n, kind):
     v = triangles(kind, n, w, h, seed=31)
