@@ -272,7 +272,6 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.chunk = kMaxChunk;
     F.stage = r->chunk;   // queue_chunk: entries per raster pass
     F.phase = r->raster_phase;
-    F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, r->seen_pairs, (uint32_t)r->num_sms, r->bw, r->bh);
     if (r->seen_pairs) {
         if (F.phase == 0u) F.phase = r->seen_pairs < 4u * r->seen_visible ? kSparsePhase : kPhase;
         // small triangles: about (pairs per visible triangle - 1) x the bin
@@ -285,6 +284,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         const uint64_t share = r->seen_pairs / (2u * grid);
         F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), r->rec_tma ? kMinChunk : kMinBlockChunk);
     }
+    F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, r->seen_pairs, (uint32_t)r->num_sms, r->bw, r->bh,
+                                        F.direct != 0u);
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;
     const MeshDev* const only = md.size() == 1u ? md.data() : nullptr;

@@ -68,8 +68,10 @@ constexpr uint32_t kDefaultRasterCtas = 6;    // record raster variant (CTAs per
 constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
 // The block raster's CTAs in a single frame of `items` work items and `pairs`
 // entries (0: none seen yet):
-//   512 threads where the items don't outnumber the SMs several times and the
-//       longest one decides;
+//   512 threads where all the items run at once, two a SM, and the longest
+//       one decides (raster of 34 items of 278 entries: 21 us, with 128 threads
+//       55; 195 items of 366: 12 and 16; but 528 items 18 and 16, 733 items of
+//       32x32 pixels 36 and 25, 855 items of 8x8 18 and 14);
 //    64 in bins of one or two 8x4-pixel blocks (warps would only share them:
 //       300k soup at 1080p, 8x8 bins, 256 us with CTAs of 128, 191 with 64),
 //       and in bins of at most four pairs of blocks where there are many items
@@ -80,11 +82,14 @@ constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
 //   128 otherwise (fewer warps wait at each of an item's barriers than in CTAs
 //       of 256: 1M soup, raster 78 us against 88, 2M soup at 4K 201 against
 //       285).
-constexpr uint32_t kWideItemsPerSm = 6;
+// A frame whose set-up pass draws its small triangles (`direct`) leaves items
+// of an entry or two, and the fewer CTAs count up to three times as many items
+// (1080p icosphere-6, 8x8 bins: 36.2 us, with CTAs of 64 threads 37.4).
+constexpr uint32_t kWideItemsPerSm = 2;
 constexpr uint32_t kShortItem = 256, kShortItemsPerSm = 48;
 __host__ __device__ inline uint32_t block_threads_for(unsigned long long items, unsigned long long pairs, uint32_t sms,
-                                                      uint32_t bw, uint32_t bh) {
-    if (items < (unsigned long long)kWideItemsPerSm * sms) return 512u;
+                                                      uint32_t bw, uint32_t bh, bool direct = false) {
+    if (items <= (unsigned long long)(direct ? 3u : 1u) * kWideItemsPerSm * sms) return 512u;
     const uint32_t across = (bw + 7u) / 8u, blocks = across * ((bh + 3u) / 4u), block_pairs = across * ((bh + 7u) / 8u);
     const bool brief = block_pairs <= 4u && pairs > 0u && pairs <= (unsigned long long)kShortItem * items &&
                        items >= (unsigned long long)kShortItemsPerSm * sms;
