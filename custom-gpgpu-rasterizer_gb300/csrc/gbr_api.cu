@@ -3,8 +3,8 @@
 // Host orchestration of one frame, replacing CUDARenderer::Render's
 // per-mesh loop, its per-256-triangle chunk loop and the device-wide
 // synchronisation after every stage (CustomCUDARasterizer/CUDARenderer.cu:
-// 206-354): a frame is four kernel launches on the caller's stream with no
-// host synchronisation, whatever the number of meshes or triangles.
+// 206-354): a frame is four to seven kernel launches on the caller's stream with
+// no host synchronisation, whatever the number of meshes or triangles.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -355,7 +355,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.fused_scan = !predicted && nb <= kFusedBins && F.count_split == (F.direct ? 2u : 1u) && !F.scan_silent_tile1 && !F.scan_spin_limit &&
                    (F.row_blocks || (F.num_tris > 0u && F.num_tris <= kFusedTris && !touch));
     if (r->timing) GBR_CUDA(cudaEventRecord(r->ev[0], s));
-    if (!F.fused_scan || !r->ctl_clean) GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
+    // (the pre-pass counts into the control block before a fused scan clears it)
+    if (!F.fused_scan || !r->ctl_clean || r->collect) GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
     r->ctl_clean = false;
     if (predicted) {
         // coarse pre-pass -> capacities -> one fused setup + fill pass; the

@@ -9,7 +9,8 @@
 //                  frames): pairs counted per bin in shared memory, one
 //                  global atomic per (block, bin) reserves the block's run.
 //   scan_kernel  : (gbr_scan.cu) bin counts -> list offsets and raster work
-//                  items (bin, chunk of <= queue_chunk ids).
+//                  items (bin, chunk of its ids); frames of at most
+//                  kFusedBins bins do it in the fill pass (fused_scan).
 //   list_touch_kernel: zeros the frame's list entries in whole words so the
 //                  fill's scattered stores merge in L2 (frames of >= 2^20
 //                  pairs).

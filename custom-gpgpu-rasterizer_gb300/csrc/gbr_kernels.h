@@ -35,7 +35,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // default).
 struct RasterGrid {
     int block64 = 1, block128 = 1, block512 = 1;   // block raster, by threads a CTA
-    int record = 1;                   // record raster (small-triangle and bulk-copy variants)
+    int record = 1;                   // record raster (bulk-copy staging)
     int& block(uint32_t threads) { return threads == 64u ? block64 : threads == 128u ? block128 : block512; }
     int block(uint32_t threads) const { return threads == 64u ? block64 : threads == 128u ? block128 : block512; }
 };

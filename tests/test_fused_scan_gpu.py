@@ -2,11 +2,13 @@
 2^16 triangles; the block-row path whatever its bins) and its 32-bin rows:
 bin lists and winners of the frame are the oracle's, frame after frame (the
 raster leaves the counts zero for the next)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import scenes
-from oracle import oracle
+from oracle import mlp_oracle, oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +43,36 @@ def test_fused_scan_against_the_oracle(gbr_lib, cuda_device, w, h, bin_size, n):
             blocks = min((n + 1023) // 1024, torch.cuda.get_device_properties(0).multi_processor_count)
             assert st["num_pairs"] >= s.num_bins_x * s.num_bins_y * blocks
             assert st["count_blocks"] == (blocks if frame and not st["raster_lanes"] else 0)
+
+
+def test_bin_features_after_a_predicted_frame(gbr_lib, cuda_device):
+    """The pre-pass counts its samples into the control block before a fused
+    scan clears it: what a predicted frame left there must not count."""
+    s = scenes.soup_scene(20_000, 640, 480, seed=5)
+    s.bin_w = s.bin_h = 16
+    nb = s.num_bins_x * s.num_bins_y
+    weights = np.zeros(mlp_oracle.NUM_PARAMS, np.float32)
+    weights[mlp_oracle.OFF_B3] = 60.0
+    w16 = mlp_oracle.f32_to_bf16(weights)
+
+    def features(predicted_first):
+        with gbr_lib.Renderer(s.width, s.height) as r:
+            r.load_scene(s)
+            r.render_scene(s)
+            r.stats()
+            if predicted_first:
+                gbr_lib.check(r._lib.gbr_set_predictor(r.h, w16.ctypes.data_as(C.c_void_p), len(w16), C.c_float(0.0),
+                                                       C.c_float(0.0), C.c_float(0.0)))
+                r.set_binning(gbr_lib.BINNING_PREDICTED)
+                r.render_scene(s)
+                r.stats()
+            x, counts = np.zeros((nb, 12), np.float32), np.zeros(nb, np.uint32)
+            cam = gbr_lib.make_camera(s.camera)
+            gbr_lib.check(r._lib.gbr_collect_bin_features(r.h, C.byref(cam), s.cull, s.sample, s.vis,
+                                                          x.ctypes.data_as(C.c_void_p), counts.ctypes.data_as(C.c_void_p), None))
+            return x, counts
+
+    x0, c0 = features(False)
+    x1, c1 = features(True)
+    assert np.array_equal(c0, c1)
+    assert np.array_equal(x0[:, 11], x1[:, 11])   # the samples' density, of a whole number
