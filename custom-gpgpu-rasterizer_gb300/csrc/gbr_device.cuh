@@ -291,7 +291,8 @@ struct __align__(16) FrameDev {
     uint32_t scan_silent_tile1;
     // raster pass size (the reference's queue size, SetupBins'
     // queueMaxSize): a work item's entries are depth-sorted and rasterised
-    // into the tile this many at a time (0 or above kBatch: kBatch)
+    // into the tile this many at a time (0 or above kBatch: kBatch; the block
+    // raster's passes are no shorter than kMinPass)
     uint32_t stage;
     // a frame split across GPUs by bin rows: this frame bins and
     // rasterises bin rows [row0, row1) and shades pixels [px_begin, px_end)

@@ -93,8 +93,9 @@ gbr_status gbr_destroy(gbr_renderer *r);
 /* SetupBins(numBins, binDim, queueMaxSize) (CUDARenderer.cu:199-204).
  * Bins are exact-sized (no capacity, no dropped triangles); queue_chunk
  * keeps the queue size's role in the raster: a bin's triangles are
- * depth-sorted and rasterised into its tile queue_chunk at a time (at most
- * 2048; 0 = 4096, i.e. 2048).  Long bins are split across raster CTAs by the
+ * depth-sorted and rasterised into its tile queue_chunk at a time (between 512
+ * or 1024 and 2048, as the raster's CTAs hold; from 1 with
+ * GBR_STAGING_TMA; 0 = 4096, i.e. 2048).  Long bins are split across raster CTAs by the
  * library, in work items of 64..4096 entries (512..4096 in the block raster)
  * sized from the last frame. */
 gbr_status gbr_setup_bins(gbr_renderer *r, uint32_t num_bins_x, uint32_t num_bins_y,
@@ -298,7 +299,7 @@ gbr_status gbr_get_stats(gbr_renderer *r, gbr_stats *out, void *stream);
 typedef struct gbr_batch gbr_batch;
 typedef struct {
     uint32_t bin_size;     /* bins of bin_size x bin_size pixels, 1..64 */
-    uint32_t queue_chunk;  /* entries depth-sorted and rasterised per pass over a tile, >= 1 (at most 2048
+    uint32_t queue_chunk;  /* entries depth-sorted and rasterised per pass over a tile, >= 1 (1024 to 2048
                               used); work items hold 2048 entries */
     uint32_t raster_ctas;  /* raster variant: CTAs per SM, 2..6 (0: 4), counted in CTAs of 256 threads */
     uint32_t raster_phase; /* 0..128; kept, without effect: a batch's raster refreshes its depth bounds after
