@@ -286,6 +286,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     }
     F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, r->seen_pairs, (uint32_t)r->num_sms, r->bw, r->bh,
                                         F.direct != 0u);
+    if (F.block_threads == 512u && r->seen_pairs && !r->rec_tma) {
+        const uint64_t mean = r->seen_pairs / std::max<uint64_t>(r->seen_items, 1u);
+        if (mean <= kShortMean) F.chunk = (uint32_t)std::max<uint64_t>(2u * mean, kMinChunk);
+    }
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;
     const MeshDev* const only = md.size() == 1u ? md.data() : nullptr;

@@ -52,6 +52,13 @@ constexpr uint32_t kMaxPhase = 128;               // setup records staged per ph
 constexpr uint32_t kSparsePhase = 64;             // the library's phase for frames of small triangles
 constexpr uint32_t kMinChunk = 64;                // smallest raster work item the library picks
 constexpr uint32_t kMinBlockChunk = 512;          // the same for the block raster
+// Frames of few items (CTAs of 512 threads), short ones on average: items of
+// at most twice the mean, so that the few long bins (a sphere's poles) do not
+// decide the frame (640x480 sphere, mean 25 entries: 32.0 -> 29.6 us; sphere
+// of 4262 visible triangles at 1273x536, mean 59: 50.2 -> 37.2).  Where the
+// mean is longer, splitting costs more depth cut than it gains (mean 112
+// entries: items of 128 32 -> 38 us).
+constexpr uint32_t kShortMean = 64;
 constexpr uint32_t kMaxChunk = 4096;              // largest raster work item the library picks
 constexpr uint32_t kBatchChunk = 2048;            // raster work items of a batch frame
 // Exact binning counts each bin in `count_split` sub-counters (at most
@@ -68,10 +75,11 @@ constexpr uint32_t kDefaultRasterCtas = 6;    // record raster variant (CTAs per
 constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
 // The block raster's CTAs in a single frame of `items` work items and `pairs`
 // entries (0: none seen yet):
-//   512 threads where all the items run at once, two a SM, and the longest
+//   512 threads where most of the items run at once, two a SM, and the longest
 //       one decides (raster of 34 items of 278 entries: 21 us, with 128 threads
-//       55; 195 items of 366: 12 and 16; but 528 items 18 and 16, 733 items of
-//       32x32 pixels 36 and 25, 855 items of 8x8 18 and 14);
+//       55; 195 items of 366: 12 and 16; frame of 410 items of 46: 51 and 55;
+//       but raster of 528 items 18 and 16, 733 items of 32x32 pixels 36 and 25,
+//       855 items of 8x8 18 and 14);
 //    64 in bins of one or two 8x4-pixel blocks (warps would only share them:
 //       300k soup at 1080p, 8x8 bins, 256 us with CTAs of 128, 191 with 64),
 //       and in bins of at most four pairs of blocks where there are many items
@@ -83,13 +91,13 @@ constexpr uint32_t kDefaultBlockCtas = 4;     // the block raster's
 //       of 256: 1M soup, raster 78 us against 88, 2M soup at 4K 201 against
 //       285).
 // A frame whose set-up pass draws its small triangles (`direct`) leaves items
-// of an entry or two, and the fewer CTAs count up to three times as many items
+// of an entry or two, and the fewer CTAs count up to twice as many items
 // (1080p icosphere-6, 8x8 bins: 36.2 us, with CTAs of 64 threads 37.4).
-constexpr uint32_t kWideItemsPerSm = 2;
+constexpr uint32_t kWideItemsPerSm = 3;
 constexpr uint32_t kShortItem = 256, kShortItemsPerSm = 48;
 __host__ __device__ inline uint32_t block_threads_for(unsigned long long items, unsigned long long pairs, uint32_t sms,
                                                       uint32_t bw, uint32_t bh, bool direct = false) {
-    if (items <= (unsigned long long)(direct ? 3u : 1u) * kWideItemsPerSm * sms) return 512u;
+    if (items <= (unsigned long long)(direct ? 2u : 1u) * kWideItemsPerSm * sms) return 512u;
     const uint32_t across = (bw + 7u) / 8u, blocks = across * ((bh + 3u) / 4u), block_pairs = across * ((bh + 7u) / 8u);
     const bool brief = block_pairs <= 4u && pairs > 0u && pairs <= (unsigned long long)kShortItem * items &&
                        items >= (unsigned long long)kShortItemsPerSm * sms;

@@ -107,6 +107,33 @@ def test_list_entries_with_and_without_depth(gbr_lib, cuda_device, n):
             assert np.array_equal(r.readback_ids(), o["ids"])
 
 
+@pytest.mark.parametrize("crowd", [10, 65, 129, 1500])
+def test_short_items_beside_a_long_one(gbr_lib, cuda_device, crowd):
+    """A frame of few, short items and one crowded bin: later frames split its
+    list at twice the mean item (no less than 64 entries)."""
+    w, h = 320, 240
+    v = triangles("small", 500 + crowd, w, h, seed=8)
+    p = v["p"].reshape(-1, 3, 3)
+    p[500:, :, :2] = np.array([0.3, -0.2]) + 0.02 * (p[500:, :, :2] - p[500:, :1, :2])   # of a pixel, in one bin
+    v["p"] = p.reshape(-1, 3)
+    s = scenes.Scene("crowd", w, h, 16, 16, scenes.identity_camera(), [scenes.Mesh(vertices=v)], cull=scenes.CULL_NONE)
+    o = oracle.render(s, oracle.RASTER_FIXED)
+    with gbr_lib.Renderer(w, h) as r:
+        r.load_scene(s)
+        for frame in range(3):
+            r.set_raster_params(16, 0)   # a phase below 32: never the small-triangle variant
+            r.render_scene(s)
+            _, depth = r.readback()
+            offsets, bins = r.get_bins()
+            assert np.array_equal(offsets, o["offsets"]) and np.array_equal(bins, o["bins"]), f"frame {frame}: lists"
+            assert np.array_equal(r.readback_ids(), o["ids"]), f"frame {frame}: winners"
+            assert np.array_equal(depth.view(np.uint32), o["depth"].view(np.uint32)), f"frame {frame}: depth"
+            items = r.stats()["num_work_items"]
+            first = items if frame == 0 else first
+            if frame:   # the first frame has no mean to split at
+                assert items == first if crowd == 10 else items >= first + (crowd > 1000) * 10
+
+
 def small_beside_large(w, h, vertex_colours, px=3.5):
     rng = np.random.default_rng(3)
     n = 9000
