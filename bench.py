@@ -504,7 +504,7 @@ def run_ours(args, rank, world, local):
                            "split": ({"bin_rows": list(band), "composite_equals_one_gpu_frame": composite_ok}
                                      if split_rows else "replicas")},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak, "traffic": profile_traffic(), "kernel": "raster_kernel",
+                             "frac": achieved / peak, "traffic": profile_traffic(), "kernel": "block_raster_kernel",
                              "peak_source": peak_kind, "algorithmic_bytes_per_launch": raster_bytes},
                 "e2e": {"value": world * N_TRI / t_e2e, "unit": UNIT, "h2d_bytes_per_step": vbytes,
                         "d2h_bytes_per_step": WIDTH * HEIGHT * 4},
