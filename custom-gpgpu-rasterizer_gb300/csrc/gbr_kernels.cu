@@ -236,9 +236,10 @@ __global__ void __launch_bounds__(256) setup_kernel(FrameDev F, const __grid_con
     // predicted pass stops once an overflow is known; neither runs after a
     // scan of the frame gave up (Ctl::overflow).  An exact frame starts here,
     // with nothing to check
-    if (MODE == 1 || F.exact_guard) {
-        if (F.ctl->overflow) return;
-        if (MODE == 0 ? !F.ctl->pred_overflow : F.ctl->pred_overflow != 0u) return;
+    if (MODE == 1) {   // one answer for the whole block: blocks that run raise pred_overflow
+        if (__syncthreads_or(F.ctl->overflow || F.ctl->pred_overflow)) return;
+    } else if (F.exact_guard) {
+        if (F.ctl->overflow || !F.ctl->pred_overflow) return;
     }
     // a resident grid strides over the triangles, so that a guarded launch
     // that does not run costs one wave of early exits
@@ -493,7 +494,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
     extern __shared__ uint32_t s_row[];
     __shared__ uint32_t s_ovf;
     pdl_wait();
-    if (F.ctl->overflow || F.ctl->pred_overflow) return;   // block-uniform
+    // one answer for the whole block: blocks that run raise pred_overflow, and
+    // a block that started with some of its warps would count with rows that
+    // nobody zeroed and store through them
+    if (__syncthreads_or(F.ctl->overflow || F.ctl->pred_overflow)) return;
     const uint32_t nb = F.num_bins, tid = threadIdx.x;
     for (uint32_t b = tid; b < nb; b += kRowThreads) s_row[b] = 0u;
     if (tid == 0) s_ovf = 0u;
