@@ -417,8 +417,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
 
 // A bounded wait of the bin scan gave up: the frame's kernels after the scan
 // returned without touching the frame buffers.  The scan state restarts
-// from zero.
+// from zero, and so do the bins' counts, which the tiles that started after
+// the flag was raised have left as they were.
 gbr_status scan_timed_out(gbr_renderer* r) {
+    GBR_CUDA(cudaMemset(r->d_counts, 0, (size_t)kCountSplit * r->nbx * r->nby * sizeof(uint32_t)));
     GBR_CUDA(cudaMemset(r->d_scan, 0, scan_state_bytes(r->nbx * r->nby)));
     return fail(GBR_ERR_TIMEOUT, "bin scan wait timed out; the frame is invalid");
 }

@@ -402,6 +402,14 @@ gbr_status render_batch(gbr_batch* b, cudaStream_t s) {
     return GBR_OK;
 }
 
+// A bounded wait of the bin scan gave up: its state and the bins' counts (left
+// by the tiles that started after the flag was raised) restart from zero.
+gbr_status scan_timed_out(gbr_batch* b) {
+    GBR_CUDA(cudaMemset(b->d_counts, 0, (size_t)kCountSplit * b->total_bins * sizeof(uint32_t)));
+    GBR_CUDA(cudaMemset(b->d_scan, 0, scan_state_bytes(b->total_bins)));
+    return fail(GBR_ERR_TIMEOUT, "bin scan wait timed out; the batch frame is invalid");
+}
+
 // Waits for the stream; re-renders with larger bin storage if the batch
 // outgrew it.
 gbr_status finish_batch(gbr_batch* b, cudaStream_t s) {
@@ -409,10 +417,7 @@ gbr_status finish_batch(gbr_batch* b, cudaStream_t s) {
     if (b->frame_checked) return GBR_OK;
     GBR_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));   // pinned: one wait
     GBR_CUDA(cudaStreamSynchronize(s));
-    if (b->h_ctl->error) {   // a bounded wait of the bin scan gave up: restart its state
-        GBR_CUDA(cudaMemset(b->d_scan, 0, scan_state_bytes(b->total_bins)));
-        return fail(GBR_ERR_TIMEOUT, "bin scan wait timed out; the batch frame is invalid");
-    }
+    if (b->h_ctl->error) return scan_timed_out(b);
     for (int attempt = 0; b->h_ctl->overflow && attempt < 3; ++attempt) {
         gbr_status st = ensure_list(b, b->h_ctl->num_pairs, b->h_ctl->items_alloc);
         if (st != GBR_OK) return st;
@@ -430,10 +435,7 @@ gbr_status finish_batch(gbr_batch* b, cudaStream_t s) {
         b->count_split = split;
         drop_graph(b);
     }
-    if (b->h_ctl->error) {   // a bounded wait of the bin scan gave up: restart its state
-        GBR_CUDA(cudaMemset(b->d_scan, 0, scan_state_bytes(b->total_bins)));
-        return fail(GBR_ERR_TIMEOUT, "bin scan wait timed out; the batch frame is invalid");
-    }
+    if (b->h_ctl->error) return scan_timed_out(b);
     b->frame_checked = true;
     return GBR_OK;
 }

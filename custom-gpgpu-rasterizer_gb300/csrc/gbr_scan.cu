@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
 #pragma unroll
             for (uint32_t k = 0; k < (uint32_t)kFeatSlots; ++k) S.feat[k * n + b] = k == 4u ? 0xFFFFFFFFu : 0u;
     }
-    if (!scan_runs(S)) return;
+    // one answer for the whole block: another tile that gives up raises the flag
+    if (!__syncthreads_and(scan_runs(S))) return;
     if (S.mode == kScanPredictedItems) {
         if (S.ctl->pred_overflow) {   // the exact pass that follows counts again
             if (blockIdx.x == 0 && threadIdx.x == 0) { S.ctl->visible = 0u; S.ctl->float_path = 0u; }
