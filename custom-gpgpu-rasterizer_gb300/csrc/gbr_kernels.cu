@@ -1351,7 +1351,8 @@ static RecordRaster record_variant(uint32_t ctas) {
 cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid* per_sm) {
     const size_t smem = record_smem(bw, bh);
     const RecordRaster k = record_variant(ctas);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit of the largest bins, whatever these are (as in block_raster_configure)
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)record_smem(kMaxBinDim, kMaxBinDim));
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm->record, k, kRasterThreads, smem);
     for (uint32_t threads : {64u, 128u, 512u})
         if (e == cudaSuccess) e = block_raster_configure(bw, bh, false, threads, ctas, &per_sm->block(threads));

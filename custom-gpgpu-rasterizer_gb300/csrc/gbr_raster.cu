@@ -597,11 +597,13 @@ BlockRaster variant(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint
 
 cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas,
                                    int* blocks_per_sm) {
-    const size_t smem = block_raster_smem(bw, bh, threads);
     const BlockRaster k = variant(bw, bh, batch, threads, ctas);
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit belongs to the kernel, not to the caller: always that of the
+    // largest bins, so that no other renderer's launches are refused
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)block_raster_smem(kMaxBinDim, kMaxBinDim, threads));
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, (int)threads, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, (int)threads, block_raster_smem(bw, bh, threads));
 }
 
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,
