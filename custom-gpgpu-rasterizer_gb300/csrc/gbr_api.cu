@@ -339,7 +339,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         if (r->d_dirty) {
             uint8_t* rd = r->d_dirty + (size_t)r->dirty_parity * nb;
             uint8_t* wr = r->d_dirty + (size_t)(r->dirty_parity ^ 1u) * nb;
-            if (!r->dirty_valid || r->dirty_vis != vis) GBR_CUDA(cudaMemsetAsync(rd, 1, nb, s));
+            if (!r->dirty_valid || r->broken || r->dirty_vis != vis) GBR_CUDA(cudaMemsetAsync(rd, 1, nb, s));
             F.dirty_rd = rd;
             F.dirty_wr = wr;
             r->dirty_parity ^= 1u;
@@ -359,9 +359,16 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.fused_scan = !predicted && nb <= kFusedBins && F.count_split == (F.direct ? 2u : 1u) && !F.scan_silent_tile1 && !F.scan_spin_limit &&
                    (F.row_blocks || (F.num_tris > 0u && F.num_tris <= kFusedTris && !touch));
     if (r->timing) GBR_CUDA(cudaEventRecord(r->ev[0], s));
+    if (r->broken) {   // launches of the last frame failed: what its passes leave for one another, and for the next frame
+        GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
+        GBR_CUDA(cudaMemsetAsync(r->d_counts, 0, (size_t)kCountSplit * nb * sizeof(uint32_t), s));
+        GBR_CUDA(cudaMemsetAsync(r->d_gvis, 0xFF, (size_t)r->W * r->H * sizeof(unsigned long long), s));
+        GBR_CUDA(cudaMemsetAsync(r->d_feat, 0, (size_t)kFeatSlots * nb * sizeof(uint32_t), s));
+        GBR_CUDA(cudaMemsetAsync(r->d_feat + 4u * nb, 0xFF, nb * sizeof(uint32_t), s));
+    }
+    r->broken = true;
     // (the pre-pass counts into the control block before a fused scan clears it)
-    if (!F.fused_scan || !r->ctl_clean || r->collect) GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
-    r->ctl_clean = false;
+    if (!F.fused_scan || r->collect) GBR_CUDA(cudaMemsetAsync(r->d_ctl, 0, sizeof(Ctl), s));
     if (predicted) {
         // coarse pre-pass -> capacities -> one fused setup + fill pass; the
         // exact kernels behind it only run if a bin overflowed.  The fused
@@ -397,7 +404,6 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     r->last_predicted = predicted;
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[2], s));
     GBR_CUDA(launch_raster(F, r->raster_grid, s));
-    r->ctl_clean = true;
     if (stages) GBR_CUDA(cudaEventRecord(r->ev[4], s));
     ShadeOne one;
     if (only) {
@@ -405,6 +411,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         memcpy(one.lights, r->lights, sizeof one.lights);
     }
     GBR_CUDA(launch_shade(F, only ? &one : nullptr, s));
+    r->broken = false;
     if (r->timing) {
         GBR_CUDA(cudaEventRecord(r->ev[3], s));
         r->ev_recorded = true;

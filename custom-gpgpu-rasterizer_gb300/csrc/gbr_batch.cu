@@ -389,6 +389,8 @@ gbr_status render_batch(gbr_batch* b, cudaStream_t s) {
         st = capture_graph(b);
         if (st != GBR_OK) return st;
     }
+    for (Member& m : b->members)   // a frame of its own that failed half-way may have drawn
+        if (m.r->broken) GBR_CUDA(cudaMemsetAsync(m.r->d_gvis, 0xFF, (size_t)m.r->W * m.r->H * sizeof(unsigned long long), s));
     if (b->timing) GBR_CUDA(cudaEventRecord(b->ev[0], s));
     GBR_CUDA(cudaGraphLaunch(b->graph, s));
     if (b->timing) {

@@ -119,7 +119,7 @@ struct gbr_renderer {
 
     gbr::Ctl* d_ctl = nullptr;
     gbr::Ctl* h_ctl = nullptr;
-    bool ctl_clean = false;   // d_ctl's counters are zero (the last frame's raster was launched)
+    bool broken = false;   // a frame's launches have begun and not all gone out
 
     gbr::LightDev* d_lights = nullptr;   // kMaxLights records
     gbr::LightDev lights[gbr::kMaxLights] = {};   // the same on the host
