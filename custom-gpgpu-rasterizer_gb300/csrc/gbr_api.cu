@@ -284,6 +284,9 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         const uint64_t share = r->seen_pairs / (2u * grid);
         F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), r->rec_tma ? kMinChunk : kMinBlockChunk);
     }
+    // what follows rests on the items that this size gives, which the split
+    // below leaves alone: the same frame is split the same way ever after
+    F.base_chunk = F.chunk;
     F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, r->seen_pairs, (uint32_t)r->num_sms, r->bw, r->bh,
                                         F.direct != 0u);
     if (F.block_threads == 512u && r->seen_pairs && !r->rec_tma) {
@@ -466,7 +469,7 @@ gbr_status finish_frame(gbr_renderer* r, cudaStream_t s, uint32_t* colour = null
     if (r->h_ctl->overflow) return fail(GBR_ERR_OUT_OF_MEMORY, "bin storage overflow persists");
     r->seen_pairs = r->h_ctl->num_pairs;
     r->seen_visible = r->h_ctl->num_visible;
-    r->seen_items = r->h_ctl->num_items;
+    r->seen_items = r->h_ctl->base_items[r->last_predicted && !r->h_ctl->pred_overflow ? 1 : 0];
     // predicted capacities that did not fit the list: grow it for the next
     // frames, within reason (the frame itself was re-binned exactly)
     const uint64_t want = r->h_ctl->pred_capacity;

@@ -271,7 +271,7 @@ void build_table(gbr_batch* b, std::vector<unsigned char>& out) {
         FrameDev F;
         frame_basics(m.r, &m.cam, m.cull, m.sample, m.vis, F);
         F.nbx = L.nbx; F.nby = L.nby; F.bw = b->cfg.bin_size; F.bh = b->cfg.bin_size; F.num_bins = L.nbx * L.nby;
-        F.chunk = kBatchChunk;
+        F.chunk = F.base_chunk = kBatchChunk;
         F.stage = b->cfg.queue_chunk;
         F.phase = b->cfg.raster_phase;
         F.raster_ctas = b->cfg.raster_ctas;
@@ -340,7 +340,7 @@ gbr_status capture_graph(gbr_batch* b) {
     L.scan.list_cap = b->list_cap;
     L.scan.items_cap = b->items_cap;
     L.scan.n = b->total_bins;
-    L.scan.chunk = kBatchChunk;
+    L.scan.chunk = L.scan.base_chunk = kBatchChunk;
     L.scan.mode = kScanExact;
     GBR_CUDA(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = launch_batch(B, L, b->cap_stream);

@@ -53,7 +53,8 @@ constexpr uint32_t kSparsePhase = 64;             // the library's phase for fra
 constexpr uint32_t kMinChunk = 64;                // smallest raster work item the library picks
 constexpr uint32_t kMinBlockChunk = 512;          // the same for the block raster
 // Frames of few items (CTAs of 512 threads), short ones on average: items of
-// at most twice the mean, so that the few long bins (a sphere's poles) do not
+// at most twice the mean (of the items before this split, Ctl::base_items: a
+// mean that the split lowers would change from frame to frame), so that the few long bins (a sphere's poles) do not
 // decide the frame (640x480 sphere, mean 25 entries: 32.0 -> 29.6 us; sphere
 // of 4262 visible triangles at 1273x536, mean 59: 50.2 -> 37.2).  Where the
 // mean is longer, splitting costs more depth cut than it gains (mean 112
@@ -232,7 +233,7 @@ struct Ctl {
     uint32_t rank_next;        // exact binning: rank slots reserved by the count pass
     uint32_t shade_count;      // two-pass shading: covered pixels queued by the light pass
     uint32_t visible, float_path;   // the count pass's running num_visible and num_float_path
-    uint32_t pad[2];
+    uint32_t base_items[2];    // num_items, had the work items held base_chunk entries: of exact lists, of predicted ones
 };
 static_assert(sizeof(Ctl) == 80, "control block is 80 bytes");
 
@@ -242,7 +243,7 @@ struct __align__(16) FrameDev {
     uint32_t nbx, nby, bw, bh, num_bins;
     uint32_t cull, sample, vis, clear_colour32;
     uint32_t num_meshes, num_tris;
-    uint32_t chunk;
+    uint32_t chunk;           // entries of a work item
     uint32_t phase;           // triangles between hierarchical-z refreshes (0: kPhase)
     uint32_t raster_ctas;     // raster_kernel variant: CTAs per SM it is compiled for (0: default)
     float cam_pos[3];
@@ -252,6 +253,8 @@ struct __align__(16) FrameDev {
     uint2* rects;
     uint32_t* keys;            // per triangle: lower bound of its fragments' depth keys (hiz_key), for the fill pass
     uint32_t key_mask;         // bits of the lists' entries that hold the bound's top 8 bits (0: none)
+    uint32_t base_chunk;       // `chunk` before the library's split of few, short items (Ctl::base_items); here, in
+                               // padding: beside `chunk` it moved what follows by 8 bytes, and frames took 0.8% longer
     uint32_t* counts;          // kCountSplit sub-counters per bin: counts[k * count_stride + bin]
     uint32_t* sub_base;        // first list entry of each sub-counter's pairs (same layout)
     uint32_t* offsets;        // num_bins + 1
@@ -369,7 +372,7 @@ struct ScanDev {
     unsigned long long list_cap;
     uint32_t items_cap;
     uint32_t n;
-    uint32_t chunk;
+    uint32_t chunk, base_chunk;    // as FrameDev's
     uint32_t mode;
     uint32_t spin_limit;           // polls of one flag before a look-back wait gives up (0: kScanSpinLimit)
     uint32_t silent_tile1;         // 1 + a tile that publishes nothing (0: none; test hook)

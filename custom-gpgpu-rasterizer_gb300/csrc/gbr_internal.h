@@ -66,8 +66,9 @@ struct gbr_renderer {
     uint32_t rec_tma = 0;             // gbr_set_raster_staging: 1 = bulk asynchronous copies
     uint32_t scan_spin_limit = 0;     // gbr_set_scan_wait (0: the library's bound)
     uint32_t scan_silent_tile1 = 0;   // gbr_set_scan_wait: 1 + the silent tile (0: none)
-    // the last finished frame's pair and visible-triangle counts: they size
-    // the next frames' raster work items and phases (0: none seen yet)
+    // the last finished frame's pairs, visible triangles and work items before
+    // short ones are split (Ctl::base_items): they size the next frames' raster
+    // work items and phases (0: none seen yet)
     uint64_t seen_pairs = 0, seen_visible = 0, seen_items = 0;
 
     // predicted-capacity binning

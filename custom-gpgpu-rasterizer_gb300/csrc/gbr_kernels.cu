@@ -265,10 +265,13 @@ template <uint32_t THREADS, bool DIRECT>
 __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
     constexpr uint32_t kWarps = THREADS / 32u;
     __shared__ unsigned long long s_a[kWarps], s_b[kWarps];
+    __shared__ uint32_t s_base[kWarps];
     const uint32_t nb = F.num_bins, lane = lane_id(), warp = threadIdx.x >> 5, chunk = F.chunk;
     const uint32_t rows = (nb + 31u) / 32u, per = (rows + kWarps - 1u) / kWarps;
     const uint32_t r0 = min(warp * per, rows), r1 = min(r0 + per, rows);
     unsigned long long a = 0, b = 0;   // entries, work items
+    uint32_t base = 0;                 // block 0, where the items are smaller than base_chunk: those of that size
+    const bool split = blockIdx.x == 0 && chunk != F.base_chunk;
 #pragma unroll 4
     for (uint32_t r = r0; r < r1; ++r) {
         const uint32_t i = r * 32u + lane;
@@ -281,7 +284,9 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
         }
         a += (unsigned long long)c + c1;
         b += (c + chunk - 1u) / chunk;
+        if (split) base += (c + F.base_chunk - 1u) / F.base_chunk;
     }
+    if (split) base = __reduce_add_sync(0xFFFFFFFFu, base);
 #pragma unroll
     for (uint32_t d = 16; d > 0; d >>= 1) {
         a += __shfl_xor_sync(0xFFFFFFFFu, a, d);
@@ -290,6 +295,7 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
     if (lane == 0u) {
         s_a[warp] = a;
         s_b[warp] = b;
+        if (split) s_base[warp] = base;
     }
     __syncthreads();
     unsigned long long total = 0, items = 0, at64 = 0, item64 = 0;
@@ -307,6 +313,10 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
         F.ctl->num_pairs = total;
         F.ctl->num_items = fits ? (uint32_t)items : 0u;
         F.ctl->items_alloc = items;
+        base = split ? 0u : (uint32_t)items;
+        for (uint32_t w = 0; w < kWarps && split; ++w) base += s_base[w];
+        F.ctl->base_items[0] = base;
+        F.ctl->base_items[1] = 0u;
         F.ctl->item_next = 0u;
         F.ctl->overflow = fits ? 0u : 1u;
         F.ctl->pred_overflow = F.ctl->error = F.ctl->num_sampled = F.ctl->shade_count = 0u;

@@ -168,7 +168,7 @@ extern "C" gbr_status gbr_render_noalloc(const void* d_vertices, uint32_t num_ve
     F.num_meshes = 1u;
     F.num_tris = (uint32_t)tris;
     F.key_mask = key_mask_for(tris);
-    F.chunk = kMaxChunk;      // work items: the library's split
+    F.chunk = F.base_chunk = kMaxChunk;      // work items: the library's split
     F.fused_scan = tris > 0u ? 1u : 0u;   // the scratch's limits are the fused scan's
     static_assert(kNaMaxBins <= kFusedBins && kNaMaxTris <= kFusedTris, "fused scan limits");
     F.stage = queue_chunk;    // entries per raster pass

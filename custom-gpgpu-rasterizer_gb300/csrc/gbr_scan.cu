@@ -164,7 +164,7 @@ __device__ __forceinline__ void look_back(ScanTile* tiles, uint32_t tile, uint32
 __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) {
     __shared__ unsigned long long s_a[32], s_b[32];
     __shared__ unsigned long long s_excl[2];
-    __shared__ uint32_t s_tile, s_tag;
+    __shared__ uint32_t s_tile, s_tag, s_base;
     pdl_wait();
     if (S.dirty && S.mode == kScanCapacity)   // before any wait: a scan that gives up has still cleared them
         for (uint32_t b = blockIdx.x * 1024u + threadIdx.x; b < S.n; b += gridDim.x * 1024u) S.dirty[b] = 0u;
@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
         if (t == ntiles - 1u) atomicExch(&S.state->ticket, 0u);   // every tile holds its ticket
         if (t >= ntiles) give_up(S.ctl);   // state left by a scan that did not finish
         s_tile = t;
+        s_base = 0u;
     }
     __syncthreads();
     const uint32_t tile = s_tile, tag = s_tag;
@@ -217,6 +218,11 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
         }
         it = bin_items(cr, S.chunk);
     }
+    const bool split = S.chunk != S.base_chunk;   // the frame's items are smaller than base_chunk
+    if (split && S.mode != kScanCapacity) {   // the tile's items of base_chunk entries (added up before the barriers below)
+        const uint32_t base = __reduce_add_sync(0xFFFFFFFFu, bin_items(cr, S.base_chunk));
+        if ((threadIdx.x & 31u) == 0u && base) atomicAdd(&s_base, base);
+    }
     unsigned long long ia = c, ib = it, ta, tb;
     block_scan2(ia, ib, s_a, s_b, ta, tb);
     if (threadIdx.x < 32u) {
@@ -236,6 +242,8 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
     const unsigned long long item = s_excl[1] + ib - it;   // first work item of bin b
     const unsigned long long total = s_excl[0] + ta, total_items = s_excl[1] + tb;
     Ctl* ctl = S.ctl;
+    if (split && threadIdx.x == 0 && S.mode != kScanCapacity)
+        atomicAdd(&ctl->base_items[S.mode == kScanPredictedItems ? 1 : 0], s_base);
     // offsets past the storage are written but never used: the frame is
     // flagged below and the kernels after the scan skip it
     if (b < S.n) {
@@ -273,6 +281,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
         ctl->num_pairs = total;
         ctl->num_items = fits ? (uint32_t)total_items : 0u;
         ctl->items_alloc = total_items;
+        if (!split) ctl->base_items[S.mode == kScanPredictedItems ? 1 : 0] = (uint32_t)total_items;
         ctl->item_next = 0u;
         if (S.mode == kScanPredictedItems) {
             if (!fits) ctl->pred_overflow = 1u;   // the exact kernels that follow take over
@@ -302,6 +311,7 @@ ScanDev scan_of(const FrameDev& F, uint32_t mode) {
     S.items_cap = F.items_cap;
     S.n = F.num_bins;
     S.chunk = F.chunk;
+    S.base_chunk = F.base_chunk;
     S.mode = mode;
     S.spin_limit = F.scan_spin_limit;
     S.silent_tile1 = F.scan_silent_tile1;

@@ -22,24 +22,20 @@ FrameDev g_last;                // the last frame's descriptor
 
 cudaError_t launched() { return g_fail > 0 && --g_fail == 0 ? cudaErrorMemoryAllocation : cudaSuccess; }
 
-uint64_t items_of(uint32_t chunk) {
-    uint64_t n = 0;
-    for (uint32_t c : g_bins) n += (c + chunk - 1u) / chunk;
-    return n;
-}
-
 // the totals of a scan over the counts that the set-up pass left
 void totals(const FrameDev& F) {
-    uint64_t pairs = 0, items = 0;
+    uint64_t pairs = 0, items = 0, base = 0;
     for (uint32_t b = 0; b < F.num_bins; ++b) {
         uint32_t c = 0;
         for (uint32_t k = 0; k < F.count_split; ++k) c += F.counts[k * F.count_stride + b];
         pairs += c;
         items += (c + F.chunk - 1u) / F.chunk;
+        base += (c + F.base_chunk - 1u) / F.base_chunk;
     }
     F.ctl->num_pairs = pairs;
     F.ctl->num_items = (uint32_t)items;
     F.ctl->items_alloc = items;
+    F.ctl->base_items[0] = (uint32_t)base;
     F.ctl->overflow = pairs > F.list_cap;
 }
 }  // namespace
@@ -56,7 +52,6 @@ void host_last_frame(uint32_t out[4]) {
     out[2] = g_last.direct;
     out[3] = g_last.fused_scan;
 }
-uint64_t host_items(uint32_t chunk) { return items_of(chunk); }
 }
 
 namespace gbr {
