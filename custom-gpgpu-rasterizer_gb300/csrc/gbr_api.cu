@@ -263,9 +263,9 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.nbx = r->nbx; F.nby = r->nby; F.bw = r->bw; F.bh = r->bh; F.num_bins = nb;
     // raster work: once a frame has been seen, items hold about half of a
     // raster CTA's share of the pairs (so a few crowded bins do not
-    // serialise the frame), within [kMinBlockChunk, kMaxChunk]; queue_chunk
-    // is the pass size (entries depth-sorted and rasterised at a time).
-    // Bulk-copy staging: at least kMinChunk, and with the library's phase,
+    // serialise the frame), within [kMinBlockChunk, kMaxChunk], or kMinChunk in
+    // frames of few layers; queue_chunk is the pass size (entries depth-sorted
+    // and rasterised at a time).  Bulk-copy staging: at least kMinChunk, and with the library's phase,
     // triangles spanning under 4 bins on average (little overdraw per bin)
     // refresh the tile's depth bound every kSparsePhase triangles rather than
     // every kPhase
@@ -274,12 +274,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.phase = r->raster_phase;
     if (r->seen_pairs) {
         if (F.phase == 0u) F.phase = r->seen_pairs < 4u * r->seen_visible ? kSparsePhase : kPhase;
-        // small triangles: about (pairs per visible triangle - 1) x the bin
-        // side of width + height each
-        if (F.phase >= kDirectPhase && r->seen_visible && !r->rec_tma) {
-            const double extent = ((double)r->seen_pairs / (double)r->seen_visible - 1.0) * 0.5 * (r->bw + r->bh);
-            F.direct = extent < kDirectExtentPx ? 1u : 0u;
-        }
+        if (F.phase >= kDirectPhase && r->seen_visible && !r->rec_tma)
+            F.direct = mean_extent(r->seen_pairs, r->seen_visible, r->bw, r->bh) < kDirectExtentPx ? 1u : 0u;
         const uint64_t grid = (uint64_t)r->num_sms * (uint64_t)(r->rec_tma ? r->raster_grid.record : r->raster_grid.block128 / 2);
         const uint64_t share = r->seen_pairs / (2u * grid);
         F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), r->rec_tma ? kMinChunk : kMinBlockChunk);
@@ -289,9 +285,13 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.base_chunk = F.chunk;
     F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, r->seen_pairs, (uint32_t)r->num_sms, r->bw, r->bh,
                                         F.direct != 0u);
-    if (F.block_threads == 512u && r->seen_pairs && !r->rec_tma) {
-        const uint64_t mean = r->seen_pairs / std::max<uint64_t>(r->seen_items, 1u);
-        if (mean <= kShortMean) F.chunk = (uint32_t)std::max<uint64_t>(2u * mean, kMinChunk);
+    if (r->seen_items && !r->rec_tma) {
+        const double extent = mean_extent(r->seen_pairs, r->seen_visible, r->bw, r->bh);
+        const uint64_t mean = r->seen_pairs / r->seen_items;
+        if (mean_layers(extent, r->seen_visible, std::min<uint64_t>(r->seen_items, nb), r->bw, r->bh) < kFewLayers)
+            F.chunk = kMinChunk;
+        else if (F.block_threads == 512u && mean <= kShortMean)
+            F.chunk = (uint32_t)std::max<uint64_t>(2u * mean, kMinChunk);
     }
     F.raster_ctas = r->raster_ctas;
     F.meshes = r->d_meshes;

@@ -51,15 +51,35 @@ constexpr uint32_t kPhase = 16;                   // triangles between hierarchi
 constexpr uint32_t kMaxPhase = 128;               // setup records staged per phase (the record ring)
 constexpr uint32_t kSparsePhase = 64;             // the library's phase for frames of small triangles
 constexpr uint32_t kMinChunk = 64;                // smallest raster work item the library picks
-constexpr uint32_t kMinBlockChunk = 512;          // the same for the block raster
-// Frames of few items (CTAs of 512 threads), short ones on average: items of
-// at most twice the mean (of the items before this split, Ctl::base_items: a
-// mean that the split lowers would change from frame to frame), so that the few long bins (a sphere's poles) do not
-// decide the frame (640x480 sphere, mean 25 entries: 32.0 -> 29.6 us; sphere
-// of 4262 visible triangles at 1273x536, mean 59: 50.2 -> 37.2).  Where the
-// mean is longer, splitting costs more depth cut than it gains (mean 112
-// entries: items of 128 32 -> 38 us).
+constexpr uint32_t kMinBlockChunk = 512;          // the same for the block raster, but for frames of few layers:
+// Items of kMinChunk entries in frames whose triangles cover the occupied bins
+// fewer than kFewLayers times over (meshes seen from outside).  Little is
+// hidden there, so a long list cut into items loses no depth cut, and left
+// whole it decides the frame (a sphere's poles: 16 spheres of 4096 triangles,
+// 1080p, 32x32 bins, mean 87 entries and longest 453, frame 133.7 -> 87.6 us;
+// 4 of 16384 at 4K, 16x16 bins, 104 -> 85; 9 of 256 at 320x240, 64x64 bins, 84
+// -> 47).  Under many layers whole items close early and cut ones do not (30k
+// soup, 12 layers and more: items of 64 36 -> 68 us at 320x240, 63 -> 112 at
+// 1280x720).  Of 831 frames (meshes and soups, 320x240 to 4K, bins of 8 to 64)
+// items of 64 took 0.5 to 1.06 times as long under 2 layers, 0.8 to 1.3 from 2
+// to 4, 0.9 to 2.9 from 8 on; lines at 2, 3 and 4 layers take all of them to
+// 0.954, 0.951 and 0.952 of the time.
+// Of the others, frames of few items (CTAs of 512 threads), short ones on
+// average (kShortMean, of the items before this split: a mean that the split
+// lowers would change from frame to frame), have items of at most twice the
+// mean, for a few crowded bins among many short ones.
+constexpr double kFewLayers = 3.0;
 constexpr uint32_t kShortMean = 64;
+// From a frame's (triangle, bin) pairs per visible triangle: the extent (width
+// + height, px) of a triangle, and how often triangles half as wide and half as
+// high cover `bins` bins (each rectangle is a pixel wider on all sides).
+inline double mean_extent(unsigned long long pairs, unsigned long long visible, uint32_t bw, uint32_t bh) {
+    return visible ? ((double)pairs / (double)visible - 1.0) * 0.5 * (bw + bh) : 0.0;
+}
+inline double mean_layers(double extent, unsigned long long visible, unsigned long long bins, uint32_t bw, uint32_t bh) {
+    const double side = extent > 4.0 ? 0.5 * (extent - 4.0) : 0.0;
+    return (double)visible * 0.5 * side * side / ((double)(bins ? bins : 1ull) * bw * bh);
+}
 constexpr uint32_t kMaxChunk = 4096;              // largest raster work item the library picks
 constexpr uint32_t kBatchChunk = 2048;            // raster work items of a batch frame
 // Exact binning counts each bin in `count_split` sub-counters (at most
@@ -253,7 +273,7 @@ struct __align__(16) FrameDev {
     uint2* rects;
     uint32_t* keys;            // per triangle: lower bound of its fragments' depth keys (hiz_key), for the fill pass
     uint32_t key_mask;         // bits of the lists' entries that hold the bound's top 8 bits (0: none)
-    uint32_t base_chunk;       // `chunk` before the library's split of few, short items (Ctl::base_items); here, in
+    uint32_t base_chunk;       // `chunk` before the split of frames of few layers (Ctl::base_items); here, in
                                // padding: beside `chunk` it moved what follows by 8 bytes, and frames took 0.8% longer
     uint32_t* counts;          // kCountSplit sub-counters per bin: counts[k * count_stride + bin]
     uint32_t* sub_base;        // first list entry of each sub-counter's pairs (same layout)

@@ -270,8 +270,8 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
     const uint32_t rows = (nb + 31u) / 32u, per = (rows + kWarps - 1u) / kWarps;
     const uint32_t r0 = min(warp * per, rows), r1 = min(r0 + per, rows);
     unsigned long long a = 0, b = 0;   // entries, work items
-    uint32_t base = 0;                 // block 0, where the items are smaller than base_chunk: those of that size
-    const bool split = blockIdx.x == 0 && chunk != F.base_chunk;
+    uint32_t base = 0;                 // the last block, where items are smaller than base_chunk: those of that size
+    const bool split = blockIdx.x == gridDim.x - 1u && chunk != F.base_chunk;
 #pragma unroll 4
     for (uint32_t r = r0; r < r1; ++r) {
         const uint32_t i = r * 32u + lane;
@@ -313,15 +313,16 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
         F.ctl->num_pairs = total;
         F.ctl->num_items = fits ? (uint32_t)items : 0u;
         F.ctl->items_alloc = items;
-        base = split ? 0u : (uint32_t)items;
-        for (uint32_t w = 0; w < kWarps && split; ++w) base += s_base[w];
-        F.ctl->base_items[0] = base;
-        F.ctl->base_items[1] = 0u;
+        if (chunk == F.base_chunk) F.ctl->base_items[0] = (uint32_t)items;
         F.ctl->item_next = 0u;
         F.ctl->overflow = fits ? 0u : 1u;
         F.ctl->pred_overflow = F.ctl->error = F.ctl->num_sampled = F.ctl->shade_count = 0u;
         F.ctl->pred_capacity = 0ull;
         if (fits) F.offsets[nb] = (uint32_t)total;
+    }
+    if (split && threadIdx.x == 0) {
+        for (uint32_t w = 1; w < kWarps; ++w) base += s_base[w];
+        F.ctl->base_items[0] = base;
     }
     if (!fits) return false;
     uint32_t at = (uint32_t)at64, item = (uint32_t)item64;   // the totals fit 32 bits

@@ -1,6 +1,6 @@
 """How a frame's work items follow from the frame before it: the same scene,
 rendered and checked again and again, settles by its third frame on one CTA
-width and one item size, also where splitting the long items takes their number
+width and one item size, also where cutting the long lists takes the items' number
 over the limit (three a SM) by which the width is chosen."""
 import numpy as np
 import pytest
@@ -23,9 +23,10 @@ def uneven_counts(bins, long_items, seed):
 
 @pytest.mark.parametrize("nbx,nby", [(20, 19), (21, 20), (43, 10), (25, 18), (38, 12), (457, 1), (50, 12)])   # 152 SMs: 456 is the limit
 @pytest.mark.parametrize("long_items", [0, 10, 40])
-def test_a_scene_settles(lib, nbx, nby, long_items):
+@pytest.mark.parametrize("pairs_each", [8.0, 2.1])   # triangles that cover their bins 40 times over, and less than 3 times
+def test_a_scene_settles(lib, nbx, nby, long_items, pairs_each):
     bins = uneven_counts(nbx * nby, long_items, seed=nbx)
-    f = Frames(lib, nbx, nby, bins, int(bins.sum()) // 8)
+    f = Frames(lib, nbx, nby, bins, int(bins.sum() / pairs_each))
     seen = []
     for _ in range(10):
         assert f.render() == 0
@@ -34,6 +35,10 @@ def test_a_scene_settles(lib, nbx, nby, long_items):
         seen.append((f.last()["threads"], f.last()["chunk"], st["num_work_items"]))
     assert len(set(seen[2:])) == 1, seen
     assert (seen[-1][0] == 512) == (nbx * nby <= 456)
+    few_layers = bins.sum() / pairs_each * (16 * (pairs_each - 1) - 4) ** 2 / 8 < 3.0 * 256 * len(bins)
+    assert few_layers or pairs_each > 3 or long_items == 40
+    mean = int(bins.sum()) // len(bins)
+    assert seen[-1][1] == (64 if few_layers else max(2 * mean, 64) if seen[-1][0] == 512 and mean <= 64 else 512)
     f.close()
 
 
@@ -74,8 +79,4 @@ def test_a_scene_settles_on_the_gpu(gbr_lib, cuda_device, nbx, nby, route):
             assert st["num_pairs"] == counts.sum() and st["predicted_overflow"] == 0
             items.append(st["num_work_items"])
         assert len(set(items[2:])) == 1, items
-        # twice the mean of the bins' entries, no less than 64: what the split leaves of every bin
-        chunk = max(2 * (int(counts.sum()) // (nbx * nby)), 64)
-        import torch
-        if nbx * nby <= 3 * torch.cuda.get_device_properties(0).multi_processor_count and chunk <= 128:
-            assert items[-1] == (-(-counts // chunk)).sum()
+        assert items[-1] == (-(-counts // 64)).sum()   # a layer of triangles: items of 64 entries
