@@ -325,10 +325,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.exact_guard = predicted ? 1u : 0u;
     // exact binning of a dense frame: block-private counter rows
     const uint32_t rows = std::min<uint32_t>((F.num_tris + kRowThreads - 1u) / kRowThreads, (uint32_t)r->num_sms);
-    if (!predicted && !F.direct && r->d_row_base && use_count_rows(r->seen_pairs, nb, rows)) {
+    if (!predicted && r->d_row_base && use_count_rows(r->seen_pairs, nb, rows, F.direct != 0u)) {
         F.row_base = r->d_row_base;
         F.row_blocks = rows;
-        F.count_split = 1u;
+        F.count_split = F.direct ? 2u : 1u;
     }
     r->last_row_blocks = F.row_blocks;
     r->last_key_mask = F.key_mask;
@@ -558,7 +558,7 @@ gbr_status gbr_setup_bins(gbr_renderer* r, uint32_t num_bins_x, uint32_t num_bin
     GBR_CUDA(cudaMemset(r->d_counts, 0, (size_t)kCountSplit * nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMalloc(&r->d_sub_base, (size_t)kCountSplit * nb * sizeof(uint32_t)));
     if (nb <= kMaxRowBins && r->num_sms > 0)
-        GBR_CUDA(cudaMalloc(&r->d_row_base, (size_t)r->num_sms * nb * sizeof(uint32_t)));
+        GBR_CUDA(cudaMalloc(&r->d_row_base, (size_t)r->num_sms * (2u * nb <= kMaxRowBins ? 2u : 1u) * nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMalloc(&r->d_offsets, (nb + 1u) * sizeof(uint32_t)));
     GBR_CUDA(cudaMemset(r->d_offsets, 0, (nb + 1u) * sizeof(uint32_t)));
     GBR_CUDA(cudaMalloc(&r->d_cursors, nb * sizeof(uint32_t)));

@@ -148,8 +148,16 @@ constexpr double kDirectExtentPx = 16.0;
 // global sub-counters.
 constexpr uint32_t kRowThreads = 1024;
 constexpr uint32_t kMaxRowBins = 32768;
-__host__ __device__ inline bool use_count_rows(unsigned long long pairs, uint32_t bins, uint32_t blocks) {
-    return bins > 0u && bins <= kMaxRowBins && blocks > 0u && pairs >= (unsigned long long)bins * blocks;
+// Frames of small triangles (FrameDev::direct) count entries that the raster
+// need not read in a second row.  From kDirectRowPairs pairs on, block rows are
+// the faster of the two there as well (158 frames, 320x240 to 4K: 0.83 of the
+// time from 2^17 to 2^18 pairs, 0.74 above 2^19, where they are taken; 16
+// spheres of 16384 triangles at 320x240, 64x64 bins, 77.3 -> 43.2 us); below
+// 2^14 they took 1.15 times as long, and between the two 0.81 to 1.12.
+constexpr unsigned long long kDirectRowPairs = 1ull << 16;
+__host__ __device__ inline bool use_count_rows(unsigned long long pairs, uint32_t bins, uint32_t blocks, bool direct) {
+    return bins > 0u && (direct ? 2u : 1u) * bins <= kMaxRowBins && blocks > 0u && pairs >= (unsigned long long)bins * blocks &&
+           (!direct || pairs >= kDirectRowPairs);
 }
 
 // The shade passes' blocks of 256 threads cover tiles of kTileW x kTileH
@@ -311,7 +319,7 @@ struct __align__(16) FrameDev {
     uint32_t count_split;      // sub-counters per bin in use: 1, 2, 4 or 8 (direct: the first half for entries the
                                // raster reads, which come first in the list)
     // exact binning with block-private counter rows (row_blocks > 0)
-    uint32_t* row_base;        // row_blocks x num_bins: a block's first entry in each bin it touched, bin-relative
+    uint32_t* row_base;        // row_blocks x num_bins (direct: x 2): a block's first entry in each bin it touched, bin-relative
     uint32_t row_blocks;       // blocks of the count and fill passes (0: sub-counters)
     uint32_t touch_words;      // block rows: 16-byte words of the list the count pass zeroes (list_touch_kernel)
     uint2* shade_list;         // two-pass shading: covered pixels' indices and winners, width x height slots (null: one pass)
@@ -831,7 +839,9 @@ __device__ __forceinline__ void prefix_2d(uint32_t* row, uint32_t nbx, uint32_t 
 // a round, cost about three times the instructions).  Lanes sit in different
 // rectangles, so their shared-memory cursors rarely meet, and a store goes
 // to a sector of its own either way: 8M of them bound the pass, whose time
-// stayed (50 us).
+// stayed (50 us).  DIRECT: entries that the raster need not read take the
+// second row of cursors.
+template <bool DIRECT>
 __device__ __forceinline__ void fill_walk(const FrameDev& F, uint2 rect, uint32_t entry, uint32_t* cursor) {
     __shared__ uint4 s_tab[kRowThreads / 32u][32];   // the warp's non-empty rectangles: first pair, first bin, w | h << 16, entry
     const uint32_t lane = threadIdx.x & 31u;
@@ -853,7 +863,7 @@ __device__ __forceinline__ void fill_walk(const FrameDev& F, uint2 rect, uint32_
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     if (total == 0u) return;   // warp-uniform
     const uint32_t some = __ballot_sync(0xFFFFFFFFu, n != 0u), rects = (uint32_t)__popc(some);
-    if (n) tab[__popc(some & ((1u << lane) - 1u))] = make_uint4(incl - n, by0 * F.nbx + bx0, w | (h << 16), entry);
+    if (n) tab[__popc(some & ((1u << lane) - 1u))] = make_uint4(incl - n, by0 * F.nbx + bx0 + (DIRECT && (rect.y & 0x80000000u) ? F.num_bins : 0u), w | (h << 16), entry);
     __syncwarp();
     // the lane's run: total / 32 pairs, one more in the first total % 32 lanes
     const uint32_t each = total >> 5, rest = total & 31u;

@@ -92,7 +92,7 @@ struct gbr_renderer {
 
     uint32_t* d_counts = nullptr;     // kCountSplit x bins
     uint32_t* d_sub_base = nullptr;   // kCountSplit x bins
-    uint32_t* d_row_base = nullptr;   // num_sms x bins (block-row exact binning; bins <= kMaxRowBins)
+    uint32_t* d_row_base = nullptr;   // num_sms x bins, x 2 where two rows fit (block-row exact binning)
     uint32_t last_row_blocks = 0;     // blocks of the last frame's block-row count pass (0: sub-counters)
     uint32_t last_key_mask = 0;       // FrameDev::key_mask of the last frame's lists
     uint32_t last_raster_lanes = 0;   // the last frame's set-up pass drew its small triangles

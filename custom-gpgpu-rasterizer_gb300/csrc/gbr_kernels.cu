@@ -123,10 +123,11 @@ __device__ __forceinline__ bool raster_direct(const FrameDev& F, const TriSetup&
 // Returns the warp's visible and float-path triangle counts (bits 0-15 and
 // 16-31), for the block's statistics.
 // `one`: the frame's only mesh (null: looked up).  DIRECT: small triangles
-// are rasterised here (a variant of its own, for the registers).
+// are rasterised here (a variant of its own, for the registers), and MODE 2
+// counts the triangles that the raster need not read in a row of their own.
 template <int MODE, bool DIRECT = false>
 __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, uint32_t walk, const MeshDev* one,
-                                              uint32_t end, uint32_t* s_row = nullptr) {
+                                              uint32_t end, uint32_t* s_row = nullptr, uint32_t* s_skipped = nullptr) {
     const bool in_range = prim < end;
     uint2 rect = empty_rect();
     bool visible = false, fpath = false, skip = true;   // skip: the raster need not read the triangle's entries
@@ -206,7 +207,7 @@ __device__ __forceinline__ uint32_t setup_tri(const FrameDev& F, uint32_t prim, 
     const uint32_t counts = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, visible)) |
                             ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, fpath)) << 16);
     if (MODE == 0) bin_walk<0, DIRECT>(F, rect, 0u, visible, walk);
-    else if (MODE == 2) count_rect(s_row, visible ? rect : empty_rect(), F.nbx, F.nby);
+    else if (MODE == 2) count_rect(DIRECT && skip ? s_skipped : s_row, visible ? rect : empty_rect(), F.nbx, F.nby);
     else bin_walk<2>(F, rect, list_entry(prim, key, skip, F.key_mask), visible, walk);
     return counts;
 }
@@ -434,16 +435,17 @@ __device__ __forceinline__ uint32_t row_share(const FrameDev& F, uint32_t& end) 
     return first;
 }
 
-template <bool ONE>
+// DIRECT: two rows, the second for entries that the raster need not read.
+template <bool ONE, bool DIRECT>
 __global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F, const __grid_constant__ MeshDev one) {
     extern __shared__ uint32_t s_row[];
-    const uint32_t nb = F.num_bins;
-    for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] = 0u;
+    const uint32_t nb = F.num_bins, all = (DIRECT ? 2u : 1u) * nb;
+    for (uint32_t b = threadIdx.x; b < all; b += blockDim.x) s_row[b] = 0u;
     __syncthreads();
     pdl_wait();
     uint32_t vis = 0, fp = 0, end;
     for (uint32_t base = row_share(F, end); base < end; base += kRowThreads) {
-        const uint32_t c = setup_tri<2>(F, base + threadIdx.x, 0u, ONE ? &one : nullptr, end, s_row);
+        const uint32_t c = setup_tri<2, DIRECT>(F, base + threadIdx.x, 0u, ONE ? &one : nullptr, end, s_row, s_row + nb);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -455,8 +457,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F, 
         zero_to[w] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     prefix_2d(s_row, F.nbx, F.nby);
-    uint32_t* const row = F.row_base + (size_t)blockIdx.x * nb;
-    reserve_runs(s_row, nb, F.counts, [&](uint32_t b, uint32_t, uint32_t at) { row[b] = at; });
+    if (DIRECT) prefix_2d(s_row + nb, F.nbx, F.nby);
+    uint32_t* const row = F.row_base + (size_t)blockIdx.x * all;
+    reserve_runs(s_row, all, F.counts, [&](uint32_t b, uint32_t, uint32_t at) { row[b] = at; });
     add_block_stats(F.ctl, vis, fp);
     pdl_release();
 }
@@ -465,17 +468,19 @@ __global__ void __launch_bounds__(kRowThreads, 1) setup_rows_kernel(FrameDev F, 
 // triangles; each bin's cursor starts at the bin's offset plus the block's
 // run start, and every pair takes the next slot with a shared-memory atomic.
 // Cursors of bins the block never touched hold unused values.
+template <bool DIRECT>
 __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
     extern __shared__ uint32_t s_row[];
     pdl_wait();
-    const uint32_t nb = F.num_bins;
-    const uint32_t* const row = F.row_base + (size_t)blockIdx.x * nb;
+    const uint32_t all = (DIRECT ? 2u : 1u) * F.num_bins;
+    const uint32_t* const row = F.row_base + (size_t)blockIdx.x * all;
     if (F.fused_scan) {
-        if (!fused_scan<kRowThreads, false>(F, s_row)) return;
-        for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] += __ldg(row + b);
+        if (!fused_scan<kRowThreads, DIRECT>(F, s_row)) return;
+        for (uint32_t b = threadIdx.x; b < all; b += blockDim.x) s_row[b] += __ldg(row + b);
     } else {
         if (F.ctl->overflow) return;
-        for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) s_row[b] = __ldg(F.offsets + b) + __ldg(row + b);
+        const uint32_t* const from = DIRECT ? F.sub_base : F.offsets;   // with one row a bin's entries start at its offset
+        for (uint32_t b = threadIdx.x; b < all; b += blockDim.x) s_row[b] = __ldg(from + b) + __ldg(row + b);
     }
     __syncthreads();
     uint32_t end;
@@ -483,7 +488,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) fill_rows_kernel(FrameDev F) {
         const uint32_t prim = base + threadIdx.x;
         const bool in_range = prim < end;
         const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-        fill_walk(F, rect, rect_entry(F, prim, rect, in_range), s_row);
+        fill_walk<DIRECT>(F, rect, rect_entry(F, prim, rect, in_range), s_row);
     }
     pdl_release();
 }
@@ -516,7 +521,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
     uint32_t vis = 0, fp = 0, end;
     const uint32_t first = row_share(F, end);
     for (uint32_t base = first; base < end; base += kRowThreads) {
-        const uint32_t c = setup_tri<2, DIRECT>(F, base + tid, 0u, ONE ? &one : nullptr, end, s_row);
+        const uint32_t c = setup_tri<2, DIRECT>(F, base + tid, 0u, ONE ? &one : nullptr, end, s_row, s_row);
         vis += c & 0xFFFFu;
         fp += c >> 16;
     }
@@ -535,7 +540,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) predicted_rows_kernel(FrameDev
             const uint32_t prim = base + tid;
             const bool in_range = prim < end;
             const uint2 rect = in_range ? F.rects[prim] : empty_rect();
-            fill_walk(F, rect, rect_entry(F, prim, rect, in_range), s_row);
+            fill_walk<false>(F, rect, rect_entry(F, prim, rect, in_range), s_row);
         }
     }
     add_block_stats(F.ctl, vis, fp);
@@ -1282,21 +1287,22 @@ static uint32_t triangle_blocks(uint32_t num_tris) {
     return std::min<uint32_t>((num_tris + 255u) / 256u, 8u * (uint32_t)sm_count());
 }
 
-// Dynamic shared memory of the block-row kernels: one counter per bin (the
+// Dynamic shared memory of the block-row kernels: `rows` counters per bin (the
 // opt-in above the default 48 KB is made once per device).
-static cudaError_t row_smem(const FrameDev& F, size_t* bytes) {
+static cudaError_t row_smem(const FrameDev& F, uint32_t rows, size_t* bytes) {
     static uint64_t opted = 0;   // bit d: done on device d (devices 0..63)
-    *bytes = (size_t)F.num_bins * sizeof(uint32_t);
+    *bytes = (size_t)rows * F.num_bins * sizeof(uint32_t);
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const uint64_t bit = dev < 64 ? (1ull << dev) : 0ull;
     if (!(opted & bit)) {
         const int most = (int)(kMaxRowBins * sizeof(uint32_t));
-        e = cudaFuncSetAttribute(fill_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        for (auto* k : {setup_rows_kernel<true>, setup_rows_kernel<false>, predicted_rows_kernel<true, true>,
-                        predicted_rows_kernel<true, false>, predicted_rows_kernel<false, true>,
-                        predicted_rows_kernel<false, false>})
+        e = cudaFuncSetAttribute(fill_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fill_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        for (auto* k : {setup_rows_kernel<true, false>, setup_rows_kernel<false, false>, setup_rows_kernel<true, true>,
+                        setup_rows_kernel<false, true>, predicted_rows_kernel<true, true>, predicted_rows_kernel<true, false>,
+                        predicted_rows_kernel<false, true>, predicted_rows_kernel<false, false>})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
         opted |= bit;
@@ -1308,9 +1314,9 @@ template <bool ONE>
 static cudaError_t launch_setup(const FrameDev& F, const MeshDev& one, bool predicted, cudaStream_t s) {
     if (F.row_blocks) {
         size_t smem = 0;
-        const cudaError_t e = row_smem(F, &smem);
+        const cudaError_t e = row_smem(F, !predicted && F.direct ? 2u : 1u, &smem);
         if (e != cudaSuccess) return e;
-        return launch_pdl(!predicted ? setup_rows_kernel<ONE>
+        return launch_pdl(!predicted ? (F.direct ? setup_rows_kernel<ONE, true> : setup_rows_kernel<ONE, false>)
                           : F.direct ? predicted_rows_kernel<ONE, true>
                                      : predicted_rows_kernel<ONE, false>,
                           dim3(F.row_blocks), dim3(kRowThreads), smem, s, F, one);
@@ -1332,9 +1338,9 @@ cudaError_t launch_setup(const FrameDev& F, const MeshDev* one, bool predicted, 
 cudaError_t launch_fill(const FrameDev& F, cudaStream_t s) {
     if (F.row_blocks) {
         size_t smem = 0;
-        const cudaError_t e = row_smem(F, &smem);
+        const cudaError_t e = row_smem(F, F.direct ? 2u : 1u, &smem);
         if (e != cudaSuccess) return e;
-        return launch_pdl(fill_rows_kernel, dim3(F.row_blocks), dim3(kRowThreads), smem, s, F);
+        return launch_pdl(F.direct ? fill_rows_kernel<true> : fill_rows_kernel<false>, dim3(F.row_blocks), dim3(kRowThreads), smem, s, F);
     }
     const uint32_t blocks = triangle_blocks(F.num_tris);
     if (blocks == 0) return cudaSuccess;
