@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -580,6 +581,10 @@ gbr_status gbr_batch_autotune(gbr_batch* b, const uint32_t* bin_sizes, uint32_t 
     b->timing = true;
     gbr_batch_config winner = base;
     float best_ms = -1.f;
+    // what has been timed, as it runs: bin size, pass, CTAs, threads.  Queue
+    // chunks that give the same pass are one configuration, reported as the
+    // first of them
+    std::vector<std::array<uint32_t, 4>> timed;
     gbr_status st = GBR_OK;
     for (uint32_t bs : bl)
         for (uint32_t ch : cl)
@@ -590,6 +595,12 @@ gbr_status gbr_batch_autotune(gbr_batch* b, const uint32_t* bin_sizes, uint32_t 
                 c.queue_chunk = ch;
                 c.raster_ctas = rc;
                 c.raster_threads = rt;
+                st = check_config(c);
+                if (st != GBR_OK) goto done;
+                const std::array<uint32_t, 4> runs = {bs, block_raster_pass(ch, ::raster_threads(c)), rc ? rc : kDefaultBlockCtas,
+                                                      ::raster_threads(c)};
+                if (std::find(timed.begin(), timed.end(), runs) != timed.end()) continue;
+                timed.push_back(runs);
                 st = gbr_batch_set_config(b, &c);
                 if (st != GBR_OK) goto done;
                 // warm-up frame: sizes the storage (overflow re-render) and captures the graph

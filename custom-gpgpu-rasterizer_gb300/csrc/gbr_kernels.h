@@ -45,6 +45,9 @@ cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid
 // 64, 128 or 512 (a frame).
 cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas,
                                    int* blocks_per_sm);
+// Entries that a pass of such CTAs sorts where a pass size of `stage` is asked
+// for (0: the most).
+uint32_t block_raster_pass(uint32_t stage, uint32_t threads);
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,
                                 uint32_t bw, uint32_t bh, uint32_t grid, cudaStream_t s);
 // one: the mesh of a frame of one mesh (null otherwise)

@@ -43,6 +43,10 @@ __device__ constexpr uint16_t kInvBlocks[9] = {0, 1025, 513, 342, 257, 205, 171,
 // of 128: passes of 32 entries 2916 us a frame, 128 1404, 512 953, 1024 897; 1M
 // soup at 1080p: 64 587, 256 274, 512 212, 1024 179).
 constexpr uint32_t kMinPass = 1024;
+__host__ __device__ constexpr uint32_t pass_of(uint32_t stage, uint32_t entries) {
+    const uint32_t least = kMinPass < entries ? kMinPass : entries;
+    return stage == 0u || stage > entries ? entries : stage < least ? least : stage;
+}
 
 enum : uint32_t { kTriNarrow = 0u, kTriWide = 1u, kTriFloat = 2u };
 
@@ -333,9 +337,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
     }
     if (Q->overflow) return;
     const uint32_t num_items = Q->num_items;
-    const uint32_t stage_req = BATCH ? B.stage : F.stage;
-    // entries per raster pass, at least kMinPass
-    const uint32_t pass = stage_req == 0u ? kEntries : max(min(stage_req, kEntries), min(kMinPass, kEntries));
+    const uint32_t pass = pass_of(BATCH ? B.stage : F.stage, kEntries);
     // the first items are the CTAs' own, the rest are taken in turn.  Thread
     // 0 runs one item ahead: the next item's queue slot is taken when an
     // item starts and its descriptor copied to shared memory meanwhile
@@ -604,6 +606,13 @@ cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_
                                                (int)block_raster_smem(kMaxBinDim, kMaxBinDim, threads));
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, (int)threads, block_raster_smem(bw, bh, threads));
+}
+
+uint32_t block_raster_pass(uint32_t stage, uint32_t threads) {
+    return pass_of(stage, threads == 64u    ? BlockShared<64>::kEntries
+                          : threads == 128u ? BlockShared<128>::kEntries
+                          : threads == 256u ? BlockShared<256>::kEntries
+                                            : BlockShared<512>::kEntries);
 }
 
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,
