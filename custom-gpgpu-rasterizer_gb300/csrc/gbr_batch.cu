@@ -109,7 +109,12 @@ namespace {
 uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1u) / b); }
 
 // raster CTA width of a configuration (0: 256)
-uint32_t raster_threads(const gbr_batch_config& c) { return c.raster_threads == 128u ? 128u : 256u; }
+// Threads of a raster CTA: as configured, but 64 in bins of one or two 8x4-pixel
+// blocks, which more warps would only share (as in block_threads_for).
+uint32_t raster_threads(const gbr_batch_config& c) {
+    if (ceil_div(c.bin_size, 8u) * ceil_div(c.bin_size, 4u) <= 2u) return 64u;
+    return c.raster_threads == 128u ? 128u : 256u;
+}
 
 void drop_graph(gbr_batch* b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);

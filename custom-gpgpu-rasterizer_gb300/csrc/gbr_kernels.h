@@ -41,8 +41,8 @@ struct RasterGrid {
 };
 cudaError_t raster_configure(uint32_t bw, uint32_t bh, uint32_t ctas, RasterGrid* per_sm);
 // The block raster (gbr_raster.cu) for a batch frame (B's scenes) or a single
-// frame (F), in CTAs of 128 or 256 threads (a batch) or of
-// 64, 128 or 512 (a frame).
+// frame (F), in CTAs of 64, 128 or 256 threads (a batch) or of 64, 128 or 512
+// (a frame).
 cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas,
                                    int* blocks_per_sm);
 // Entries that a pass of such CTAs sorts where a pass size of `stage` is asked

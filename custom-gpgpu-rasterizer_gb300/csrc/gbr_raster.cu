@@ -588,6 +588,7 @@ int pixels_per_lane(uint32_t bw, uint32_t bh, uint32_t threads) {
 
 BlockRaster variant(uint32_t bw, uint32_t bh, bool batch, uint32_t threads, uint32_t ctas) {
     const bool two = pixels_per_lane(bw, bh, threads) == 2;
+    if (batch && threads == 64u) return variant<true, 64, 1>(ctas);   // bins of one or two blocks
     if (batch && threads != 128u) return two ? variant<true, 256, 2>(ctas) : variant<true, 256, 1>(ctas);
     if (batch) return two ? variant<true, 128, 2>(ctas) : variant<true, 128, 1>(ctas);
     if (threads == 512u) return block_raster_kernel<2, false, 512, 1>;
