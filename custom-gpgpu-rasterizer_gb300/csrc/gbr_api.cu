@@ -272,10 +272,10 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.chunk = kMaxChunk;
     F.stage = r->chunk;   // queue_chunk: entries per raster pass
     F.phase = r->raster_phase;
+    const double extent = mean_extent(r->seen_pairs, r->seen_visible, r->bw, r->bh);
     if (r->seen_pairs) {
         if (F.phase == 0u) F.phase = r->seen_pairs < 4u * r->seen_visible ? kSparsePhase : kPhase;
-        if (F.phase >= kDirectPhase && r->seen_visible && !r->rec_tma)
-            F.direct = mean_extent(r->seen_pairs, r->seen_visible, r->bw, r->bh) < kDirectExtentPx ? 1u : 0u;
+        if (F.phase >= kDirectPhase && r->seen_visible && !r->rec_tma) F.direct = extent < kDirectExtentPx ? 1u : 0u;
         const uint64_t grid = (uint64_t)r->num_sms * (uint64_t)(r->rec_tma ? r->raster_grid.record : r->raster_grid.block128 / 2);
         const uint64_t share = r->seen_pairs / (2u * grid);
         F.chunk = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(share, kMaxChunk), r->rec_tma ? kMinChunk : kMinBlockChunk);
@@ -285,8 +285,7 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
     F.base_chunk = F.chunk;
     F.block_threads = block_threads_for(r->seen_pairs ? r->seen_items : nb, r->seen_pairs, (uint32_t)r->num_sms, r->bw, r->bh,
                                         F.direct != 0u);
-    if (r->seen_items && !r->rec_tma) {
-        const double extent = mean_extent(r->seen_pairs, r->seen_visible, r->bw, r->bh);
+    if (r->seen_items && !r->rec_tma && !(predicted && F.direct && extent < kDrawnExtentPx)) {
         const uint64_t mean = r->seen_pairs / r->seen_items;
         if (mean_layers(extent, r->seen_visible, std::min<uint64_t>(r->seen_items, nb), r->bw, r->bh) < kFewLayers)
             F.chunk = kMinChunk;

@@ -69,6 +69,7 @@ struct gbr_batch {
     uint32_t* d_counts = nullptr;     // kCountSplit x bins
     uint32_t* d_sub_base = nullptr;   // kCountSplit x bins
     uint32_t count_split = 1;         // sub-counters per bin in use
+    uint32_t chunk = kBatchChunk;     // entries of a work item
     uint32_t all_flat = 0;            // BatchDev::all_flat (the captured shade variant)
     uint32_t* d_offsets = nullptr;
     uint32_t* d_cursors = nullptr;
@@ -138,7 +139,7 @@ gbr_status ensure_list(gbr_batch* b, uint64_t pairs, uint64_t items) {
     uint64_t cap = std::max<uint64_t>(std::max<uint64_t>(pairs + pairs / 4u, b->list_cap), 1u << 20);
     if (cap > 0x7FFFFFFFull) cap = 0x7FFFFFFFull;
     if (pairs > cap) return fail(GBR_ERR_OUT_OF_MEMORY, "batch needs %llu bin entries (max 2^31-1)", (unsigned long long)pairs);
-    uint64_t icap = std::max<uint64_t>(items + items / 4u, (uint64_t)b->total_bins + cap / kBatchChunk + 1u);
+    uint64_t icap = std::max<uint64_t>(items + items / 4u, (uint64_t)b->total_bins + cap / kMinChunk + 1u);
     icap = std::max<uint64_t>(icap, b->items_cap);
     if (icap > 0xFFFFFFFFull) icap = 0xFFFFFFFFull;
     drop_graph(b);
@@ -346,7 +347,8 @@ gbr_status capture_graph(gbr_batch* b) {
     L.scan.list_cap = b->list_cap;
     L.scan.items_cap = b->items_cap;
     L.scan.n = b->total_bins;
-    L.scan.chunk = L.scan.base_chunk = kBatchChunk;
+    L.scan.chunk = b->chunk;
+    L.scan.base_chunk = kBatchChunk;
     L.scan.mode = kScanExact;
     GBR_CUDA(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = launch_batch(B, L, b->cap_stream);
@@ -436,11 +438,17 @@ gbr_status finish_batch(gbr_batch* b, cudaStream_t s) {
         GBR_CUDA(cudaStreamSynchronize(s));
     }
     if (b->h_ctl->overflow) return fail(GBR_ERR_OUT_OF_MEMORY, "batch bin storage overflow persists");
-    // sub-counters per bin for the next frames, from this frame's density
-    // (a change is captured anew: the scan's parameters live in the graph)
-    const uint32_t split = count_split_for(b->h_ctl->num_pairs, b->total_bins);
-    if (split != b->count_split) {
+    // sub-counters per bin and the items' size for the next frames, from this
+    // frame's density and layers (a change is captured anew: the scan's
+    // parameters live in the graph)
+    const uint32_t split = count_split_for(b->h_ctl->num_pairs, b->total_bins), bs = b->cfg.bin_size;
+    const uint64_t pairs = b->h_ctl->num_pairs, visible = b->h_ctl->num_visible;
+    const double layers = mean_layers(mean_extent(pairs, visible, bs, bs), visible,
+                                      std::min(b->h_ctl->base_items[0], b->total_bins), bs, bs);
+    const uint32_t chunk = layers < kFewLayers ? kMinChunk : kBatchChunk;
+    if (split != b->count_split || chunk != b->chunk) {
         b->count_split = split;
+        b->chunk = chunk;
         drop_graph(b);
     }
     if (b->h_ctl->error) return scan_timed_out(b);

@@ -139,6 +139,13 @@ __host__ __device__ inline uint32_t block_threads_for(unsigned long long items, 
 constexpr uint32_t kDirectPhase = 32;
 constexpr int kDirectPixels = 16;
 constexpr double kDirectExtentPx = 16.0;
+// Predicted lists hold the drawn triangles among the others.  Below this
+// estimate (rectangles a pixel wider on all sides; boxes of kDirectPixels
+// pixels) most are drawn, and cutting their lists (kFewLayers) costs a tile an
+// item for nothing (16 spheres of 16384 triangles, 64x64 bins: 640x480, 7.7
+// px, 148 us cut and 89 whole; 1280x720, 8.2 px, 146 and 89; at 1080p, 10.3 px,
+// 174 and 165; 4 spheres of 4096 at 1280x720, above 12 px, 74 and 118).
+constexpr double kDrawnExtentPx = 12.0;
 // Exact binning with block-private counter rows: one block of kRowThreads
 // per SM counts its pairs per bin in shared memory (num_bins <=
 // kMaxRowBins), then takes its run of every bin it touched with one global

@@ -43,10 +43,6 @@ __device__ constexpr uint16_t kInvBlocks[9] = {0, 1025, 513, 342, 257, 205, 171,
 // of 128: passes of 32 entries 2916 us a frame, 128 1404, 512 953, 1024 897; 1M
 // soup at 1080p: 64 587, 256 274, 512 212, 1024 179).
 constexpr uint32_t kMinPass = 1024;
-__host__ __device__ constexpr uint32_t pass_of(uint32_t stage, uint32_t entries) {
-    const uint32_t least = kMinPass < entries ? kMinPass : entries;
-    return stage == 0u || stage > entries ? entries : stage < least ? least : stage;
-}
 
 enum : uint32_t { kTriNarrow = 0u, kTriWide = 1u, kTriFloat = 2u };
 
@@ -332,12 +328,16 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
         zero_counts(F);
         if (blockIdx.x == 0u && tid == 0u) close_counters(Q);
     } else {
-        for (uint32_t i = blockIdx.x * THREADS + tid; i < B.num_scenes; i += gridDim.x * THREADS)
+        for (uint32_t i = blockIdx.x * THREADS + tid; i < B.num_scenes; i += gridDim.x * THREADS) {
             close_counters(B.scenes[i].ctl);
+            atomicAdd(&Q->num_visible, B.scenes[i].ctl->num_visible);
+        }
     }
     if (Q->overflow) return;
     const uint32_t num_items = Q->num_items;
-    const uint32_t pass = pass_of(BATCH ? B.stage : F.stage, kEntries);
+    const uint32_t stage_req = BATCH ? B.stage : F.stage;
+    // entries per raster pass, at least kMinPass
+    const uint32_t pass = stage_req == 0u ? kEntries : max(min(stage_req, kEntries), min(kMinPass, kEntries));
     // the first items are the CTAs' own, the rest are taken in turn.  Thread
     // 0 runs one item ahead: the next item's queue slot is taken when an
     // item starts and its descriptor copied to shared memory meanwhile
@@ -609,11 +609,14 @@ cudaError_t block_raster_configure(uint32_t bw, uint32_t bh, bool batch, uint32_
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, (int)threads, block_raster_smem(bw, bh, threads));
 }
 
+// As the kernel reckons it (which calls no function for it: frames took 0.7%
+// longer).
 uint32_t block_raster_pass(uint32_t stage, uint32_t threads) {
-    return pass_of(stage, threads == 64u    ? BlockShared<64>::kEntries
-                          : threads == 128u ? BlockShared<128>::kEntries
-                          : threads == 256u ? BlockShared<256>::kEntries
-                                            : BlockShared<512>::kEntries);
+    const uint32_t entries = threads == 64u    ? BlockShared<64>::kEntries
+                             : threads == 128u ? BlockShared<128>::kEntries
+                             : threads == 256u ? BlockShared<256>::kEntries
+                                               : BlockShared<512>::kEntries;
+    return stage == 0u ? entries : std::max(std::min(stage, entries), std::min(kMinPass, entries));
 }
 
 cudaError_t launch_block_raster(const FrameDev& F, const BatchDev& B, bool batch, uint32_t threads, uint32_t ctas,

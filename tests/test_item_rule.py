@@ -80,3 +80,37 @@ def test_a_scene_settles_on_the_gpu(gbr_lib, cuda_device, nbx, nby, route):
             items.append(st["num_work_items"])
         assert len(set(items[2:])) == 1, items
         assert items[-1] == (-(-counts // 64)).sum()   # a layer of triangles: items of 64 entries
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bin_size", [16, 64])
+def test_batches_of_few_layers_cut_their_lists(gbr_lib, cuda_device, bin_size):
+    """Spheres cover their bins once or twice: items of 64 entries from the
+    second frame on.  Soups cover them many times: items of 2048."""
+    for make, chunk in ((lambda k: scenes.sphere_scene(320, 240, lon=64, lat=32 + k), 64),
+                        (lambda k: scenes.soup_scene(20_000, 320, 240, seed=k), 2048)):
+        sl = [make(k) for k in range(3)]
+        with gbr_lib.Batch() as b:
+            rs = []
+            for s in sl:
+                r = gbr_lib.Renderer(s.width, s.height)
+                r.load_scene(s)
+                b.add_scene(r, s)
+                rs.append(r)
+            b.set_config(bin_size, 4096)
+            first = None
+            for frame in range(4):
+                b.render()
+                counts = np.concatenate([np.diff(b.get_bins(i)[0].astype(np.int64)) for i in range(len(sl))])
+                now = [b.readback(i)[2] for i in range(len(sl))]
+                first = first or now
+                assert all(np.array_equal(x, y) for x, y in zip(first, now))
+                st = b.stats()
+                assert st["num_work_items"] == (-(-counts // (chunk if frame else 2048))).sum()
+            assert b.stats()["graph_captures"] <= 2
+            b.close()
+            for i, r in enumerate(rs):
+                r.load_scene(sl[i])
+                r.render_scene(sl[i])
+                assert np.array_equal(r.readback_ids(), first[i])
+                r.close()
