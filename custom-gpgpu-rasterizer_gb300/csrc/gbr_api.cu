@@ -339,12 +339,8 @@ gbr_status render_frame(gbr_renderer* r, const gbr_camera* cam, uint32_t cull, u
         F.shade_list = r->d_shade_list;
         // the light pass leaves bins that stay clean untouched
         if (r->d_dirty) {
-            uint8_t* rd = r->d_dirty + (size_t)r->dirty_parity * nb;
-            uint8_t* wr = r->d_dirty + (size_t)(r->dirty_parity ^ 1u) * nb;
-            if (!r->dirty_valid || r->broken || r->dirty_vis != vis) GBR_CUDA(cudaMemsetAsync(rd, 1, nb, s));
-            F.dirty_rd = rd;
-            F.dirty_wr = wr;
-            r->dirty_parity ^= 1u;
+            F.dirty = r->d_dirty;
+            if (!r->dirty_valid || r->broken || r->dirty_vis != vis) GBR_CUDA(cudaMemsetAsync(r->d_dirty, kDirtyNow, nb, s));
             r->dirty_valid = true;
             r->dirty_vis = vis;
         }
@@ -564,7 +560,7 @@ gbr_status gbr_setup_bins(gbr_renderer* r, uint32_t num_bins_x, uint32_t num_bin
     GBR_CUDA(cudaMalloc(&r->d_capacity, nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMemset(r->d_capacity, 0, nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMalloc(&r->d_bin_end, nb * sizeof(uint32_t)));
-    GBR_CUDA(cudaMalloc(&r->d_dirty, 2u * (size_t)nb));
+    GBR_CUDA(cudaMalloc(&r->d_dirty, nb));
     GBR_CUDA(cudaMalloc(&r->d_scan, scan_state_bytes(nb)));
     GBR_CUDA(cudaMemset(r->d_scan, 0, scan_state_bytes(nb)));
     GBR_CUDA(cudaMemset(r->d_bin_end, 0, nb * sizeof(uint32_t)));

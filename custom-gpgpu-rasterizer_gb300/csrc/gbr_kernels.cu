@@ -281,7 +281,7 @@ __device__ __forceinline__ bool fused_scan(const FrameDev& F, uint32_t* s_off) {
         if (i < nb) {
             s_off[i] = c;
             if (DIRECT) s_off[nb + i] = c1;
-            if (F.dirty_wr && r % gridDim.x == blockIdx.x) F.dirty_wr[i] = c + c1 ? 1u : 0u;
+            if (F.dirty && r % gridDim.x == blockIdx.x) F.dirty[i] = next_dirty(F.dirty[i], c + c1 != 0u);
         }
         a += (unsigned long long)c + c1;
         b += (c + chunk - 1u) / chunk;
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
         __syncthreads();
         const uint32_t bin = S.item[0];
         if (bin == 0xFFFFFFFFu) break;
-        if (tid == 0 && F.dirty_wr) F.dirty_wr[bin] = 1u;   // the bin's pixels may now be drawn
+        if (tid == 0 && F.dirty) F.dirty[bin] |= kDirtyNow;   // the bin's pixels may now be drawn
         const uint32_t start = S.item[1], count = S.item[2], nchunks = S.item[3];
         const int tx0 = (int)((bin % F.nbx) * F.bw), ty0 = (int)((bin / F.nbx) * F.bh);
         const int tw = min((int)F.bw, (int)F.width - tx0), th = min((int)F.bh, (int)F.height - ty0);
@@ -1016,9 +1016,9 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
     if (F.ctl->overflow) {
         // not rasterised: the buffers keep the last frame's pixels, and the
         // next frame must find those bins as they were
-        if (F.dirty_rd)
+        if (F.dirty)
             for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < F.num_bins; b += gridDim.x * blockDim.x)
-                F.dirty_wr[b] |= F.dirty_rd[b];
+                if (F.dirty[b]) F.dirty[b] |= kDirtyNow;
         // what the set-up pass has drawn goes
         if (F.direct)
             for (uint32_t i = F.px_begin + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
     // drawn in this one already holds the clear values (pixels outside the
     // bin grid are always written)
     bool live = i0 < n;
-    if (F.dirty_rd) {
+    if (F.dirty) {
         // the quad's row and column: one division per warp (its 32 quads
         // are consecutive), then at most one row wrap per lane on frames at
         // least 128 pixels wide
@@ -1059,14 +1059,14 @@ __global__ void __launch_bounds__(256) shade_queue_kernel(FrameDev F) {
             const uint32_t bx0 = p2 ? x >> sx : x / F.bw, bx1 = p2 ? (x + 3u) >> sx : (x + 3u) / F.bw;
             live = by >= F.nby || bx1 >= F.nbx;
             for (uint32_t bx = bx0; !live && bx <= bx1; ++bx)
-                live = (F.dirty_rd[by * F.nbx + bx] | F.dirty_wr[by * F.nbx + bx]) != 0u;
+                live = F.dirty[by * F.nbx + bx] != 0u;
         } else {   // a quad that wraps a row, or the frame's last pixels
             live = false;
             const uint32_t last = min(i0 + 3u, n - 1u);
             for (uint32_t i = i0; i <= last; ++i) {
                 const uint32_t yi = i / F.width, xi = i - yi * F.width;
                 const uint32_t bx = xi / F.bw, by = yi / F.bh;
-                live |= bx >= F.nbx || by >= F.nby || (F.dirty_rd[by * F.nbx + bx] | F.dirty_wr[by * F.nbx + bx]) != 0u;
+                live |= bx >= F.nbx || by >= F.nby || F.dirty[by * F.nbx + bx] != 0u;
             }
         }
         if (!__any_sync(0xFFFFFFFFu, live)) return;   // the warp's 128 pixels already hold the clear values

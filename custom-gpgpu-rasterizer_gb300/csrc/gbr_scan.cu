@@ -166,8 +166,9 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
     __shared__ unsigned long long s_excl[2];
     __shared__ uint32_t s_tile, s_tag, s_base;
     pdl_wait();
-    if (S.dirty && S.mode == kScanCapacity)   // before any wait: a scan that gives up has still cleared them
-        for (uint32_t b = blockIdx.x * 1024u + threadIdx.x; b < S.n; b += gridDim.x * 1024u) S.dirty[b] = 0u;
+    if (S.dirty && S.mode == kScanCapacity)   // before any wait: a scan that gives up has still handed them on
+        for (uint32_t b = blockIdx.x * 1024u + threadIdx.x; b < S.n; b += gridDim.x * 1024u)
+            S.dirty[b] = next_dirty(S.dirty[b], false);
     if (S.mode == kScanPredictedItems && S.feat) {
         // the pre-pass accumulators start the next frame empty (also when
         // this frame was flagged)
@@ -212,7 +213,10 @@ __global__ void __launch_bounds__(1024) scan_kernel(ScanDev S, uint32_t ntiles) 
                     if (k < S.raster_split) cr += sub[k];
                 }
             }
-            if (S.dirty) S.dirty[b] = c ? 1u : 0u;
+            if (S.dirty) {   // (behind a predicted pass they have been handed on)
+                if (S.mode == kScanExact) S.dirty[b] = next_dirty(S.dirty[b], c != 0u);
+                else if (c) S.dirty[b] |= kDirtyNow;
+            }
         } else {
             c = cr = predicted_size(S, b);
         }
@@ -316,8 +320,8 @@ ScanDev scan_of(const FrameDev& F, uint32_t mode) {
     S.spin_limit = F.scan_spin_limit;
     S.silent_tile1 = F.scan_silent_tile1;
     // the scan that places a frame's exact lists flags its bins; the
-    // capacity scan clears the flags for the raster
-    S.dirty = mode == kScanPredictedItems ? nullptr : F.dirty_wr;
+    // capacity scan leaves them to the raster
+    S.dirty = mode == kScanPredictedItems ? nullptr : F.dirty;
     return S;
 }
 
