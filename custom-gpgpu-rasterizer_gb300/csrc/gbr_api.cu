@@ -3,8 +3,10 @@
 // Host orchestration of one frame, replacing CUDARenderer::Render's
 // per-mesh loop, its per-256-triangle chunk loop and the device-wide
 // synchronisation after every stage (CustomCUDARasterizer/CUDARenderer.cu:
-// 206-354): a frame is four to seven kernel launches on the caller's stream with
-// no host synchronisation, whatever the number of meshes or triangles.
+// 206-354): a frame is four to seven kernel launches on the caller's stream (with
+// predicted binning ten or eleven, three of which return at once unless a
+// capacity was exceeded) and no host synchronisation, whatever the number of
+// meshes or triangles.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -560,7 +562,7 @@ gbr_status gbr_setup_bins(gbr_renderer* r, uint32_t num_bins_x, uint32_t num_bin
     GBR_CUDA(cudaMalloc(&r->d_capacity, nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMemset(r->d_capacity, 0, nb * sizeof(uint32_t)));
     GBR_CUDA(cudaMalloc(&r->d_bin_end, nb * sizeof(uint32_t)));
-    GBR_CUDA(cudaMalloc(&r->d_dirty, nb));
+    GBR_CUDA(cudaMalloc(&r->d_dirty, ((size_t)nb + 3u) & ~(size_t)3u));   // also written in words
     GBR_CUDA(cudaMalloc(&r->d_scan, scan_state_bytes(nb)));
     GBR_CUDA(cudaMemset(r->d_scan, 0, scan_state_bytes(nb)));
     GBR_CUDA(cudaMemset(r->d_bin_end, 0, nb * sizeof(uint32_t)));

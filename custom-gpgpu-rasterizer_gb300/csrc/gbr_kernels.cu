@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(kRasterThreads, MIN_CTAS) raster_kernel(FrameD
         __syncthreads();
         const uint32_t bin = S.item[0];
         if (bin == 0xFFFFFFFFu) break;
-        if (tid == 0 && F.dirty) F.dirty[bin] |= kDirtyNow;   // the bin's pixels may now be drawn
+        if (tid == 0) mark_drawn(F, bin);
         const uint32_t start = S.item[1], count = S.item[2], nchunks = S.item[3];
         const int tx0 = (int)((bin % F.nbx) * F.bw), ty0 = (int)((bin / F.nbx) * F.bh);
         const int tw = min((int)F.bw, (int)F.width - tx0), th = min((int)F.bh, (int)F.height - ty0);

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : MIN_CTAS * (256 
         __syncthreads();
         const uint32_t bin = S.item[turn][0];
         if (bin == 0xFFFFFFFFu) break;
-        if (!BATCH && tid == 0 && F.dirty) F.dirty[bin] |= kDirtyNow;   // the bin's pixels may now be drawn
+        if (!BATCH && tid == 0) mark_drawn(F, bin);
         if (BATCH) {
             const uint32_t sc = S.scene[turn];
             if (sc != S.scene_loaded) {   // uniform across the CTA

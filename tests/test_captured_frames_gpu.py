@@ -18,9 +18,12 @@ def moving_sphere(textured):
     return s
 
 
-@pytest.mark.parametrize("textured", [True, False])   # shaded in two passes, and in one
-def test_replays_over_moving_vertices(gbr_lib, cuda_device, textured):
+@pytest.mark.parametrize("textured,route", [(True, "fused scan"), (True, "scan kernel"), (True, "predicted"), (True, "tma"),
+                                            (False, "fused scan")])   # shaded in two passes, and in one
+def test_replays_over_moving_vertices(gbr_lib, cuda_device, textured, route):
+    import ctypes as C
     import torch
+    from oracle import mlp_oracle
     s = moving_sphere(textured)
     m = s.meshes[0]
     at = [(0.0, 0.0), (0.9, 0.3), (-0.9, -0.4), (0.2, 0.7), (0.0, 0.0)]
@@ -39,6 +42,16 @@ def test_replays_over_moving_vertices(gbr_lib, cuda_device, textured):
         tex = [r.add_texture(t) if t is not None else -1 for t in m.textures]
         r.bind_mesh_device(v.data_ptr(), len(m.vertices), m.vertex_format, ix.data_ptr(), len(m.indices), m.topology,
                            m.world, tex)
+        r.set_raster_staging(route == "tma")
+        if route == "scan kernel":
+            r.set_scan_wait(1 << 20, -1)
+        if route == "predicted":
+            weights = np.zeros(mlp_oracle.NUM_PARAMS, np.float32)
+            weights[mlp_oracle.OFF_B3] = 512.0   # more than any bin holds
+            w16 = mlp_oracle.f32_to_bf16(weights)
+            gbr_lib.check(r._lib.gbr_set_predictor(r.h, w16.ctypes.data_as(C.c_void_p), len(w16), C.c_float(0.0),
+                                                   C.c_float(0.0), C.c_float(0.0)))
+            r.set_binning(gbr_lib.BINNING_PREDICTED)
         return r
 
     want = []
