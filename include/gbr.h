@@ -93,11 +93,14 @@ gbr_status gbr_destroy(gbr_renderer *r);
 /* SetupBins(numBins, binDim, queueMaxSize) (CUDARenderer.cu:199-204).
  * Bins are exact-sized (no capacity, no dropped triangles); queue_chunk
  * keeps the queue size's role in the raster: a bin's triangles are
- * depth-sorted and rasterised into its tile queue_chunk at a time (between 512
- * or 1024 and 2048, as the raster's CTAs hold; from 1 with
- * GBR_STAGING_TMA; 0 = 4096, i.e. 2048).  Long bins are split across raster CTAs by the
- * library, in work items of 64..4096 entries (512..4096 in the block raster)
- * sized from the last frame. */
+ * depth-sorted and rasterised into its tile that many at a time.  The default
+ * raster sorts at least 1024 at once and at most what its CTAs hold: 512 or
+ * 1024 in CTAs of 64 or 128 threads, where queue_chunk therefore has no
+ * effect, and 2048 in those of 512; with GBR_STAGING_TMA passes are of 1 to 2048
+ * (0 = 4096, i.e. the most).  Long bins are split across raster CTAs by the
+ * library, in work items of 64..4096 entries sized from the last frame (of
+ * 512 or more where triangles cover their bins three times over or more,
+ * but for frames of few, short items). */
 gbr_status gbr_setup_bins(gbr_renderer *r, uint32_t num_bins_x, uint32_t num_bins_y,
                           uint32_t bin_w, uint32_t bin_h, uint32_t queue_chunk);
 
@@ -225,8 +228,9 @@ gbr_status gbr_set_binning(gbr_renderer *r, uint32_t method);
 /* Raster tuning (no counterpart in the reference; used by the autotuner):
  * phase = triangles the raster with bulk-copy staging rasterises between hierarchical-z refreshes, 0..128
  * (0: the library's choice: 16, 64 for frames of small triangles); the default raster refreshes after every
- * triangle, and with a phase of 1..31 leaves no triangle to the set-up pass; ctas_per_sm = occupancy variant of the raster kernel in CTAs of 256 threads, 2..6 (0: the
- * library's choice). */
+ * triangle, and with a phase of 1..31 leaves no triangle to the set-up pass; ctas_per_sm = occupancy variant
+ * of the raster kernel in CTAs of 256 threads, 2..6 (0: the library's choice; without effect in frames of few
+ * items, which run CTAs of 512 threads, two an SM). */
 gbr_status gbr_set_raster_params(gbr_renderer *r, uint32_t phase, uint32_t ctas_per_sm);
 /* How the raster stages triangle-setup records into shared memory (no
  * counterpart in the reference, whose RA_PerTileKernel reads them from global
@@ -271,7 +275,10 @@ gbr_status gbr_render(gbr_renderer *r, const gbr_camera *cam, uint32_t cull, uin
 /* Present (CUDARenderer.cu:383-395) without a window: waits for `stream`
  * and copies the framebuffer (and optionally the per-pixel interpolated
  * depth, 0 where no fragment landed) to host memory.  If the frame's bin
- * storage overflowed, the frame is re-rendered with exact storage first. */
+ * storage overflowed, the frame is re-rendered with exact storage and copied
+ * again.  The copies are queued together with the frame's status, so after an
+ * error (GBR_ERR_TIMEOUT, GBR_ERR_OUT_OF_MEMORY) the two buffers hold pixels of
+ * no particular frame. */
 gbr_status gbr_readback(gbr_renderer *r, uint32_t *colour, float *depth, void *stream);
 /* Winning primitive id per pixel (0xFFFFFFFF where empty). */
 gbr_status gbr_readback_ids(gbr_renderer *r, uint32_t *ids, void *stream);
@@ -300,13 +307,15 @@ typedef struct gbr_batch gbr_batch;
 typedef struct {
     uint32_t bin_size;     /* bins of bin_size x bin_size pixels, 1..64 */
     uint32_t queue_chunk;  /* entries depth-sorted and rasterised per pass over a tile, >= 1 (1024 to 2048
-                              used); work items hold 2048 entries */
+                              used; CTAs of 128 threads 1024, of 64 512, whatever is asked); work items hold
+                              2048 entries, or 64 where the scenes' triangles cover their bins fewer than
+                              three times over */
     uint32_t raster_ctas;  /* raster variant: CTAs per SM, 2..6 (0: 4), counted in CTAs of 256 threads */
     uint32_t raster_phase; /* 0..128; kept, without effect: a batch's raster refreshes its depth bounds after
                               every triangle */
-    uint32_t raster_threads; /* threads per bin: raster CTAs of 128 or 256 threads (0: 256); a 128-thread CTA
-                                depth-sorts 1024 entries at a time (else 2048), and twice raster_ctas
-                                of them are resident per SM */
+    uint32_t raster_threads; /* threads per bin: raster CTAs of 128 or 256 threads (0: 256; bins of up to 8x8
+                                pixels run CTAs of 64); a 128-thread CTA depth-sorts 1024 entries at a time
+                                (else 2048), and twice raster_ctas of them are resident per SM */
 } gbr_batch_config;
 typedef struct {
     uint32_t num_scenes;
@@ -331,7 +340,9 @@ gbr_status gbr_batch_get_config(const gbr_batch *b, gbr_batch_config *cfg);
 /* Times `frames` batch frames (after one warm-up frame) for every
  * combination of the candidate bin sizes, queue chunks, raster variants
  * (CTAs per SM) and threads per bin (a NULL list keeps the current value)
- * and keeps the fastest; *best gets it.  Synchronises `stream`. */
+ * and keeps the fastest; *best gets it.  Combinations that run the same (queue
+ * chunks that give the same pass, above all) are timed once, and the first of
+ * them is reported.  Synchronises `stream`. */
 gbr_status gbr_batch_autotune(gbr_batch *b, const uint32_t *bin_sizes, uint32_t num_bin_sizes, const uint32_t *chunks,
                               uint32_t num_chunks, const uint32_t *raster_ctas, uint32_t num_raster_ctas,
                               const uint32_t *raster_threads, uint32_t num_raster_threads, uint32_t frames,
