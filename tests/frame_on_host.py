@@ -12,7 +12,7 @@ import scenes
 
 
 def load(tmp_dir) -> C.CDLL:
-    gbr_build.build()
+    gbr_build.build(force=not os.path.exists(os.path.join(gbr_build.OUT_DIR, "gbr_api.o")))
     lib = os.path.join(str(tmp_dir), "frame_on_host.so")
     src = [os.path.join(gbr_build.ROOT, "tests", "cpp", f) for f in ("frame_on_host.cu", "cuda_on_host.cpp")]
     subprocess.run([gbr_build.nvcc(), "-shared", "-cudart", "none", "-std=c++17", "-O1", *gbr_build.ARCH, "-Xcompiler",
